@@ -234,13 +234,13 @@ __global__ void __launch_bounds__(512, MODE == MODE_EXACT ? 1 : 4) k_batch_sweep
 	// block's own loads: requests in flight that hold no registers
 	if (p.pf_ahead > 0) {
 		const int64_t bt = (int64_t)blockIdx.x + p.pf_ahead;
-		const int lines = (int)blockDim.x / 32;
-		if (bt < (int64_t)gridDim.x && (int)threadIdx.x < 9 * lines) {
+		const int shift = blockDim.x >= 512 ? 4 : (blockDim.x >= 256 ? 3 : 2); // log2 of the lines per plane
+		if (bt < (int64_t)gridDim.x && (int)threadIdx.x < 9 << shift) {
 			const int4 *tt = reinterpret_cast<const int4 *>(p.trec + bt);
 			const int4 q0 = __ldg(tt), q1 = __ldg(tt + 1);
 			if (q1.w) {
 				const int64_t c0 = (int64_t)(((uint64_t)(uint32_t)q0.y << 32) | (uint32_t)q0.x);
-				const int i = (int)threadIdx.x / lines, k = (int)threadIdx.x - i * lines;
+				const int i = (int)threadIdx.x >> shift, k = (int)threadIdx.x & ((1 << shift) - 1);
 				asm volatile("prefetch.global.L2 [%0];" ::"l"(p.f + i * p.plane + c0 + k * 32));
 			}
 		}

@@ -679,6 +679,7 @@ extern "C" int kel_upload_field(kel_lattice *L, int32_t field, const float *host
 	}
 	if (field == KEL_FIELD_FORCE) {
 		if ((rc = ensure_field(L, &L->force, L->plane * L->d.D, 0.0f))) return rc;
+		L->force_zero = false;
 		return field_io(L, L->force, nullptr, host, L->d.D);
 	}
 	if (field == KEL_FIELD_HLBM_N) {
@@ -898,7 +899,9 @@ static SweepParams make_params(kel_lattice *L, const kel_step_program *P) {
 	p.rho = L->rho;
 	p.u = L->u;
 	p.por = L->por;
-	p.force = L->force;
+	// an untouched force field is zero: the sweeps don't read it (8 of 85 bytes
+	// per D2Q9 cell, 12 of 229 per D3Q27 cell)
+	p.force = L->force_zero ? nullptr : L->force;
 	p.hN = L->hN;
 	p.hD = L->hD;
 	p.profile = L->profile;
@@ -917,18 +920,21 @@ static SweepParams make_params(kel_lattice *L, const kel_step_program *P) {
 	for (int i = 0; i < 27; ++i) p.wshift[i] = L->wshift[i];
 	p.cpt = L->cpt;
 	p.idx32 = (int64_t)L->d.Q * L->plane < ((int64_t)1 << 31) ? 1 : 0;
-	p.block = L->block;
+	if (p.idx32)
+		for (int i = 0; i < L->d.Q; ++i) {
+			p.off_even[i] = (int)(i * L->plane);
+			p.off_odd[i] = (int)(i * L->plane + L->d.c[i][0] + (L->d.c[i][1] + L->d.c[i][2] * L->desc.ny) * L->nxp);
+		}
+	// Rows are covered by whole blocks: with no launch shape asked for, 64
+	// threads where that leaves fewer idle ones in a row's last block than 128
+	// (64-cell rows half filled their blocks: D3Q19 64^3 12.0 us per step)
+	p.block = !L->tuned && L->cpt == 1 && (L->nxp + 63) / 64 * 64 < (L->nxp + 127) / 128 * 128 ? 64 : L->block;
 	p.hw_mask = L->hw_active ? L->hw_mask : nullptr;
 	p.plain = L->plain_flags;
 	p.stages = L->cpt == CPT_ROWS ? L->block : 0;
 	p.sms = L->sms;
 	p.err = L->d_err;
 	if (L->cpt == CPT_ROWS) L->rows_used = true;
-	// one-cell sweep: prefetch the rows of the block one resident wave later
-	// (32 warps per SM at most: 1024 / block blocks on each SM); measured at
-	// 256^3: D3Q19 FP32 0.92 -> 0.97 of HBM, FP16S 0.50 -> 0.55, D3Q27 FP32
-	// 0.88 -> 0.95; two or three waves ahead gained less
-	p.pf_ahead = L->sms * (1024 / (L->block > 0 ? L->block : 256));
 	return p;
 }
 
@@ -1068,6 +1074,8 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 	if ((rc = ensure_collision_fields(L, P->collision))) return rc;
 
 	SweepParams p = make_params(L, P);
+	// a caller's graph may be replayed after an upload of the force field
+	if (capturing && !L->own_capture) p.force = L->force;
 	const bool exact = P->arithmetic == KEL_ARITH_REFERENCE;
 	uint64_t s = 0;
 	// Long runs without macro output replay a captured graph of GRAPH_STEPS

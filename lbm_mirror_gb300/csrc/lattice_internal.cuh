@@ -50,6 +50,8 @@ struct kel_lattice {
 	void *f = nullptr;
 	uint8_t *flags = nullptr;
 	float *rho = nullptr, *u = nullptr, *por = nullptr, *force = nullptr, *profile = nullptr;
+	bool force_zero = true; // nothing but the initial zeros was ever written to `force`
+	bool own_capture = false; // this library is capturing a graph of its own on `stream`
 	float *hN = nullptr, *hD = nullptr; // HLBM particle_N (D planes) and particle_D, on first use
 	// Counts writes of the porosity field: an uploaded field, an HLBM couple
 	// and every PSM couple advance it, so a particle set sees whether the

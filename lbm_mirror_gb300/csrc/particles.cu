@@ -1895,6 +1895,7 @@ int check_params(const kel_particles *ps, const kel_particle_params *prm, const 
 			return fail(KEL_ERR_UNSUPPORTED, "%s: FPLBM coupling needs a non-periodic lattice", who);
 		int rc;
 		if ((rc = ensure_field(ps->lat, &ps->lat->force, ps->lat->plane * ps->lat->d.D, 0.0f))) return rc;
+		ps->lat->force_zero = false; // the couple writes it
 	}
 	if (prm->coupling == KEL_COUPLING_HLBM) {
 		if (ps->lat->d.Q != 9) return fail(KEL_ERR_UNSUPPORTED, "%s: HLBM coupling is D2Q9 only", who);
@@ -2437,8 +2438,10 @@ static int ensure_particle_graph(kel_particles *ps, const kel_particle_params *p
 		cudaGetLastError();
 		return KEL_ERR_CUDA;
 	}
+	L->own_capture = true;
 	rc = coupled_step(ps, prm, prog, 0, ps->side);
 	if (rc == KEL_OK) rc = coupled_step(ps, prm, prog, 0, ps->side);
+	L->own_capture = false;
 	cudaGraph_t g = nullptr;
 	cudaError_t e = cudaStreamEndCapture(L->stream, &g);
 	L->t = t0;

@@ -69,7 +69,7 @@ struct SweepParams {
 	float *rho;       // macros "density" (plane layout)
 	float *u;         // macros "velocity", D planes
 	const float *por; // macros "porosity"
-	const float *force; // macros "force", D planes
+	const float *force; // macros "force", D planes (null: zero everywhere, not read)
 	const float *hN;    // HLBM "particle_N", D planes
 	const float *hD;    // HLBM "particle_D"
 	const float *profile; // inlet u_x per y
@@ -84,7 +84,13 @@ struct SweepParams {
 	float g[3];       // global force
 	float wshift[27]; // FP16S: stored value is f - wshift[i]
 	int cpt;          // cells per thread: 1 (sweep1_kernel), 2 (sweep2_kernel), 4 (sweep_kernel), CPT_ROWS (sweep_rows_kernel)
-	int idx32;        // Q * plane < 2^31: offsets from a cell fit 32-bit arithmetic
+	int idx32;        // Q * plane < 2^31: a population's index fits 32-bit arithmetic
+	// idx32: index offsets from a cell in plane 0 -- off_even[i]: its slot in
+	// plane i; off_odd[i]: the slot of x + c_i in plane i.  Read from the
+	// parameter bank, an access costs one 32-bit add; formed from the plane
+	// stride it costs four to five integer instructions, a third of the
+	// sweep's issue slots.
+	int off_even[27], off_odd[27];
 	int block;        // threads per block
 	int wpr2;         // sweep2_kernel: warps per row (32 cell pairs per warp)
 	const uint32_t *hw_mask; // half-way walls: per cell, bit i = the neighbour x + c_i is one (null: none)
@@ -94,8 +100,10 @@ struct SweepParams {
 	// bit f: flag value f (1 .. MAX_FLAGS-1) has no boundary step and collides,
 	// so its cells skip the operation-table dispatch (same result)
 	uint32_t plain;
-	// sweep1_kernel: blocks ahead whose rows a block prefetches into L2 (0: none)
-	int pf_ahead;
+	// sweep1_kernel: how far ahead a block prefetches rows into L2, in grid
+	// coordinates (the launch fills them in: no division in the kernel), and
+	// log2 of the 128-byte lines of a block's x range per direction plane
+	int pf_x, pf_y, pf_z, pf_shift;
 };
 
 // What the per-cell physics needs from a launch: the flag -> operation table,
@@ -342,18 +350,40 @@ __device__ __forceinline__ void equilibrium(float rho, const float (&u)[3], floa
 	}
 }
 
-// Guo forcing term F_i, modules/core/c++/collision.hpp:170-196
-template <class L, bool EXACT>
-__device__ __forceinline__ float guo_term(int i, const float (&u)[3], const float (&F)[3]) {
+// Guo forcing term F_i, modules/core/c++/collision.hpp:170-196: the sum over
+// the axes of ((c_k - u_k) 3 + c_k s) F_k with s = 9 c.u, in the reference's
+// order.  An axis with c_k = 0 contributes (-u_k 3) F_k, since (-u_k 3) + 0 s
+// is (-u_k 3) exactly (an infinite s comes with an infinite u^2, which makes
+// the equilibrium and so the cell NaN either way); that product and the
+// (+-1 - u_k) 3 are the same for every direction and are formed once
+// (GuoAxes).  D3Q27 with a force: 703 -> 594 FP32 operations per cell.
+struct GuoAxes {
+	float up[3], dn[3], zero[3]; // (1 - u) 3, (-1 - u) 3, ((0 - u) 3) F
+};
+
+template <class L>
+__device__ __forceinline__ GuoAxes guo_axes(const float (&u)[3], const float (&F)[3]) {
+	using A = Ar<true>;
+	GuoAxes g;
+#pragma unroll
+	for (int k = 0; k < L::D; ++k) {
+		g.up[k] = A::mul(A::sub(1.f, u[k]), 3.0f);
+		g.dn[k] = A::mul(A::sub(-1.f, u[k]), 3.0f);
+		g.zero[k] = A::mul(A::mul(A::sub(0.f, u[k]), 3.0f), F[k]);
+	}
+	return g;
+}
+
+template <class L>
+__device__ __forceinline__ float guo_term(int i, const float (&u)[3], const float (&F)[3], const GuoAxes &g) {
 	using A = Ar<true>;
 	const float s = A::mul(A::mul(cdot<L, true>(i, u), 3.0f), 3.0f);
 	float proj = 0.f;
 #pragma unroll
 	for (int k = 0; k < L::D; ++k) {
-		const float ck = (float)cdir<L>(i, k);
-		const float t1 = A::mul(A::sub(ck, u[k]), 3.0f);
-		const float t2 = A::mul(ck, s);
-		proj = A::add(proj, A::mul(A::add(t1, t2), F[k]));
+		const int c = cdir<L>(i, k);
+		const float t = c > 0 ? A::mul(A::add(g.up[k], s), F[k]) : (c < 0 ? A::mul(A::sub(g.dn[k], s), F[k]) : g.zero[k]);
+		proj = k == 0 ? A::add(0.f, t) : A::add(proj, t);
 	}
 	return A::mul((float)L::w(i), proj);
 }
@@ -491,6 +521,7 @@ __device__ __forceinline__ void collide(float (&f)[L::Q], const CellCtx &p, floa
 #pragma unroll
 		for (int k = 0; k < L::D; ++k) F[k] = A::add(Fc[k], p.g[k]);
 	}
+	const GuoAxes ga = guo_axes<L>(u, F); // unused without a force
 	if (COLL == COLL_BGK || COLL == COLL_HLBM) {
 #pragma unroll
 		for (int i = 0; i < L::Q; ++i)
@@ -498,7 +529,7 @@ __device__ __forceinline__ void collide(float (&f)[L::Q], const CellCtx &p, floa
 	} else if (COLL == COLL_BGK_GUO) {
 #pragma unroll
 		for (int i = 0; i < L::Q; ++i) {
-			const float Fi = guo_term<L, EXACT>(i, u, F);
+			const float Fi = guo_term<L>(i, u, F, ga);
 			f[i] = A::add(A::add(f[i], A::mul(p.omega, A::sub(eq[i], f[i]))), A::mul(Fi, p.guo_scale));
 		}
 	} else { // PSM, psm.hpp:79-88
@@ -510,7 +541,7 @@ __device__ __forceinline__ void collide(float (&f)[L::Q], const CellCtx &p, floa
 		for (int i = 0; i < L::Q; ++i) {
 			float v = A::add(pre[i], A::mul(A::mul(p.omega, A::sub(eq[i], pre[i])), por));
 			v = A::add(v, A::mul(A::sub(pre[L::opp(i)], pre[i]), flip));
-			if (COLL == COLL_PSM_GUO) v = A::add(v, A::mul(guo_term<L, EXACT>(i, u, F), p.guo_scale));
+			if (COLL == COLL_PSM_GUO) v = A::add(v, A::mul(guo_term<L>(i, u, F, ga), p.guo_scale));
 			f[i] = v;
 		}
 	}
@@ -661,7 +692,7 @@ __global__ void __launch_bounds__(256) sweep_kernel(const __grid_constant__ Swee
 	if ((COLL == COLL_PSM || COLL == COLL_PSM_GUO) && active)
 		porv = *reinterpret_cast<const float4 *>(p.por + rbase + x0);
 	float4 fcv[3] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && active) {
+	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force && active) {
 #pragma unroll
 		for (int k = 0; k < L::D; ++k) fcv[k] = *reinterpret_cast<const float4 *>(p.force + k * p.plane + rbase + x0);
 	}
@@ -848,7 +879,7 @@ __global__ void __launch_bounds__(256) sweep2_kernel(const __grid_constant__ Swe
 	if ((COLL == COLL_PSM || COLL == COLL_PSM_GUO || COLL == COLL_HLBM) && active)
 		porv = *reinterpret_cast<const float2 *>(p.por + rbase + x0);
 	float2 fcv[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && active) {
+	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force && active) {
 #pragma unroll
 		for (int k = 0; k < L::D; ++k) fcv[k] = *reinterpret_cast<const float2 *>(p.force + k * p.plane + rbase + x0);
 	}
@@ -1032,7 +1063,7 @@ __global__ void __launch_bounds__(256, 4) sweep2h_kernel(const __grid_constant__
 	if ((COLL == COLL_PSM || COLL == COLL_PSM_GUO || COLL == COLL_HLBM) && active)
 		porv = *reinterpret_cast<const float2 *>(p.por + rbase + x0);
 	float2 fcv[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && active) {
+	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force && active) {
 #pragma unroll
 		for (int k = 0; k < L::D; ++k) fcv[k] = *reinterpret_cast<const float2 *>(p.force + k * p.plane + rbase + x0);
 	}
@@ -1133,6 +1164,12 @@ __global__ void __launch_bounds__(256, 4) sweep2h_kernel(const __grid_constant__
 // global-load latency, and 32 resident warps per SM keep more loads in
 // flight than 24 at 80 registers (measured +3 % FP32, +6 % FP16S at 256^3;
 // the few spilled words stay in L1).
+// Index tables in the parameter bank, prefetch coordinates by carries and the
+// force terms shared between directions took the instructions per cell from
+// 567 / 621 (even / odd step) to 449 / 518 for D3Q19 FP32, 611 / 714 to
+// 533 / 616 FP16S, 1,421 / 1,366 to 1,071 / 1,234 for D3Q27 with a force.
+// Measured: FP16S 256^3 (40 steps) 15.55 -> 14.05 ms, D3Q27 173x131x97 with a
+// force (24 steps) 4.63 -> 3.91 ms, D3Q19 64^3 (100 steps) 1.37 -> 1.19 ms.
 // HW: the lattice has half-way walls (p.hw_mask set); a separate
 // instantiation, so that the stores' redirection costs the common case
 // nothing.
@@ -1157,53 +1194,54 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	const bool ok_xm = has_xm || p.periodic;  // x - 1 exists
 	const bool ok_xp = has_xp || p.periodic;  // x + 1 exists
 	const bool row_interior = y > 0 && y + 1 < p.ny && (L::D == 2 || (z > 0 && z + 1 < p.nz));
-	// 32-bit offsets from this cell's slot in plane 0 (when they fit): one
-	// 32-bit multiply-add per population instead of 64-bit index arithmetic
 	using ST = typename S::T;
-	ST *const fc = static_cast<ST *>(p.f) + cell;
-	const int pl32 = (int)p.plane, oy32 = nxp, oz32 = nxp * p.ny;
-	// L2 prefetch of the rows the block p.pf_ahead places later in launch
-	// order will read (its x range in every direction plane; in odd steps its
+	const int c32 = (int)cell; // p.idx32: the cell's index in plane 0
+	// L2 prefetch of the rows the block (pf_x, pf_y, pf_z) later will read (its x range in every direction plane; in odd steps its
 	// neighbours' rows are prefetched by their own predecessors): requests in
 	// flight that hold no registers, one 128-byte line per thread.
-	if (p.pf_ahead > 0) {
-		const unsigned gx = gridDim.x;
-		const int64_t nblk = (int64_t)gx * gridDim.y * gridDim.z;
-		const int64_t b = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gx + blockIdx.x + p.pf_ahead;
-		if (b < nblk) {
-			const int x0 = (int)(b % gx) * (int)blockDim.x;
-			const int64_t row = b / gx;
-			const int n = min((int)blockDim.x, nxp - x0);
+	{
+		// by carries: the 64-bit divisions of a flat block index cost every
+		// thread 40 to 50 instructions
+		int bx = (int)blockIdx.x + p.pf_x, by = (int)blockIdx.y + p.pf_y, bz = (int)blockIdx.z + p.pf_z;
+		if (bx >= (int)gridDim.x) {
+			bx -= (int)gridDim.x;
+			++by;
+		}
+		if (by >= (int)gridDim.y) {
+			by -= (int)gridDim.y;
+			++bz;
+		}
+		if (bz < (int)gridDim.z) {
 			constexpr int per = 128 / (int)sizeof(ST); // cells per line
-			const int lines = (n + per - 1) / per;
-			const int t = threadIdx.x;
-			if (t < Q * lines) {
-				const int i = t / lines, l = t - i * lines;
-				const ST *a = static_cast<const ST *>(p.f) + i * p.plane + row * nxp + x0 + l * per;
+			const int i = (int)threadIdx.x >> p.pf_shift;
+			const int x0 = bx * (int)blockDim.x + ((int)threadIdx.x & ((1 << p.pf_shift) - 1)) * per;
+			if (i < Q && x0 < nxp) {
+				const ST *a = static_cast<const ST *>(p.f) + i * p.plane + (static_cast<int64_t>(bz) * p.ny + by) * nxp + x0;
 				asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
 			}
 		}
 	}
 
 	float f[Q];
+	// p.idx32, odd steps: the cell's index for accesses to x - 1 and x + 1
+	// (periodic rows wrap)
+	const int c32m = c32 + (has_xm ? 0 : nxp), c32p = c32 - (has_xp ? 0 : nxp);
 	if (!ODD && p.idx32) {
 #pragma unroll
-		for (int i = 0; i < Q; ++i) f[i] = S::ld1(fc, i * pl32, p.wshift[i]);
+		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_even[i], p.wshift[i]);
 	} else if (!ODD) {
 #pragma unroll
 		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, i * p.plane + cell, p.wshift[i]);
 	} else if (row_interior && p.idx32 && x_inner) {
-		// every neighbour exists: unit x offsets, no predicates
+		// every neighbour exists: no predicates (x - c_i in plane opp i)
 #pragma unroll
-		for (int i = 0; i < Q; ++i)
-			f[i] = S::ld1(fc, L::opp(i) * pl32 - L::cx(i) - L::cy(i) * oy32 - L::cz(i) * oz32, p.wshift[i]);
+		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_odd[L::opp(i)], p.wshift[i]);
 	} else if (row_interior && p.idx32) {
 #pragma unroll
 		for (int i = 0; i < Q; ++i) {
-			const int cx = L::cx(i), cy = L::cy(i), cz = L::cz(i);
-			const int off = L::opp(i) * pl32 + (cx > 0 ? xm : (cx < 0 ? xp : 0)) - cy * oy32 - cz * oz32;
+			const int cx = L::cx(i);
 			const bool ok = cx > 0 ? ok_xm : (cx < 0 ? ok_xp : true);
-			f[i] = ok ? S::ld1(fc, off, p.wshift[i]) : 0.f;
+			f[i] = ok ? S::ld1(p.f, (cx > 0 ? c32m : (cx < 0 ? c32p : c32)) + p.off_odd[L::opp(i)], p.wshift[i]) : 0.f;
 		}
 	} else if (row_interior) {
 #pragma unroll
@@ -1229,7 +1267,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	const int flag = p.flags[cell];
 	const float por = (COLL == COLL_PSM || COLL == COLL_PSM_GUO || COLL == COLL_HLBM) ? p.por[cell] : 1.f;
 	float Fc[3] = {0.f, 0.f, 0.f};
-	if (COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) {
+	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force) {
 #pragma unroll
 		for (int k = 0; k < L::D; ++k) Fc[k] = p.force[k * p.plane + cell];
 	}
@@ -1286,26 +1324,25 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 		}
 	}
 	if (!ODD) {
+		if (p.idx32) {
 #pragma unroll
-		for (int i = 0; i < Q; ++i) {
-			if (p.idx32) S::st1(fc, L::opp(i) * pl32, f[i], p.wshift[i]);
-			else S::st1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell, f[i], p.wshift[i]);
+			for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_even[L::opp(i)], f[i], p.wshift[i]);
+		} else {
+#pragma unroll
+			for (int i = 0; i < Q; ++i)
+				S::st1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell, f[i], p.wshift[i]);
 		}
 	} else if (row_interior && p.idx32 && x_inner) {
 		// every destination exists and no source lies outside: no predicates
 #pragma unroll
-		for (int i = 0; i < Q; ++i)
-			S::st1(fc, i * pl32 + L::cx(i) + L::cy(i) * oy32 + L::cz(i) * oz32, f[i], p.wshift[i]);
+		for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_odd[i], f[i], p.wshift[i]);
 	} else if (row_interior && p.idx32) {
 #pragma unroll
 		for (int i = 0; i < Q; ++i) {
-			const int cx = L::cx(i), cy = L::cy(i), cz = L::cz(i);
-			const int pb = i * pl32;
-			if (cx > 0 && !ok_xm) S::st1(fc, pb, 0.f, p.wshift[i]);
-			if (cx < 0 && !ok_xp) S::st1(fc, pb, 0.f, p.wshift[i]);
-			const int off = (cx > 0 ? xp : (cx < 0 ? xm : 0)) + cy * oy32 + cz * oz32;
+			const int cx = L::cx(i);
+			if ((cx > 0 && !ok_xm) || (cx < 0 && !ok_xp)) S::st1(p.f, c32 + p.off_even[i], 0.f, p.wshift[i]);
 			const bool ok = cx > 0 ? ok_xp : (cx < 0 ? ok_xm : true);
-			if (ok) S::st1(fc, pb + off, f[i], p.wshift[i]);
+			if (ok) S::st1(p.f, (cx > 0 ? c32p : (cx < 0 ? c32m : c32)) + p.off_odd[i], f[i], p.wshift[i]);
 		}
 	} else if (row_interior) {
 #pragma unroll

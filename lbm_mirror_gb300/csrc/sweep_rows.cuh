@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(ROWS_MAX_NXP + 32, 2) sweep_rows_kernel(const 
 		float Fc[3] = {0.f, 0.f, 0.f};
 		if (active) {
 			if (COLL == COLL_PSM || COLL == COLL_PSM_GUO || COLL == COLL_HLBM) por = p.por[cell];
-			if (COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) {
+			if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force) {
 #pragma unroll
 				for (int d = 0; d < L::D; ++d) Fc[d] = p.force[d * p.plane + cell];
 			}
