@@ -17,6 +17,7 @@
 #include "lattice_internal.cuh"
 #include "sweep_dispatch.cuh"
 #include "sweep_rows.cuh"
+#include "sweep_tile.cuh"
 
 using namespace kel::gb;
 
@@ -198,6 +199,7 @@ extern "C" int kel_lattice_destroy(kel_lattice *L) {
 	if (L->stream) cudaStreamSynchronize(L->stream);
 	else cudaDeviceSynchronize();
 	cudaFree(L->f);
+	cudaFree(L->f2);
 	cudaFree(L->flags);
 	cudaFree(L->d_seen);
 	cudaFree(L->d_err);
@@ -865,6 +867,7 @@ extern "C" int kel_lattice_set_launch(kel_lattice *L, int32_t cells_per_thread, 
 	L->cpt = cells_per_thread;
 	L->block = block_threads;
 	L->tuned = true;
+	L->shape_asked = true;
 	return KEL_OK;
 }
 
@@ -931,6 +934,7 @@ static SweepParams make_params(kel_lattice *L, const kel_step_program *P) {
 	p.block = !L->tuned && L->cpt == 1 && (L->nxp + 63) / 64 * 64 < (L->nxp + 127) / 128 * 128 ? 64 : L->block;
 	p.hw_mask = L->hw_active ? L->hw_mask : nullptr;
 	p.plain = L->plain_flags;
+	p.bounce = L->bounce_flags;
 	p.stages = L->cpt == CPT_ROWS ? L->block : 0;
 	p.sms = L->sms;
 	p.err = L->d_err;
@@ -999,19 +1003,87 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 	L->cpt = bc;
 	L->block = bb;
 	L->tuned = true;
+	L->shape_asked = false;
 	if (cells_per_thread) *cells_per_thread = bc;
 	if (block_threads) *block_threads = bb;
 	if (ms_per_step) *ms_per_step = best;
 	return KEL_OK;
 }
 
+// Tiles of a lattice of nxp x ny cells on `sms` multiprocessors (two blocks of
+// either shape run on each).  From 1.5 M cells up the wide tiles fill the
+// device several times over (2048x1024: 19.5 us per step against 19.7 for the
+// best small ones, 4096^2 117 against 129); below, the small ones with the
+// fewest rows that give every SM one block (each block's steps follow one
+// another, so a launch takes as long as its rows: 256x64 6 rows 1.55 us per
+// step, 16 rows 2.5), else two, else 20 rows (1021x347: 20 rows 5.5, 12 rows
+// 6.1, 40 rows 5.7).
+static TilePlan plan_tiles(int nxp, int ny, int sms) {
+	TilePlan t;
+	auto blocks = [&](int tx, int ty) { return (int64_t)((nxp + tx - 1) / tx) * ((ny + ty - 1) / ty); };
+	t.wide = (int64_t)nxp * ny >= 1500000;
+	if (t.wide) { // fewest rows of work per SM, tile row sums 4 ty + 20
+		const int tx = TileWide::W - 2 * TILE_K;
+		int64_t best = -1;
+		for (int ty = 24; ty <= 32; ty += 4) {
+			const int64_t w = (blocks(tx, ty) + 2 * sms - 1) / (2 * sms) * (4 * ty + 20);
+			if (best < 0 || w < best) {
+				best = w;
+				t.ty = ty;
+			}
+		}
+		return t;
+	}
+	const int tx = TileSmall::W - 2 * TILE_K;
+	for (t.ty = 4; t.ty <= 8; t.ty += 2)
+		if (blocks(tx, t.ty) <= sms) return t;
+	for (t.ty = 4; t.ty <= 24; t.ty += 2)
+		if (blocks(tx, t.ty) <= 2 * sms) return t;
+	t.ty = 20;
+	return t;
+}
+
+// The second population array, on first use.  A lattice that would not leave
+// three quarters of the free memory to others runs without the tiles.
+static bool ensure_f2(kel_lattice *L) {
+	if (L->f2) return true;
+	if (L->no_f2) return false;
+	const size_t bytes = (size_t)L->d.Q * L->plane * L->elem;
+	size_t free_b = 0, total_b = 0;
+	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
+		cudaMalloc(&L->f2, bytes) != cudaSuccess) {
+		cudaGetLastError();
+		L->f2 = nullptr;
+		L->no_f2 = true;
+		return false;
+	}
+	return true;
+}
+
+// 2 TILE_K steps from an even one: into the second array and back, so that
+// the populations are where they were.
+static cudaError_t launch_tile_pair(const kel_lattice *L, const SweepParams &p, int coll, bool exact) {
+	TileParams q;
+	q.p = p;
+	q.ty = L->tile.ty;
+	for (int k = 0; k < 2; ++k) {
+		q.p.f = k ? L->f2 : L->f;
+		q.out = k ? L->f : L->f2;
+		cudaError_t e = launch_tile(q, L->desc.storage, coll, exact, L->tile.wide, L->stream);
+		if (e != cudaSuccess) return e;
+	}
+	return cudaSuccess;
+}
+
 constexpr int GRAPH_STEPS = 64;
+static_assert(GRAPH_STEPS % (2 * TILE_K) == 0, "a graph holds whole tile pairs");
 
 // The captured graph of GRAPH_STEPS sweeps from an even step, for launch
 // parameters p (compared bit for bit with those of the cached graph; a
 // change re-captures).  A failed capture leaves the caller on plain launches.
-static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, bool exact) {
-	if (L->graph && L->graph_coll == coll && L->graph_exact == exact && memcmp(&L->graph_params, &p, sizeof(p)) == 0)
+static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, bool exact, bool tiled) {
+	if (L->graph && L->graph_coll == coll && L->graph_exact == exact && L->graph_tiled == tiled &&
+		memcmp(&L->graph_params, &p, sizeof(p)) == 0)
 		return KEL_OK;
 	if (L->graph) cudaGraphExecDestroy(L->graph);
 	L->graph = nullptr;
@@ -1021,7 +1093,10 @@ static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, boo
 		return KEL_ERR_CUDA;
 	}
 	cudaError_t e = cudaSuccess;
-	for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) e = launch_one(L, p, coll, exact, (k & 1) != 0);
+	if (tiled)
+		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; k += 2 * TILE_K) e = launch_tile_pair(L, p, coll, exact);
+	else
+		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) e = launch_one(L, p, coll, exact, (k & 1) != 0);
 	cudaError_t e2 = cudaStreamEndCapture(L->stream, &g);
 	if (e == cudaSuccess && e2 == cudaSuccess && g) e = cudaGraphInstantiate(&L->graph, g, 0);
 	else if (e == cudaSuccess) e = e2;
@@ -1034,6 +1109,7 @@ static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, boo
 	L->graph_params = p;
 	L->graph_coll = coll;
 	L->graph_exact = exact;
+	L->graph_tiled = tiled;
 	return KEL_OK;
 }
 
@@ -1061,6 +1137,9 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 			if ((ops[fl].bc == KEL_BC_NONE || ops[fl].bc == KEL_BC_FLUID) && ops[fl].collide && !ops[fl].no_macros)
 				plain |= 1u << fl;
 		L->plain_flags = plain;
+		L->bounce_flags = 0;
+		for (int fl = 1; fl < MAX_FLAGS; ++fl)
+			if (ops[fl].bc == KEL_BC_BOUNCE_BACK && !ops[fl].collide) L->bounce_flags |= 1u << fl;
 		uint32_t fp = 0;
 		for (int fl = 1; fl < MAX_FLAGS; ++fl)
 			if ((ops[fl].bc == KEL_BC_NONE || ops[fl].bc == KEL_BC_FLUID) && ops[fl].collide) fp |= 1u << fl;
@@ -1076,6 +1155,8 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 	SweepParams p = make_params(L, P);
 	// a caller's graph may be replayed after an upload of the force field
 	if (capturing && !L->own_capture) p.force = L->force;
+	// consecutive sweeps of this call overlap the next one's launch
+	p.overlap = L->cpt == 1 && L->stream != nullptr && !capturing ? 1 : 0;
 	const bool exact = P->arithmetic == KEL_ARITH_REFERENCE;
 	uint64_t s = 0;
 	// Long runs without macro output replay a captured graph of GRAPH_STEPS
@@ -1084,20 +1165,31 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 	const uint64_t plain = (step_flags & KEL_STEP_ALL_MACROS)
 							   ? 0
 							   : ((step_flags & KEL_STEP_WRITE_MACROS) && n_steps > 0 ? n_steps - 1 : n_steps);
-	if (L->stream != nullptr && !capturing && L->cpt != CPT_ROWS && plain >= 2 * GRAPH_STEPS) {
+	// D2Q9 runs without macro output do TILE_K steps per launch on tiles, in
+	// pairs of launches from an even step (the remaining steps follow one by one).
+	const bool tiled = L->d.Q == 9 && !capturing && !L->shape_asked && !L->hw_active && p.idx32 &&
+					   P->collision <= KEL_COLL_PSM_GUO && plain >= (L->t & 1u) + 2 * TILE_K && ensure_f2(L);
+	if (tiled && !L->tile.ty) L->tile = plan_tiles(L->nxp, (int)L->desc.ny, L->sms);
+	constexpr uint64_t pair = 2 * TILE_K;
+	const bool graphed = L->stream != nullptr && !capturing && L->cpt != CPT_ROWS && plain >= 2 * GRAPH_STEPS;
+	if (tiled || graphed) {
 		p.write_macros = 0;
 		for (; (L->t & 1u) && s < plain; ++s, ++L->t) {
 			cudaError_t e = launch_one(L, p, P->collision, exact, true);
 			if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_step: launch failed: %s", cudaGetErrorString(e));
 		}
-		const uint64_t reps = (plain - s) / GRAPH_STEPS;
-		if (reps > 0 && ensure_step_graph(L, p, P->collision, exact) == KEL_OK) {
+		const uint64_t reps = graphed ? (plain - s) / GRAPH_STEPS : 0;
+		if (reps > 0 && ensure_step_graph(L, p, P->collision, exact, tiled) == KEL_OK) {
 			for (uint64_t r = 0; r < reps; ++r) {
 				cudaError_t e = cudaGraphLaunch(L->graph, L->stream);
 				if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_step: graph launch failed: %s", cudaGetErrorString(e));
 			}
 			s += reps * GRAPH_STEPS;
 			L->t += reps * GRAPH_STEPS;
+		}
+		for (; tiled && plain - s >= pair; s += pair, L->t += pair) {
+			cudaError_t e = launch_tile_pair(L, p, P->collision, exact);
+			if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_step: launch failed: %s", cudaGetErrorString(e));
 		}
 	}
 	for (; s < n_steps; ++s) {

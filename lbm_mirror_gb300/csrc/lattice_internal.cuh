@@ -31,6 +31,12 @@ struct HostDesc {
 	double w[27];
 };
 
+// How a D2Q9 lattice is cut into tiles of TILE_K steps per launch (sweep_tile.cuh).
+struct TilePlan {
+	bool wide = false;
+	int ty = 0; // tile rows; 0: not planned yet
+};
+
 int grid_for(int64_t n);
 // Launch parameters of the sweep kel_step runs for program P on lattice L.
 SweepParams sweep_params(kel_lattice *L, const kel_step_program *P);
@@ -64,7 +70,7 @@ struct kel_lattice {
 	uint64_t t = 0;
 	float wshift[27];
 	bool have_ops = false;
-	uint32_t plain_flags = 0; // SweepParams::plain of the current program
+	uint32_t plain_flags = 0, bounce_flags = 0; // SweepParams::plain and bounce of the current program
 	// flags whose op has no boundary step and collides (the FPLBM drivers'
 	// info 2), from the last program passed to kel_step
 	uint32_t plain_flags_fplbm = 1u << 2;
@@ -82,6 +88,10 @@ struct kel_lattice {
 	cudaGraphExec_t graph = nullptr;    // GRAPH_STEPS captured sweeps (kel_step), for graph_params
 	kel::gb::SweepParams graph_params;
 	int graph_coll = -1;
-	bool graph_exact = false;
+	bool graph_exact = false, graph_tiled = false;
 	bool tuned = false;
+	bool shape_asked = false; // kel_lattice_set_launch named a shape: every step runs it
+	void *f2 = nullptr;       // second population array of the multi-step tiles (TilePlan)
+	bool no_f2 = false;       // it could not be had
+	kel::gb::TilePlan tile;
 };

@@ -100,6 +100,8 @@ struct SweepParams {
 	// bit f: flag value f (1 .. MAX_FLAGS-1) has no boundary step and collides,
 	// so its cells skip the operation-table dispatch (same result)
 	uint32_t plain;
+	int overlap;     // launch with programmatic stream serialization (see grid_dependency_wait)
+	uint32_t bounce; // bit f: flag value f bounces back and does not collide
 	// sweep1_kernel: how far ahead a block prefetches rows into L2, in grid
 	// coordinates (the launch fills them in: no division in the kernel), and
 	// log2 of the 128-byte lines of a block's x range per direction plane
@@ -127,6 +129,14 @@ __device__ __forceinline__ CellCtx cell_ctx(const SweepParams &p) {
 	c.g[2] = p.g[2];
 	return c;
 }
+
+// Programmatic dependent launch: a sweep lets the next one's blocks start as
+// soon as its own have all started, and waits itself for the sweep before
+// (all of it, with its writes visible) before it touches a population.  Both
+// do nothing when the launch does not ask for it.  Between two sweeps this
+// leaves the drain of one and the start of the next, not the launch latency.
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // Arithmetic policy.  EXACT: the reference's rounding sequence (no fused
@@ -547,11 +557,9 @@ __device__ __forceinline__ void collide(float (&f)[L::Q], const CellCtx &p, floa
 	}
 }
 
-// Boundary step + collision of one cell (the body of a driver's switch(info)).
-// Returns true when the cell collided (its moments go to the macro fields).
-template <class L, int COLL, bool EXACT>
-__device__ __forceinline__ bool cell_update(float (&f)[L::Q], int flag, int y, const CellCtx &p, float por,
-											const float (&Fc)[3], float &rho, float (&u)[3]) {
+// Boundary step of one cell; returns true when its op collides afterwards.
+template <class L, bool EXACT>
+__device__ __forceinline__ bool boundary_step(float (&f)[L::Q], int flag, int y, const CellCtx &p) {
 	using A = Ar<true>;
 	if (flag == 0) { // outside the lattice: what the zero ghost ring supplies
 #pragma unroll
@@ -603,19 +611,26 @@ __device__ __forceinline__ bool cell_update(float (&f)[L::Q], int flag, int y, c
 	default:
 		break;
 	}
-	if (__ldg(&op->collide)) {
-		if (COLL == COLL_BGK_GUO) {
-			if (__ldg(&op->bgk_only)) {
-				collide<L, COLL_BGK, EXACT>(f, p, por, Fc, rho, u);
-				return true;
-			}
-			collide<L, COLL, EXACT>(f, p, por, Fc, rho, u);
-			return !__ldg(&op->no_macros);
+	return __ldg(&op->collide) != 0;
+}
+
+// Boundary step + collision of one cell (the body of a driver's switch(info)).
+// Returns true when the cell collided (its moments go to the macro fields).
+template <class L, int COLL, bool EXACT>
+__device__ __forceinline__ bool cell_update(float (&f)[L::Q], int flag, int y, const CellCtx &p, float por,
+											const float (&Fc)[3], float &rho, float (&u)[3]) {
+	if (!boundary_step<L, EXACT>(f, flag, y, p)) return false;
+	const OpEntry *op = p.ops + flag;
+	if (COLL == COLL_BGK_GUO) {
+		if (__ldg(&op->bgk_only)) {
+			collide<L, COLL_BGK, EXACT>(f, p, por, Fc, rho, u);
+			return true;
 		}
 		collide<L, COLL, EXACT>(f, p, por, Fc, rho, u);
-		return true;
+		return !__ldg(&op->no_macros);
 	}
-	return false;
+	collide<L, COLL, EXACT>(f, p, por, Fc, rho, u);
+	return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1178,6 +1193,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	using S = Store<STORE>;
 	constexpr int Q = L::Q;
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
+	grid_dependents_launch();
 	if (x >= p.nxp) return;
 	const int y = blockIdx.y, z = blockIdx.z;
 	const int nxp = p.nxp;
@@ -1222,6 +1238,9 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 		}
 	}
 
+	const int flag = p.flags[cell];
+	grid_dependency_wait();
+
 	float f[Q];
 	// p.idx32, odd steps: the cell's index for accesses to x - 1 and x + 1
 	// (periodic rows wrap)
@@ -1264,7 +1283,6 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 					  : 0.f;
 		}
 	}
-	const int flag = p.flags[cell];
 	const float por = (COLL == COLL_PSM || COLL == COLL_PSM_GUO || COLL == COLL_HLBM) ? p.por[cell] : 1.f;
 	float Fc[3] = {0.f, 0.f, 0.f};
 	if ((COLL == COLL_BGK_GUO || COLL == COLL_PSM_GUO) && p.force) {

@@ -11,6 +11,7 @@
 #include "sweep.cuh"
 #include "sweep_dispatch.cuh"
 #include "sweep_rows.cuh"
+#include "sweep_tile.cuh"
 
 namespace kel {
 namespace gb {
@@ -54,6 +55,23 @@ static cudaError_t launch_rows(const SweepParams &p, cudaStream_t st) {
 	return cudaGetLastError();
 }
 
+// A launch that may start while the one before it on the stream drains
+// (overlap; the kernel waits for it with grid_dependency_wait).
+template <class Kernel, class P>
+static cudaError_t launch_overlapped(Kernel kern, dim3 grid, int block, int smem, cudaStream_t st, bool overlap, const P &p) {
+	cudaLaunchAttribute at;
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = dim3(block);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cfg.attrs = &at;
+	cfg.numAttrs = overlap ? 1 : 0;
+	return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
 // One cell per thread: the grid, and the prefetch distance -- the block one
 // resident wave later (32 warps per SM at most: 1024 / block blocks on each
 // SM; measured at 256^3: D3Q19 FP32 0.92 -> 0.97 of HBM, FP16S 0.50 -> 0.55,
@@ -68,8 +86,7 @@ static cudaError_t launch_sweep1(SweepParams p, int block, cudaStream_t st) {
 	p.pf_z = ahead / (int)grid.x / (int)grid.y;
 	const int lines = block * (int)sizeof(typename Store<STORE>::T) / 128;
 	p.pf_shift = lines >= 8 ? 3 : (lines >= 4 ? 2 : (lines >= 2 ? 1 : 0));
-	sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW><<<grid, block, 0, st>>>(p);
-	return cudaGetLastError();
+	return launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW>, grid, block, 0, st, p.overlap != 0, p);
 }
 
 template <class L, int STORE, bool ODD, int COLL, bool EXACT>
@@ -125,6 +142,55 @@ cudaError_t launch_sweep_part(const SweepParams &p, bool odd, int coll, cudaStre
 	else
 		return odd ? launch_coll<L, STORE_FP16S, true, false>(p, coll, st)
 				   : launch_coll<L, STORE_FP16S, false, false>(p, coll, st);
+}
+
+// Lets a kernel use `bytes` of dynamic shared memory; the attribute is set to
+// the device's whole opt-in size once per kernel and device (`done`: bit per
+// device), so that no later call with a smaller footprint lowers it under
+// another thread.
+template <class Kernel>
+static cudaError_t allow_smem(Kernel kern, int bytes, std::atomic<uint64_t> &done) {
+	if (bytes <= 48 * 1024) return cudaSuccess;
+	int dev = 0, optin = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess) return e;
+	const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+	if (bit && (done.load() & bit)) return cudaSuccess;
+	if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+	if (bytes > optin) return cudaErrorInvalidConfiguration;
+	if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess) return e;
+	done.fetch_or(bit);
+	return cudaSuccess;
+}
+
+template <int STORE, int COLL, bool EXACT, class TS>
+static cudaError_t launch_tile_variant(const TileParams &q, cudaStream_t st) {
+	static std::atomic<uint64_t> done{0};
+	auto kern = sweep_tile_kernel<STORE, COLL, EXACT, TS>;
+	const int smem = tile_smem(TS::W, TS::K, q.ty, (int)sizeof(typename TileStore<STORE>::T));
+	cudaError_t e = allow_smem(kern, smem, done);
+	if (e != cudaSuccess) return e;
+	constexpr int TX = TS::W - 2 * TS::K;
+	const dim3 grid((q.p.nxp + TX - 1) / TX, (q.p.ny + q.ty - 1) / q.ty);
+	return launch_overlapped(kern, grid, TS::NT, smem, st, q.p.overlap != 0, q);
+}
+
+template <int PART>
+cudaError_t launch_tile_part(const TileParams &q, int coll, bool wide, cudaStream_t st) {
+	constexpr int STORE = PART == PART_FP16S ? STORE_FP16S : STORE_FP32;
+	constexpr bool EXACT = PART == PART_EXACT32;
+#define KEL_TILE(C)                                                                                                    \
+	case C:                                                                                                            \
+		return wide ? launch_tile_variant<STORE, C, EXACT, TileWide>(q, st)                                            \
+					: launch_tile_variant<STORE, C, EXACT, TileSmall>(q, st)
+	switch (coll) {
+		KEL_TILE(COLL_BGK);
+		KEL_TILE(COLL_BGK_GUO);
+		KEL_TILE(COLL_PSM);
+		KEL_TILE(COLL_PSM_GUO);
+	}
+#undef KEL_TILE
+	return cudaErrorInvalidValue;
 }
 
 } // namespace gb
