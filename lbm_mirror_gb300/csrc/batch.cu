@@ -18,11 +18,14 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "lattice_internal.cuh"
+#include "launch_util.cuh"
+#include "sweep_tile.cuh"
 
 using namespace kel::gb;
 
@@ -52,6 +55,17 @@ struct __align__(16) TileRec {
 	int live;      // channel still running
 };
 
+// One tile of the multi-step launches (sweep_tile.cuh): its place in a channel.
+struct __align__(16) StepTile {
+	int base;       // packed index of the channel's first cell
+	int nxp, ny;    // channel extents
+	int x0, y0, ty; // the tile's first cell within the channel, its rows
+	int ch;         // channel
+	float omega;
+	int prof_off;
+	int pad[3];
+};
+
 struct BatchParams {
 	TileRec *trec;   // per launched block
 	int *lfirst;     // per channel: index of its first tile in the launch list (-1: not launched)
@@ -71,6 +85,12 @@ struct BatchParams {
 	int shifted; // populations hold g = f - w_i (MODE_SHIFTED)
 	int idx32;   // 9 * plane < 2^31: population offsets from a cell fit 32-bit arithmetic
 	int pf_ahead; // launched blocks ahead whose tiles a block prefetches into L2 (0: none)
+	// multi-step tiles
+	const StepTile *tiles;
+	float *out;   // the other population array
+	int tile_ty;  // most rows of a tile
+	int off[9];   // index of a cell's slot in plane i
+	uint32_t plain, bounce; // as SweepParams::plain and bounce
 };
 
 // Arithmetic of a batch: the library's two (fast, reference rounding) on
@@ -87,8 +107,7 @@ enum { MODE_FAST = 0, MODE_EXACT = 1, MODE_SHIFTED = 2 };
 // keeps its linear updates (pairs of equal weight cancel) with the closure
 // sums taken on g (the weights of the summed populations add up to 1); BGK
 // relaxes g towards g_eq = w (rho - 1) + w rho (3 c.u + 4.5 (c.u)^2 - 1.5 u^2).
-__device__ __forceinline__ bool cell_update_shifted(float (&g)[9], int flag, int y, const CellCtx &p, float &rho,
-													float (&u)[3]) {
+__device__ __forceinline__ bool boundary_shifted(float (&g)[9], int flag, int y, const CellCtx &p) {
 	using L = D2Q9;
 	if (flag == 0) {
 #pragma unroll
@@ -154,7 +173,13 @@ __device__ __forceinline__ bool cell_update_shifted(float (&g)[9], int flag, int
 	default:
 		break;
 	}
-	if (!__ldg(&op->collide)) return false;
+	return __ldg(&op->collide) != 0;
+}
+
+// The fused multiply-adds are written out: the same bits from every kernel
+// that collides (k_batch_sweep, k_batch_tiles).
+__device__ __forceinline__ void collide_shifted(float (&g)[9], float omega, float &rho, float (&u)[3]) {
+	using L = D2Q9;
 	// moments on g: rho - 1 = sum g, rho u = sum c g
 	float drho = 0.f, jx = 0.f, jy = 0.f;
 #pragma unroll
@@ -167,18 +192,108 @@ __device__ __forceinline__ bool cell_update_shifted(float (&g)[9], int flag, int
 	}
 	rho = 1.0f + drho;
 	const float ir = 1.0f / rho;
-	u[0] = jx * ir;
-	u[1] = jy * ir;
+	u[0] = __fmul_rn(jx, ir);
+	u[1] = __fmul_rn(jy, ir);
 	u[2] = 0.f;
-	const float h = 1.5f * (u[0] * u[0] + u[1] * u[1]);
+	const float h = __fmul_rn(1.5f, __fmaf_rn(u[0], u[0], __fmul_rn(u[1], u[1])));
 #pragma unroll
 	for (int i = 0; i < 9; ++i) {
 		const float w = (float)L::w(i);
-		const float vcc = 3.f * ((float)L::cx(i) * u[0] + (float)L::cy(i) * u[1]);
-		const float geq = __fmaf_rn(w * rho, vcc + __fmaf_rn(0.5f * vcc, vcc, -h), w * drho);
-		g[i] = __fmaf_rn(p.omega, geq - g[i], g[i]);
+		const float vcc = __fmul_rn(3.f, __fadd_rn((float)L::cx(i) * u[0], (float)L::cy(i) * u[1]));
+		const float geq = __fmaf_rn(__fmul_rn(w, rho), __fadd_rn(vcc, __fmaf_rn(0.5f * vcc, vcc, -h)), __fmul_rn(w, drho));
+		g[i] = __fmaf_rn(omega, __fadd_rn(geq, -g[i]), g[i]);
 	}
+}
+
+__device__ __forceinline__ bool cell_update_shifted(float (&g)[9], int flag, int y, const CellCtx &p, float &rho,
+													float (&u)[3]) {
+	if (!boundary_shifted(g, flag, y, p)) return false;
+	collide_shifted(g, p.omega, rho, u);
 	return true;
+}
+
+// TILE_K steps of every listed tile (sweep_tile.cuh), channel by channel with
+// its own relaxation rate and inlet profile.
+__device__ __noinline__ Bounded tile_boundary_shifted(const OpEntry *ops, const float *profile, float f0, float f1,
+													  float f2, float f3, float f4, float f5, float f6, float f7,
+													  float f8, int flag, int y) {
+	float f[9] = {f0, f1, f2, f3, f4, f5, f6, f7, f8};
+	CellCtx ctx;
+	ctx.ops = ops;
+	ctx.profile = profile;
+	Bounded r;
+	r.collides = boundary_shifted(f, flag, y, ctx);
+#pragma unroll
+	for (int i = 0; i < 9; ++i) r.f[i] = f[i];
+	return r;
+}
+
+template <int MODE>
+struct ChannelCells {
+	const BatchParams &p;
+	const float *profile;
+	float omega;
+	__device__ __forceinline__ bool is_plain(int flag) const { return flag < MAX_FLAGS && ((p.plain >> flag) & 1u); }
+	__device__ __forceinline__ bool boundary(float (&f)[9], int flag, int y) const {
+		if (is_plain(flag)) return true;
+		const bool wall = flag < MAX_FLAGS && ((p.bounce >> flag) & 1u);
+		if (flag == 0 || wall) {
+			bounce_or_zero(f, wall);
+			return false;
+		}
+		const Bounded r = MODE == MODE_SHIFTED
+							  ? tile_boundary_shifted(p.ops, profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], flag, y)
+							  : tile_boundary<MODE == MODE_EXACT>(p.ops, profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6],
+																  f[7], f[8], flag, y);
+#pragma unroll
+		for (int i = 0; i < 9; ++i) f[i] = r.f[i];
+		return r.collides != 0;
+	}
+	template <int R>
+	__device__ __forceinline__ void cells(float (&f)[R][9], int, int) const {
+#pragma unroll
+			for (int k = 0; k < R; ++k) {
+				float rho, u[3];
+				if (MODE == MODE_SHIFTED) {
+					collide_shifted(f[k], omega, rho, u);
+				} else {
+					CellCtx ctx;
+					ctx.omega = omega;
+					const float Fc[3] = {0.f, 0.f, 0.f};
+					collide<D2Q9, COLL_BGK, MODE == MODE_EXACT>(f[k], ctx, 1.f, Fc, rho, u);
+				}
+			}
+	}
+};
+
+template <int MODE, class TS>
+__global__ void __launch_bounds__(TS::NT, TS::BPS) k_batch_tiles(const __grid_constant__ BatchParams p) {
+	extern __shared__ __align__(16) unsigned char tile_mem[];
+	grid_dependents_launch();
+	const StepTile t = p.tiles[blockIdx.x];
+	grid_dependency_wait(); // the residual pass may have stopped the channel
+	if (!p.active[t.ch]) return;
+	TileGeom g;
+	g.in = p.f;
+	g.out = p.out;
+#pragma unroll
+	for (int i = 0; i < 9; ++i) g.off[i] = p.off[i];
+	g.base = t.base;
+	g.nxp = t.nxp;
+	g.ny = t.ny;
+	g.periodic = 0;
+	g.x0 = t.x0 - TS::K;
+	g.y0 = t.y0 - TS::K;
+	const int left = t.ny - t.y0;
+	g.rows = min(t.ty, (left + TS::R - 1) / TS::R * TS::R) + 2 * TS::K;
+	g.t_end = min(t.ty, left) + TS::K;
+	g.flags = p.flags;
+	const int cells = (p.tile_ty + 2 * TS::K) * TS::W;
+	float *const sm = reinterpret_cast<float *>(tile_mem);
+	uint32_t *const bnd = reinterpret_cast<uint32_t *>(sm + 9 * cells);
+	uint8_t *const fl = reinterpret_cast<uint8_t *>(bnd + cells / 32);
+	tile_steps<STORE_FP32, TS>(g, [](int) { return 0.f; }, sm, bnd, fl,
+							   ChannelCells<MODE>{p, p.profiles + t.prof_off, t.omega});
 }
 
 template <bool ODD, int MODE>
@@ -544,6 +659,13 @@ struct kel_batch {
 	int *d_lfirst = nullptr;   // per channel: first launch index of its tiles, -1 if not launched
 	double2 *partial = nullptr;
 	double *d_residual = nullptr;
+	float *f2 = nullptr;         // second population array of the multi-step tiles
+	bool no_f2 = false;          // it could not be had
+	StepTile *d_tiles = nullptr; // tiles of the listed channels
+	int ntiles = 0, tile_ty = 0;
+	uint32_t plain = 0, bounce = 0;
+	float *staging = nullptr;    // downloads
+	int64_t staging_len = 0;
 	OpEntry *ops = nullptr;
 	bool have_ops = false;
 	kel_step_program prog;
@@ -570,6 +692,12 @@ void free_device(kel_batch *B) {
 	cudaFree(B->d_blist);
 	cudaFree(B->d_trec);
 	cudaFree(B->d_lfirst);
+	cudaFree(B->f2);
+	cudaFree(B->d_tiles);
+	B->f2 = nullptr;
+	B->no_f2 = false;
+	B->d_tiles = nullptr;
+	B->ntiles = 0;
 	B->d_trec = nullptr;
 	B->d_lfirst = nullptr;
 	cudaFree(B->d_active);
@@ -611,6 +739,12 @@ BatchParams params(const kel_batch *B, int write_macros) {
 	// prefetch the tiles one resident wave later (2048 threads per SM):
 	// measured with 1024 channels 0.82 -> 0.85 of HBM; two waves gained less
 	p.pf_ahead = B->sms * (2048 / (B->tile > 0 ? B->tile : 256));
+	p.tiles = B->d_tiles;
+	p.out = B->f2;
+	p.tile_ty = B->tile_ty;
+	for (int i = 0; i < 9; ++i) p.off[i] = (int)(i * B->plane); // used with 9 planes < 2^31 only
+	p.plain = B->plain;
+	p.bounce = B->bounce;
 	return p;
 }
 
@@ -636,6 +770,96 @@ int upload_tile_records(kel_batch *B) {
 	KEL_CUDA(cudaMemcpyAsync(B->d_lfirst, lf.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice, B->stream));
 	KEL_CUDA(cudaStreamSynchronize(B->stream));
 	return KEL_OK;
+}
+
+// Rows of a channel's tiles: the fewest passes of a block over its rows, all
+// tiles and steps together (a block covers 16 rows at once; the steps cover
+// ty + 8, 6, 4 and 2 rows).
+int tile_rows(int ny, int most_rows) {
+	constexpr int at_once = TileSmall::NT / TileSmall::W;
+	auto passes = [&](int ty) {
+		int n = 0;
+		for (int m = 0; m < TILE_K; ++m) n += (ty + 2 * (TILE_K - m) + at_once - 1) / at_once;
+		return n;
+	};
+	int best = 0, least = 0;
+	for (int ty = 4; ty <= most_rows; ty += 2) {
+		const int whole = ny / ty, rest = ny - whole * ty;
+		const int n = whole * passes(ty) + (rest ? passes(rest) : 0);
+		if (!best || n <= least) {
+			best = ty;
+			least = n;
+		}
+	}
+	return best;
+}
+
+// Multi-step tiles of the channels in the launch list (every channel in the
+// list is running).  Small tiles throughout: a channel is a few tiles wide, so
+// the wide ones spend their lanes beyond its end (192 channels of 64-512 x
+// 32-128, 4.5 M cells: small 51.6 us per step, wide 56.1, one step per launch
+// 58.0; 64 channels of 256x64: 13.9, 17.1, 16.9; 16 channels 6.2, 8.2, 9.3).
+// Below 700,000 cells tiles of at most 24 rows fill the device better (8
+// channels of 256x64: 4.2 us against 5.5), above it 40 rows redo less (192
+// channels: 51.6 against 58.8).
+int upload_step_tiles(kel_batch *B) {
+	std::vector<uint8_t> listed(B->n, 0);
+	int64_t cells = 0;
+	for (int k = 0; k < B->nlaunch; ++k) {
+		const int c = B->blist[k].y;
+		if (!listed[c]) cells += (int64_t)B->rec[c].nxp * B->rec[c].ny;
+		listed[c] = 1;
+	}
+	constexpr int tx = TileSmall::W - 2 * TILE_K;
+	std::vector<StepTile> tiles;
+	B->tile_ty = 0;
+	for (int c = 0; c < B->n; ++c) {
+		if (!listed[c]) continue;
+		const ChannelRec &r = B->rec[c];
+		const int ty = tile_rows(r.ny, cells < 700000 ? 24 : 40);
+		if (ty > B->tile_ty) B->tile_ty = ty;
+		for (int y0 = 0; y0 < r.ny; y0 += ty)
+			for (int x0 = 0; x0 < r.nxp; x0 += tx) {
+				StepTile t = {};
+				t.base = (int)r.off;
+				t.nxp = r.nxp;
+				t.ny = r.ny;
+				t.x0 = x0;
+				t.y0 = y0;
+				t.ty = ty;
+				t.ch = c;
+				t.omega = r.omega;
+				t.prof_off = r.prof_off;
+				tiles.push_back(t);
+			}
+	}
+	if ((int)tiles.size() > B->ntiles || !B->d_tiles) {
+		cudaFree(B->d_tiles);
+		B->d_tiles = nullptr;
+		KEL_CUDA(cudaMalloc(&B->d_tiles, sizeof(StepTile) * tiles.size()));
+	}
+	B->ntiles = (int)tiles.size();
+	KEL_CUDA(cudaMemcpyAsync(B->d_tiles, tiles.data(), sizeof(StepTile) * tiles.size(), cudaMemcpyHostToDevice, B->stream));
+	KEL_CUDA(cudaStreamSynchronize(B->stream));
+	return KEL_OK;
+}
+
+// The second population array and the tiles, on first use (a batch that would
+// not leave three quarters of the free memory to others runs without).
+bool ensure_tiles(kel_batch *B) {
+	if (9 * B->plane >= ((int64_t)1 << 31)) return false;
+	if (B->no_f2) return false;
+	if (!B->f2) {
+		const size_t bytes = sizeof(float) * 9 * (size_t)B->plane;
+		size_t free_b = 0, total_b = 0;
+		if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 || cudaMalloc(&B->f2, bytes) != cudaSuccess) {
+			cudaGetLastError();
+			B->f2 = nullptr;
+			B->no_f2 = true;
+			return false;
+		}
+	}
+	return B->d_tiles || upload_step_tiles(B) == KEL_OK;
 }
 
 // Lay the channels out in tiles of `tile` cells and allocate the device side.
@@ -744,6 +968,47 @@ cudaError_t launch_sweep_batch(const kel_batch *B, bool odd, int write_macros) {
 	return cudaGetLastError();
 }
 
+template <int MODE>
+cudaError_t launch_tiles(const kel_batch *B, const BatchParams &p) {
+	using TS = TileSmall;
+	static std::atomic<uint64_t> done{0};
+	auto kern = k_batch_tiles<MODE, TS>;
+	const int smem = tile_smem(TS::W, TS::K, B->tile_ty, sizeof(float));
+	cudaError_t e = allow_smem(kern, smem, done);
+	return e != cudaSuccess ? e : launch_overlapped(kern, dim3(B->ntiles), TS::NT, smem, B->stream, true, p);
+}
+
+// 2 TILE_K steps from an even one: into the second array and back.
+cudaError_t launch_tile_pair(const kel_batch *B) {
+	BatchParams p = params(B, 0);
+	for (int k = 0; k < 2; ++k) {
+		p.f = k ? B->f2 : B->f;
+		p.out = k ? B->f : B->f2;
+		cudaError_t e;
+		if (B->mode == MODE_EXACT) e = launch_tiles<MODE_EXACT>(B, p);
+		else if (B->mode == MODE_SHIFTED) e = launch_tiles<MODE_SHIFTED>(B, p);
+		else e = launch_tiles<MODE_FAST>(B, p);
+		if (e != cudaSuccess) return e;
+	}
+	return cudaSuccess;
+}
+
+// n steps from time step t, the last one writing the macros: tile pairs from
+// an even step, the others one by one.
+cudaError_t launch_steps(const kel_batch *B, uint64_t t, uint64_t n, bool tiled) {
+	cudaError_t e = cudaSuccess;
+	for (uint64_t s = 0; s < n && e == cudaSuccess;) {
+		if (tiled && ((t + s) & 1u) == 0 && n - s > 2 * TILE_K) { // the last step is none of theirs
+			e = launch_tile_pair(B);
+			s += 2 * TILE_K;
+		} else {
+			e = launch_sweep_batch(B, ((t + s) & 1u) != 0, s + 1 == n);
+			++s;
+		}
+	}
+	return e;
+}
+
 cudaError_t launch_residual(const kel_batch *B, double tol) {
 	BatchParams p = params(B, 0);
 	k_batch_residual_partial<<<B->nlaunch, B->tile, 0, B->stream>>>(p);
@@ -805,6 +1070,7 @@ extern "C" int kel_batch_destroy(kel_batch *B) {
 	if (!B) return KEL_OK;
 	cudaStreamSynchronize(B->stream);
 	free_device(B);
+	cudaFree(B->staging);
 	cudaFree(B->ops);
 	if (B->own_stream) cudaStreamDestroy(B->stream);
 	delete B;
@@ -848,6 +1114,11 @@ extern "C" int kel_batch_set_program(kel_batch *B, const kel_step_program *P) {
 		k_batch_shift<<<grid_for(B->plane), 256, 0, B->stream>>>(params(B, 0), shifted ? -1.f : 1.f);
 		KEL_CUDA(cudaGetLastError());
 	}
+	B->plain = B->bounce = 0;
+	for (int fl = 1; fl < MAX_FLAGS; ++fl) {
+		if ((ops[fl].bc == KEL_BC_NONE || ops[fl].bc == KEL_BC_FLUID) && ops[fl].collide) B->plain |= 1u << fl;
+		if (ops[fl].bc == KEL_BC_BOUNCE_BACK && !ops[fl].collide) B->bounce |= 1u << fl;
+	}
 	KEL_CUDA(cudaMemcpyAsync(B->ops, ops, sizeof(ops), cudaMemcpyHostToDevice, B->stream));
 	KEL_CUDA(cudaStreamSynchronize(B->stream));
 	B->prog = *P;
@@ -874,10 +1145,8 @@ extern "C" int kel_batch_step(kel_batch *B, uint64_t n_steps) {
 	uint64_t t = global_t(B);
 	for (int c = 0; c < B->n; ++c)
 		if (act[c] && B->t[c] != t) return fail(KEL_ERR_STATE, "kel_batch_step: channel time steps diverged");
-	for (uint64_t s = 0; s < n_steps; ++s) {
-		cudaError_t e = launch_sweep_batch(B, ((t + s) & 1u) != 0, s + 1 == n_steps);
-		if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_step: %s", cudaGetErrorString(e));
-	}
+	const cudaError_t e = launch_steps(B, t, n_steps, n_steps > 2 * TILE_K && ensure_tiles(B));
+	if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_step: %s", cudaGetErrorString(e));
 	for (int c = 0; c < B->n; ++c)
 		if (act[c]) B->t[c] += n_steps;
 	KEL_CUDA(cudaStreamSynchronize(B->stream));
@@ -901,6 +1170,7 @@ static int compact(kel_batch *B, const std::vector<int> &act) {
 	B->nlaunch = keep;
 	int rc = upload_tile_records(B);
 	if (rc) return rc;
+	if (B->d_tiles && (rc = upload_step_tiles(B))) return rc;
 	if (B->graph) cudaGraphExecDestroy(B->graph);
 	B->graph = nullptr;
 	return KEL_OK;
@@ -912,9 +1182,9 @@ static int build_graph(kel_batch *B, int check, double tol) {
 	if (B->graph) cudaGraphExecDestroy(B->graph);
 	B->graph = nullptr;
 	cudaGraph_t g;
+	const bool tiled = check > 2 * TILE_K && ensure_tiles(B); // no allocation inside the capture
 	KEL_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-	cudaError_t e = cudaSuccess;
-	for (int s = 0; s < check && e == cudaSuccess; ++s) e = launch_sweep_batch(B, (s & 1) != 0, s + 1 == check);
+	cudaError_t e = launch_steps(B, 0, (uint64_t)check, tiled);
 	if (e == cudaSuccess) e = launch_residual(B, tol);
 	cudaError_t e2 = cudaStreamEndCapture(B->stream, &g);
 	if (e != cudaSuccess || e2 != cudaSuccess)
@@ -949,11 +1219,8 @@ extern "C" int kel_batch_run_until(kel_batch *B, double tol, uint64_t check_ever
 		if (use_graph) {
 			KEL_CUDA(cudaGraphLaunch(B->graph, B->stream));
 		} else {
-			for (uint64_t s = 0; s < check_every; ++s) {
-				cudaError_t e = launch_sweep_batch(B, (s & 1u) != 0, s + 1 == check_every);
-				if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_run_until: %s", cudaGetErrorString(e));
-			}
-			cudaError_t e = launch_residual(B, tol);
+			cudaError_t e = launch_steps(B, 0, check_every, check_every > 2 * TILE_K && ensure_tiles(B));
+			if (e == cudaSuccess) e = launch_residual(B, tol);
 			if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_run_until: %s", cudaGetErrorString(e));
 		}
 		done += check_every;
@@ -989,14 +1256,21 @@ static int batch_download(kel_batch *B, int32_t channel, int what, float *host) 
 		return fail(KEL_ERR_INVALID_ARGUMENT, "kel_batch_download: bad arguments");
 	const ChannelRec ch = B->rec[channel];
 	const int64_t n = (int64_t)ch.nx * ch.ny * (what == 0 ? 9 : 3);
-	float *d = nullptr;
-	KEL_CUDA(cudaMalloc(&d, sizeof(float) * n));
+	// the staging buffer is kept (it grows to the largest channel read): an
+	// allocation and a free per call cost up to 100 us, by what else holds the
+	// driver's chunks
+	if (B->staging_len < n) {
+		cudaFree(B->staging);
+		B->staging = nullptr;
+		B->staging_len = 0;
+		KEL_CUDA(cudaMalloc(&B->staging, sizeof(float) * n));
+		B->staging_len = n;
+	}
 	k_batch_download<<<grid_for((int64_t)ch.nx * ch.ny), 256, 0, B->stream>>>(params(B, 0), ch, (int)(B->t[channel] & 1u),
-																			  what, d);
+																			  what, B->staging);
 	cudaError_t e = cudaGetLastError();
-	if (e == cudaSuccess) e = cudaMemcpyAsync(host, d, sizeof(float) * n, cudaMemcpyDeviceToHost, B->stream);
+	if (e == cudaSuccess) e = cudaMemcpyAsync(host, B->staging, sizeof(float) * n, cudaMemcpyDeviceToHost, B->stream);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
-	cudaFree(d);
 	if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_download: %s", cudaGetErrorString(e));
 	return KEL_OK;
 }

@@ -108,7 +108,9 @@ __device__ __forceinline__ void collide_bgk2(float (&fa)[9], float (&fb)[9], flo
 	}
 	const float2 ir = make_float2(__frcp_rn(r.x), __frcp_rn(r.y));
 	const float2 ux = __fmul2_rn(jx, ir), uy = __fmul2_rn(jy, ir);
-	const float2 vv = __fadd2_rn(__fmul2_rn(ux, ux), __fmul2_rn(uy, uy));
+	// scalar: the compiler fuses a two-wide product into a two-wide sum
+	const float2 vv = make_float2(__fadd_rn(__fmul_rn(ux.x, ux.x), __fmul_rn(uy.x, uy.x)),
+								  __fadd_rn(__fmul_rn(ux.y, ux.y), __fmul_rn(uy.y, uy.y)));
 	const float2 nh = __fmul2_rn(both(-1.5f), vv), om = both(omega);
 	auto relax = [&](float2 v, float2 eq) { return __ffma2_rn(om, __fadd2_rn(eq, neg2(v)), v); };
 	const float2 w0 = __fmul2_rn(both((float)L::w(0)), r);
@@ -127,6 +129,17 @@ __device__ __forceinline__ void collide_bgk2(float (&fa)[9], float (&fb)[9], flo
 		fa[i] = f[i].x;
 		fb[i] = f[i].y;
 	}
+}
+
+// A wall cell's full-way bounce-back, or (not a wall) a cell outside the lattice.
+__device__ __forceinline__ void bounce_or_zero(float (&f)[9], bool wall) {
+#pragma unroll
+	for (int i = 1; i < 9; i += 2) { // opp(i) = i + 1
+		const float t = f[i];
+		f[i] = wall ? f[i + 1] : 0.f;
+		f[i + 1] = wall ? t : 0.f;
+	}
+	f[0] = wall ? f[0] : 0.f;
 }
 
 // A cell's populations after its boundary step, and whether it collides then.
@@ -287,17 +300,10 @@ struct LatticeCells {
 	const SweepParams &p;
 	__device__ __forceinline__ bool is_plain(int flag) const { return flag < MAX_FLAGS && ((p.plain >> flag) & 1u); }
 	__device__ __forceinline__ bool boundary(float (&f)[9], int flag, int y) const {
-		using L = D2Q9;
 		if (is_plain(flag)) return true;
 		const bool wall = flag < MAX_FLAGS && ((p.bounce >> flag) & 1u);
 		if (flag == 0 || wall) {
-#pragma unroll
-			for (int i = 1; i < 9; i += 2) { // opp(i) = i + 1
-				const float t = f[i];
-				f[i] = wall ? f[i + 1] : 0.f;
-				f[i + 1] = wall ? t : 0.f;
-			}
-			f[0] = wall ? f[0] : 0.f;
+			bounce_or_zero(f, wall);
 			return false;
 		}
 		const Bounded r = tile_boundary<EXACT>(p.ops, p.profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], flag, y);

