@@ -18,14 +18,12 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "lattice_internal.cuh"
 #include "launch_util.cuh"
-#include "sweep_tile.cuh"
 
 using namespace kel::gb;
 
@@ -41,7 +39,7 @@ struct ChannelRec {
 	float guo_scale; // 1 - omega / 2
 };
 
-// What one launched block of the sweep needs, in one 32-byte record read at
+// What one launched block of the sweep needs, in one 48-byte record read at
 // the block's start (the block's tile and its channel's extents, relaxation
 // rate and inlet profile), so that its population loads follow a single
 // load instead of a chain (launch list -> channel record).  `live` drops to
@@ -53,16 +51,7 @@ struct __align__(16) TileRec {
 	float omega;   // channel relaxation rate
 	int prof_off;  // channel inlet profile offset
 	int live;      // channel still running
-};
-
-// One tile of the multi-step launches (sweep_tile.cuh): its place in a channel.
-struct __align__(16) StepTile {
-	int base;       // packed index of the channel's first cell
-	int nxp, ny;    // channel extents
-	int x0, y0, ty; // the tile's first cell within the channel, its rows
-	int ch;         // channel
-	float omega;
-	int prof_off;
+	uint32_t by_nxp; // floor(l / nxp) = l * by_nxp / 2^32 for the channel's cells l; 0: divide
 	int pad[3];
 };
 
@@ -85,12 +74,8 @@ struct BatchParams {
 	int shifted; // populations hold g = f - w_i (MODE_SHIFTED)
 	int idx32;   // 9 * plane < 2^31: population offsets from a cell fit 32-bit arithmetic
 	int pf_ahead; // launched blocks ahead whose tiles a block prefetches into L2 (0: none)
-	// multi-step tiles
-	const StepTile *tiles;
-	float *out;   // the other population array
-	int tile_ty;  // most rows of a tile
-	int off[9];   // index of a cell's slot in plane i
-	uint32_t plain, bounce; // as SweepParams::plain and bounce
+	int off[9];     // idx32: index of a cell's slot in plane i
+	uint32_t plain; // as SweepParams::plain
 };
 
 // Arithmetic of a batch: the library's two (fast, reference rounding) on
@@ -176,8 +161,8 @@ __device__ __forceinline__ bool boundary_shifted(float (&g)[9], int flag, int y,
 	return __ldg(&op->collide) != 0;
 }
 
-// The fused multiply-adds are written out: the same bits from every kernel
-// that collides (k_batch_sweep, k_batch_tiles).
+// The multiply-adds are written out, so that no choice of the compiler's
+// changes the bits.
 __device__ __forceinline__ void collide_shifted(float (&g)[9], float omega, float &rho, float (&u)[3]) {
 	using L = D2Q9;
 	// moments on g: rho - 1 = sum g, rho u = sum c g
@@ -212,135 +197,71 @@ __device__ __forceinline__ bool cell_update_shifted(float (&g)[9], int flag, int
 	return true;
 }
 
-// TILE_K steps of every listed tile (sweep_tile.cuh), channel by channel with
-// its own relaxation rate and inlet profile.
-__device__ __noinline__ Bounded tile_boundary_shifted(const OpEntry *ops, const float *profile, float f0, float f1,
-													  float f2, float f3, float f4, float f5, float f6, float f7,
-													  float f8, int flag, int y) {
-	float f[9] = {f0, f1, f2, f3, f4, f5, f6, f7, f8};
-	CellCtx ctx;
-	ctx.ops = ops;
-	ctx.profile = profile;
-	Bounded r;
-	r.collides = boundary_shifted(f, flag, y, ctx);
-#pragma unroll
-	for (int i = 0; i < 9; ++i) r.f[i] = f[i];
-	return r;
-}
-
-template <int MODE>
-struct ChannelCells {
-	const BatchParams &p;
-	const float *profile;
-	float omega;
-	__device__ __forceinline__ bool is_plain(int flag) const { return flag < MAX_FLAGS && ((p.plain >> flag) & 1u); }
-	__device__ __forceinline__ bool boundary(float (&f)[9], int flag, int y) const {
-		if (is_plain(flag)) return true;
-		const bool wall = flag < MAX_FLAGS && ((p.bounce >> flag) & 1u);
-		if (flag == 0 || wall) {
-			bounce_or_zero(f, wall);
-			return false;
-		}
-		const Bounded r = MODE == MODE_SHIFTED
-							  ? tile_boundary_shifted(p.ops, profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], flag, y)
-							  : tile_boundary<MODE == MODE_EXACT>(p.ops, profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6],
-																  f[7], f[8], flag, y);
-#pragma unroll
-		for (int i = 0; i < 9; ++i) f[i] = r.f[i];
-		return r.collides != 0;
-	}
-	template <int R>
-	__device__ __forceinline__ void cells(float (&f)[R][9], int, int) const {
-#pragma unroll
-			for (int k = 0; k < R; ++k) {
-				float rho, u[3];
-				if (MODE == MODE_SHIFTED) {
-					collide_shifted(f[k], omega, rho, u);
-				} else {
-					CellCtx ctx;
-					ctx.omega = omega;
-					const float Fc[3] = {0.f, 0.f, 0.f};
-					collide<D2Q9, COLL_BGK, MODE == MODE_EXACT>(f[k], ctx, 1.f, Fc, rho, u);
-				}
-			}
-	}
-};
-
-template <int MODE, class TS>
-__global__ void __launch_bounds__(TS::NT, TS::BPS) k_batch_tiles(const __grid_constant__ BatchParams p) {
-	extern __shared__ __align__(16) unsigned char tile_mem[];
-	grid_dependents_launch();
-	const StepTile t = p.tiles[blockIdx.x];
-	grid_dependency_wait(); // the residual pass may have stopped the channel
-	if (!p.active[t.ch]) return;
-	TileGeom g;
-	g.in = p.f;
-	g.out = p.out;
-#pragma unroll
-	for (int i = 0; i < 9; ++i) g.off[i] = p.off[i];
-	g.base = t.base;
-	g.nxp = t.nxp;
-	g.ny = t.ny;
-	g.periodic = 0;
-	g.x0 = t.x0 - TS::K;
-	g.y0 = t.y0 - TS::K;
-	const int left = t.ny - t.y0;
-	g.rows = min(t.ty, (left + TS::R - 1) / TS::R * TS::R) + 2 * TS::K;
-	g.t_end = min(t.ty, left) + TS::K;
-	g.flags = p.flags;
-	const int cells = (p.tile_ty + 2 * TS::K) * TS::W;
-	float *const sm = reinterpret_cast<float *>(tile_mem);
-	uint32_t *const bnd = reinterpret_cast<uint32_t *>(sm + 9 * cells);
-	uint8_t *const fl = reinterpret_cast<uint8_t *>(bnd + cells / 32);
-	tile_steps<STORE_FP32, TS>(g, [](int) { return 0.f; }, sm, bnd, fl,
-							   ChannelCells<MODE>{p, p.profiles + t.prof_off, t.omega});
-}
-
+// One step of the listed tiles.  What bounds it is HBM for batches beyond the
+// L2 and instruction issue otherwise: the index tables, the row found without
+// a division and one path per warp (all cells interior, or predicated) took
+// 343 / 447 instructions per cell (even / odd step) to 258 / 317; launches of
+// a run overlap (grid_dependency_wait).  Measured, per step: 64 channels of
+// 256x64 15.5 -> 11.5 us, 192 channels of 64-512 x 32-128 58 -> 52 us (0.94 of
+// measured HBM).  Tiles of four steps in shared memory (sweep_tile.cuh) were
+// no faster: 15.2 and 51.6 us.
 template <bool ODD, int MODE>
 __global__ void __launch_bounds__(512, MODE == MODE_EXACT ? 1 : 4) k_batch_sweep(const __grid_constant__ BatchParams p) {
 	using L = D2Q9;
+	grid_dependents_launch();
+	// the records are written before the first sweep of a run starts, and only
+	// that sweep may directly follow the residual pass (launch_steps)
 	const int4 *tr = reinterpret_cast<const int4 *>(p.trec + blockIdx.x);
 	const int4 r0 = __ldg(tr), r1 = __ldg(tr + 1);
-	TileRec ch;
-	ch.cell0 = (int64_t)(((uint64_t)(uint32_t)r0.y << 32) | (uint32_t)r0.x);
-	ch.l0 = r0.z;
-	ch.nxp = r0.w;
-	ch.ny = r1.x;
-	ch.omega = __int_as_float(r1.y);
-	ch.prof_off = r1.z;
+	const uint32_t by_nxp = __ldg(reinterpret_cast<const uint32_t *>(tr + 2));
+	const int64_t cell0 = (int64_t)(((uint64_t)(uint32_t)r0.y << 32) | (uint32_t)r0.x);
+	const int l0 = r0.z, nxp = r0.w, ny = r1.x;
 	if (!r1.w) return; // converged channel
-	const int l = ch.l0 + (int)threadIdx.x;
-	if (l >= ch.nxp * ch.ny) return;
-	const int y = l / ch.nxp, x = l - y * ch.nxp;
-	const int64_t cell = ch.cell0 + threadIdx.x;
-	const int64_t ch_off = ch.cell0 - ch.l0; // the channel's first cell
-	// interior cells: every neighbour inside the channel, offsets from the
-	// cell in 32-bit arithmetic
-	const bool fast = p.idx32 && x > 0 && x + 1 < ch.nxp && y > 0 && y + 1 < ch.ny;
-	const float *const fc = p.f + cell;
-	const int pl32 = static_cast<int>(p.plane), nxp = ch.nxp;
+	const int l = l0 + (int)threadIdx.x;
+	if (l >= nxp * ny) return;
+	const int y = by_nxp ? (int)__umulhi((unsigned)l, by_nxp) : l / nxp, x = l - y * nxp;
+	const int64_t cell = cell0 + threadIdx.x;
+	const int flag = p.flags[cell];
+	const unsigned lanes = __activemask(); // a channel's last tile may be partial
+	const bool has_xm = x > 0, has_xp = x + 1 < nxp, has_ym = y > 0, has_yp = y + 1 < ny;
+	const bool inner = __all_sync(lanes, has_xm && has_xp && has_ym && has_yp);
+	auto has = [&](int cx, int cy) { // the neighbour x + c exists
+		return (cx > 0 ? has_xp : (cx < 0 ? has_xm : true)) && (cy > 0 ? has_yp : (cy < 0 ? has_ym : true));
+	};
+	// p.idx32: index of the cell, of the one above and of the one below, in plane 0
+	const int c32 = (int)cell, c_up = c32 + nxp, c_dn = c32 - nxp;
+	auto row = [&](int cy) { return cy > 0 ? c_up : (cy < 0 ? c_dn : c32); };
+	grid_dependency_wait();
+
 	float f[9];
-	if (fast) {
-#pragma unroll
-		for (int i = 0; i < 9; ++i)
-			f[i] = ODD ? __ldcs(fc + (L::opp(i) * pl32 - L::cx(i) - L::cy(i) * nxp)) : __ldcs(fc + i * pl32);
-	} else {
+	if (!p.idx32) {
+		const int64_t ch_off = cell0 - l0; // the channel's first cell
 #pragma unroll
 		for (int i = 0; i < 9; ++i) {
 			if (!ODD) {
 				f[i] = __ldcs(p.f + i * p.plane + cell);
 			} else {
-				const int sx = x - L::cx(i), sy = y - L::cy(i);
-				const bool in = sx >= 0 && sx < ch.nxp && sy >= 0 && sy < ch.ny;
-				f[i] = in ? __ldcs(p.f + L::opp(i) * p.plane + ch_off + sy * ch.nxp + sx) : 0.f;
+				f[i] = has(-L::cx(i), -L::cy(i))
+						   ? __ldcs(p.f + L::opp(i) * p.plane + ch_off + (int64_t)(y - L::cy(i)) * nxp + (x - L::cx(i)))
+						   : 0.f;
 			}
 		}
+	} else if (!ODD) {
+#pragma unroll
+		for (int i = 0; i < 9; ++i) f[i] = __ldcs(p.f + (c32 + p.off[i]));
+	} else if (inner) {
+#pragma unroll
+		for (int i = 0; i < 9; ++i) f[i] = __ldcs(p.f + (row(-L::cy(i)) + p.off[L::opp(i)]) - L::cx(i));
+	} else {
+#pragma unroll
+		for (int i = 0; i < 9; ++i)
+			f[i] = has(-L::cx(i), -L::cy(i)) ? __ldcs(p.f + (row(-L::cy(i)) + p.off[L::opp(i)]) - L::cx(i)) : 0.f;
 	}
 	CellCtx ctx;
 	ctx.ops = p.ops;
-	ctx.profile = p.profiles + ch.prof_off;
-	ctx.omega = ch.omega;
-	ctx.guo_scale = 1.0f - 0.5f * ch.omega; // unused by BGK
+	ctx.profile = p.profiles + r1.z;
+	ctx.omega = __int_as_float(r1.y);
+	ctx.guo_scale = 1.0f - 0.5f * ctx.omega; // unused by BGK
 	ctx.g[0] = ctx.g[1] = ctx.g[2] = 0.f;
 	const float Fc[3] = {0.f, 0.f, 0.f};
 	float rho = 1.f, u[3] = {0.f, 0.f, 0.f};
@@ -360,31 +281,42 @@ __global__ void __launch_bounds__(512, MODE == MODE_EXACT ? 1 : 4) k_batch_sweep
 			}
 		}
 	}
-	const bool col = MODE == MODE_SHIFTED
-						 ? cell_update_shifted(f, p.flags[cell], y, ctx, rho, u)
-						 : cell_update<L, COLL_BGK, MODE == MODE_EXACT>(f, p.flags[cell], y, ctx, 1.f, Fc, rho, u);
+	bool col = true;
+	if (__all_sync(lanes, flag < MAX_FLAGS && ((p.plain >> flag) & 1u))) { // no boundary step: straight to the collision
+		if (MODE == MODE_SHIFTED) collide_shifted(f, ctx.omega, rho, u);
+		else collide<L, COLL_BGK, MODE == MODE_EXACT>(f, ctx, 1.f, Fc, rho, u);
+	} else {
+		col = MODE == MODE_SHIFTED ? cell_update_shifted(f, flag, y, ctx, rho, u)
+								   : cell_update<L, COLL_BGK, MODE == MODE_EXACT>(f, flag, y, ctx, 1.f, Fc, rho, u);
+	}
 	if (p.write_macros && col) {
 		p.rho[cell] = rho;
 		p.u[cell] = u[0];
 		p.u[p.plane + cell] = u[1];
 	}
-	float *const fw = p.f + cell;
-	if (fast) {
+	if (!p.idx32) {
+		const int64_t ch_off = cell0 - l0;
 #pragma unroll
-		for (int i = 0; i < 9; ++i)
-			__stcs(fw + (ODD ? i * pl32 + L::cx(i) + L::cy(i) * nxp : L::opp(i) * pl32), f[i]);
-		return;
-	}
+		for (int i = 0; i < 9; ++i) {
+			if (!ODD) {
+				__stcs(p.f + L::opp(i) * p.plane + cell, f[i]);
+			} else {
+				float *const pl = p.f + i * p.plane;
+				if (!has(-L::cx(i), -L::cy(i))) __stcs(pl + cell, 0.f);
+				if (has(L::cx(i), L::cy(i))) __stcs(pl + ch_off + (int64_t)(y + L::cy(i)) * nxp + (x + L::cx(i)), f[i]);
+			}
+		}
+	} else if (!ODD) {
 #pragma unroll
-	for (int i = 0; i < 9; ++i) {
-		if (!ODD) {
-			__stcs(p.f + L::opp(i) * p.plane + cell, f[i]);
-		} else {
-			const int64_t pb = static_cast<int64_t>(i) * p.plane;
-			const int sx = x - L::cx(i), sy = y - L::cy(i);
-			if (sx < 0 || sx >= ch.nxp || sy < 0 || sy >= ch.ny) __stcs(p.f + pb + cell, 0.f);
-			const int dx = x + L::cx(i), dy = y + L::cy(i);
-			if (dx >= 0 && dx < ch.nxp && dy >= 0 && dy < ch.ny) __stcs(p.f + pb + ch_off + dy * ch.nxp + dx, f[i]);
+		for (int i = 0; i < 9; ++i) __stcs(p.f + (c32 + p.off[L::opp(i)]), f[i]);
+	} else if (inner) {
+#pragma unroll
+		for (int i = 0; i < 9; ++i) __stcs(p.f + (row(L::cy(i)) + p.off[i]) + L::cx(i), f[i]);
+	} else {
+#pragma unroll
+		for (int i = 0; i < 9; ++i) {
+			if (!has(-L::cx(i), -L::cy(i))) __stcs(p.f + (c32 + p.off[i]), 0.f); // the ghost ring's zero
+			if (has(L::cx(i), L::cy(i))) __stcs(p.f + (row(L::cy(i)) + p.off[i]) + L::cx(i), f[i]);
 		}
 	}
 }
@@ -659,11 +591,7 @@ struct kel_batch {
 	int *d_lfirst = nullptr;   // per channel: first launch index of its tiles, -1 if not launched
 	double2 *partial = nullptr;
 	double *d_residual = nullptr;
-	float *f2 = nullptr;         // second population array of the multi-step tiles
-	bool no_f2 = false;          // it could not be had
-	StepTile *d_tiles = nullptr; // tiles of the listed channels
-	int ntiles = 0, tile_ty = 0;
-	uint32_t plain = 0, bounce = 0;
+	uint32_t plain = 0; // SweepParams::plain of the program
 	float *staging = nullptr;    // downloads
 	int64_t staging_len = 0;
 	OpEntry *ops = nullptr;
@@ -692,12 +620,6 @@ void free_device(kel_batch *B) {
 	cudaFree(B->d_blist);
 	cudaFree(B->d_trec);
 	cudaFree(B->d_lfirst);
-	cudaFree(B->f2);
-	cudaFree(B->d_tiles);
-	B->f2 = nullptr;
-	B->no_f2 = false;
-	B->d_tiles = nullptr;
-	B->ntiles = 0;
 	B->d_trec = nullptr;
 	B->d_lfirst = nullptr;
 	cudaFree(B->d_active);
@@ -739,12 +661,8 @@ BatchParams params(const kel_batch *B, int write_macros) {
 	// prefetch the tiles one resident wave later (2048 threads per SM):
 	// measured with 1024 channels 0.82 -> 0.85 of HBM; two waves gained less
 	p.pf_ahead = B->sms * (2048 / (B->tile > 0 ? B->tile : 256));
-	p.tiles = B->d_tiles;
-	p.out = B->f2;
-	p.tile_ty = B->tile_ty;
-	for (int i = 0; i < 9; ++i) p.off[i] = (int)(i * B->plane); // used with 9 planes < 2^31 only
+	for (int i = 0; i < 9; ++i) p.off[i] = p.idx32 ? (int)(i * B->plane) : 0;
 	p.plain = B->plain;
-	p.bounce = B->bounce;
 	return p;
 }
 
@@ -765,101 +683,16 @@ int upload_tile_records(kel_batch *B) {
 		t.omega = r.omega;
 		t.prof_off = r.prof_off;
 		t.live = 1;
+		// exact where l (by_nxp nxp - 2^32) < 2^32; the factor is at most nxp
+		t.by_nxp = r.nxp > 1 && (int64_t)r.nxp * r.nxp * r.ny < ((int64_t)1 << 32)
+					   ? (uint32_t)((((uint64_t)1 << 32) + (uint64_t)r.nxp - 1) / (uint64_t)r.nxp)
+					   : 0u;
+		t.pad[0] = t.pad[1] = t.pad[2] = 0;
 	}
 	KEL_CUDA(cudaMemcpyAsync(B->d_trec, tr.data(), sizeof(TileRec) * B->nlaunch, cudaMemcpyHostToDevice, B->stream));
 	KEL_CUDA(cudaMemcpyAsync(B->d_lfirst, lf.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice, B->stream));
 	KEL_CUDA(cudaStreamSynchronize(B->stream));
 	return KEL_OK;
-}
-
-// Rows of a channel's tiles: the fewest passes of a block over its rows, all
-// tiles and steps together (a block covers 16 rows at once; the steps cover
-// ty + 8, 6, 4 and 2 rows).
-int tile_rows(int ny, int most_rows) {
-	constexpr int at_once = TileSmall::NT / TileSmall::W;
-	auto passes = [&](int ty) {
-		int n = 0;
-		for (int m = 0; m < TILE_K; ++m) n += (ty + 2 * (TILE_K - m) + at_once - 1) / at_once;
-		return n;
-	};
-	int best = 0, least = 0;
-	for (int ty = 4; ty <= most_rows; ty += 2) {
-		const int whole = ny / ty, rest = ny - whole * ty;
-		const int n = whole * passes(ty) + (rest ? passes(rest) : 0);
-		if (!best || n <= least) {
-			best = ty;
-			least = n;
-		}
-	}
-	return best;
-}
-
-// Multi-step tiles of the channels in the launch list (every channel in the
-// list is running).  Small tiles throughout: a channel is a few tiles wide, so
-// the wide ones spend their lanes beyond its end (192 channels of 64-512 x
-// 32-128, 4.5 M cells: small 51.6 us per step, wide 56.1, one step per launch
-// 58.0; 64 channels of 256x64: 13.9, 17.1, 16.9; 16 channels 6.2, 8.2, 9.3).
-// Below 700,000 cells tiles of at most 24 rows fill the device better (8
-// channels of 256x64: 4.2 us against 5.5), above it 40 rows redo less (192
-// channels: 51.6 against 58.8).
-int upload_step_tiles(kel_batch *B) {
-	std::vector<uint8_t> listed(B->n, 0);
-	int64_t cells = 0;
-	for (int k = 0; k < B->nlaunch; ++k) {
-		const int c = B->blist[k].y;
-		if (!listed[c]) cells += (int64_t)B->rec[c].nxp * B->rec[c].ny;
-		listed[c] = 1;
-	}
-	constexpr int tx = TileSmall::W - 2 * TILE_K;
-	std::vector<StepTile> tiles;
-	B->tile_ty = 0;
-	for (int c = 0; c < B->n; ++c) {
-		if (!listed[c]) continue;
-		const ChannelRec &r = B->rec[c];
-		const int ty = tile_rows(r.ny, cells < 700000 ? 24 : 40);
-		if (ty > B->tile_ty) B->tile_ty = ty;
-		for (int y0 = 0; y0 < r.ny; y0 += ty)
-			for (int x0 = 0; x0 < r.nxp; x0 += tx) {
-				StepTile t = {};
-				t.base = (int)r.off;
-				t.nxp = r.nxp;
-				t.ny = r.ny;
-				t.x0 = x0;
-				t.y0 = y0;
-				t.ty = ty;
-				t.ch = c;
-				t.omega = r.omega;
-				t.prof_off = r.prof_off;
-				tiles.push_back(t);
-			}
-	}
-	if ((int)tiles.size() > B->ntiles || !B->d_tiles) {
-		cudaFree(B->d_tiles);
-		B->d_tiles = nullptr;
-		KEL_CUDA(cudaMalloc(&B->d_tiles, sizeof(StepTile) * tiles.size()));
-	}
-	B->ntiles = (int)tiles.size();
-	KEL_CUDA(cudaMemcpyAsync(B->d_tiles, tiles.data(), sizeof(StepTile) * tiles.size(), cudaMemcpyHostToDevice, B->stream));
-	KEL_CUDA(cudaStreamSynchronize(B->stream));
-	return KEL_OK;
-}
-
-// The second population array and the tiles, on first use (a batch that would
-// not leave three quarters of the free memory to others runs without).
-bool ensure_tiles(kel_batch *B) {
-	if (9 * B->plane >= ((int64_t)1 << 31)) return false;
-	if (B->no_f2) return false;
-	if (!B->f2) {
-		const size_t bytes = sizeof(float) * 9 * (size_t)B->plane;
-		size_t free_b = 0, total_b = 0;
-		if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 || cudaMalloc(&B->f2, bytes) != cudaSuccess) {
-			cudaGetLastError();
-			B->f2 = nullptr;
-			B->no_f2 = true;
-			return false;
-		}
-	}
-	return B->d_tiles || upload_step_tiles(B) == KEL_OK;
 }
 
 // Lay the channels out in tiles of `tile` cells and allocate the device side.
@@ -949,63 +782,25 @@ int layout(kel_batch *B, int tile) {
 	return KEL_OK;
 }
 
-cudaError_t launch_sweep_batch(const kel_batch *B, bool odd, int write_macros) {
-	BatchParams p = params(B, write_macros);
-	const dim3 g(B->nlaunch), b(B->tile);
+// overlap: the launch before on the stream is a sweep or tile launch of the
+// same run (see k_batch_sweep)
+cudaError_t launch_sweep_batch(const kel_batch *B, bool odd, int write_macros, bool overlap = false) {
+	const BatchParams p = params(B, write_macros);
+	const dim3 g(B->nlaunch);
+	auto go = [&](auto kern) { return launch_overlapped(kern, g, B->tile, 0, B->stream, overlap, p); };
 	switch (B->mode) {
-	case MODE_EXACT:
-		if (odd) k_batch_sweep<true, MODE_EXACT><<<g, b, 0, B->stream>>>(p);
-		else k_batch_sweep<false, MODE_EXACT><<<g, b, 0, B->stream>>>(p);
-		break;
-	case MODE_SHIFTED:
-		if (odd) k_batch_sweep<true, MODE_SHIFTED><<<g, b, 0, B->stream>>>(p);
-		else k_batch_sweep<false, MODE_SHIFTED><<<g, b, 0, B->stream>>>(p);
-		break;
-	default:
-		if (odd) k_batch_sweep<true, MODE_FAST><<<g, b, 0, B->stream>>>(p);
-		else k_batch_sweep<false, MODE_FAST><<<g, b, 0, B->stream>>>(p);
+	case MODE_EXACT: return odd ? go(k_batch_sweep<true, MODE_EXACT>) : go(k_batch_sweep<false, MODE_EXACT>);
+	case MODE_SHIFTED: return odd ? go(k_batch_sweep<true, MODE_SHIFTED>) : go(k_batch_sweep<false, MODE_SHIFTED>);
+	default: return odd ? go(k_batch_sweep<true, MODE_FAST>) : go(k_batch_sweep<false, MODE_FAST>);
 	}
-	return cudaGetLastError();
 }
 
-template <int MODE>
-cudaError_t launch_tiles(const kel_batch *B, const BatchParams &p) {
-	using TS = TileSmall;
-	static std::atomic<uint64_t> done{0};
-	auto kern = k_batch_tiles<MODE, TS>;
-	const int smem = tile_smem(TS::W, TS::K, B->tile_ty, sizeof(float));
-	cudaError_t e = allow_smem(kern, smem, done);
-	return e != cudaSuccess ? e : launch_overlapped(kern, dim3(B->ntiles), TS::NT, smem, B->stream, true, p);
-}
-
-// 2 TILE_K steps from an even one: into the second array and back.
-cudaError_t launch_tile_pair(const kel_batch *B) {
-	BatchParams p = params(B, 0);
-	for (int k = 0; k < 2; ++k) {
-		p.f = k ? B->f2 : B->f;
-		p.out = k ? B->f : B->f2;
-		cudaError_t e;
-		if (B->mode == MODE_EXACT) e = launch_tiles<MODE_EXACT>(B, p);
-		else if (B->mode == MODE_SHIFTED) e = launch_tiles<MODE_SHIFTED>(B, p);
-		else e = launch_tiles<MODE_FAST>(B, p);
-		if (e != cudaSuccess) return e;
-	}
-	return cudaSuccess;
-}
-
-// n steps from time step t, the last one writing the macros: tile pairs from
-// an even step, the others one by one.
-cudaError_t launch_steps(const kel_batch *B, uint64_t t, uint64_t n, bool tiled) {
+// n steps from time step t, the last one writing the macros; all but the
+// first overlap the one before.
+cudaError_t launch_steps(const kel_batch *B, uint64_t t, uint64_t n) {
 	cudaError_t e = cudaSuccess;
-	for (uint64_t s = 0; s < n && e == cudaSuccess;) {
-		if (tiled && ((t + s) & 1u) == 0 && n - s > 2 * TILE_K) { // the last step is none of theirs
-			e = launch_tile_pair(B);
-			s += 2 * TILE_K;
-		} else {
-			e = launch_sweep_batch(B, ((t + s) & 1u) != 0, s + 1 == n);
-			++s;
-		}
-	}
+	for (uint64_t s = 0; s < n && e == cudaSuccess; ++s)
+		e = launch_sweep_batch(B, ((t + s) & 1u) != 0, s + 1 == n, s > 0);
 	return e;
 }
 
@@ -1114,11 +909,9 @@ extern "C" int kel_batch_set_program(kel_batch *B, const kel_step_program *P) {
 		k_batch_shift<<<grid_for(B->plane), 256, 0, B->stream>>>(params(B, 0), shifted ? -1.f : 1.f);
 		KEL_CUDA(cudaGetLastError());
 	}
-	B->plain = B->bounce = 0;
-	for (int fl = 1; fl < MAX_FLAGS; ++fl) {
+	B->plain = 0;
+	for (int fl = 1; fl < MAX_FLAGS; ++fl)
 		if ((ops[fl].bc == KEL_BC_NONE || ops[fl].bc == KEL_BC_FLUID) && ops[fl].collide) B->plain |= 1u << fl;
-		if (ops[fl].bc == KEL_BC_BOUNCE_BACK && !ops[fl].collide) B->bounce |= 1u << fl;
-	}
 	KEL_CUDA(cudaMemcpyAsync(B->ops, ops, sizeof(ops), cudaMemcpyHostToDevice, B->stream));
 	KEL_CUDA(cudaStreamSynchronize(B->stream));
 	B->prog = *P;
@@ -1145,7 +938,7 @@ extern "C" int kel_batch_step(kel_batch *B, uint64_t n_steps) {
 	uint64_t t = global_t(B);
 	for (int c = 0; c < B->n; ++c)
 		if (act[c] && B->t[c] != t) return fail(KEL_ERR_STATE, "kel_batch_step: channel time steps diverged");
-	const cudaError_t e = launch_steps(B, t, n_steps, n_steps > 2 * TILE_K && ensure_tiles(B));
+	const cudaError_t e = launch_steps(B, t, n_steps);
 	if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_step: %s", cudaGetErrorString(e));
 	for (int c = 0; c < B->n; ++c)
 		if (act[c]) B->t[c] += n_steps;
@@ -1170,7 +963,6 @@ static int compact(kel_batch *B, const std::vector<int> &act) {
 	B->nlaunch = keep;
 	int rc = upload_tile_records(B);
 	if (rc) return rc;
-	if (B->d_tiles && (rc = upload_step_tiles(B))) return rc;
 	if (B->graph) cudaGraphExecDestroy(B->graph);
 	B->graph = nullptr;
 	return KEL_OK;
@@ -1182,9 +974,8 @@ static int build_graph(kel_batch *B, int check, double tol) {
 	if (B->graph) cudaGraphExecDestroy(B->graph);
 	B->graph = nullptr;
 	cudaGraph_t g;
-	const bool tiled = check > 2 * TILE_K && ensure_tiles(B); // no allocation inside the capture
 	KEL_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-	cudaError_t e = launch_steps(B, 0, (uint64_t)check, tiled);
+	cudaError_t e = launch_steps(B, 0, (uint64_t)check);
 	if (e == cudaSuccess) e = launch_residual(B, tol);
 	cudaError_t e2 = cudaStreamEndCapture(B->stream, &g);
 	if (e != cudaSuccess || e2 != cudaSuccess)
@@ -1219,7 +1010,7 @@ extern "C" int kel_batch_run_until(kel_batch *B, double tol, uint64_t check_ever
 		if (use_graph) {
 			KEL_CUDA(cudaGraphLaunch(B->graph, B->stream));
 		} else {
-			cudaError_t e = launch_steps(B, 0, check_every, check_every > 2 * TILE_K && ensure_tiles(B));
+			cudaError_t e = launch_steps(B, 0, check_every);
 			if (e == cudaSuccess) e = launch_residual(B, tol);
 			if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_batch_run_until: %s", cudaGetErrorString(e));
 		}

@@ -929,9 +929,11 @@ static SweepParams make_params(kel_lattice *L, const kel_step_program *P) {
 			p.off_odd[i] = (int)(i * L->plane + L->d.c[i][0] + (L->d.c[i][1] + L->d.c[i][2] * L->desc.ny) * L->nxp);
 		}
 	// Rows are covered by whole blocks: with no launch shape asked for, 64
-	// threads where that leaves fewer idle ones in a row's last block than 128
-	// (64-cell rows half filled their blocks: D3Q19 64^3 12.0 us per step)
-	p.block = !L->tuned && L->cpt == 1 && (L->nxp + 63) / 64 * 64 < (L->nxp + 127) / 128 * 128 ? 64 : L->block;
+	// threads where 128 would leave an eighth of a row's threads idle (64-cell
+	// rows half filled their blocks: D3Q19 64^3 13.0 -> 12.0 us per step; on
+	// long rows 64 threads are the slower block: FP16S 3000x2000 96 us, 60 with 128)
+	const int row64 = (L->nxp + 63) / 64 * 64, row128 = (L->nxp + 127) / 128 * 128;
+	p.block = !L->tuned && L->cpt == 1 && row128 - row64 >= row128 / 8 ? 64 : L->block;
 	p.hw_mask = L->hw_active ? L->hw_mask : nullptr;
 	p.plain = L->plain_flags;
 	p.bounce = L->bounce_flags;
@@ -1011,18 +1013,17 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 }
 
 // Tiles of a lattice of nxp x ny cells on `sms` multiprocessors (two blocks of
-// either shape run on each).  From 1.5 M cells up the wide tiles fill the
-// device several times over (2048x1024: 19.5 us per step against 19.7 for the
-// best small ones, 4096^2 117 against 129); below, the small ones with the
-// fewest rows that give every SM one block (each block's steps follow one
-// another, so a launch takes as long as its rows: 256x64 6 rows 1.55 us per
-// step, 16 rows 2.5), else two, else 20 rows (1021x347: 20 rows 5.5, 12 rows
-// 6.1, 40 rows 5.7).
-static TilePlan plan_tiles(int nxp, int ny, int sms) {
+// either shape run on each), or none: small tiles up to 100,000 cells, wide
+// ones where the populations (pop_bytes) exceed the L2; the lines are where
+// the tiles stop and start to be the faster form (figures in sweep_tile.cuh).
+// Small tiles take the fewest rows that give every SM one block (a block's
+// steps follow one another, so a launch takes as long as its rows: 256x64 6
+// rows 1.55 us per step, 16 rows 2.5), else two.
+static TilePlan plan_tiles(int nxp, int ny, int64_t pop_bytes, int64_t l2_bytes, int sms) {
 	TilePlan t;
 	auto blocks = [&](int tx, int ty) { return (int64_t)((nxp + tx - 1) / tx) * ((ny + ty - 1) / ty); };
-	t.wide = (int64_t)nxp * ny >= 1500000;
-	if (t.wide) { // fewest rows of work per SM, tile row sums 4 ty + 20
+	if (pop_bytes > l2_bytes - l2_bytes / 8) { // fewest rows of work per SM, tile row sums 4 ty + 20
+		t.wide = true;
 		const int tx = TileWide::W - 2 * TILE_K;
 		int64_t best = -1;
 		for (int ty = 24; ty <= 32; ty += 4) {
@@ -1034,12 +1035,12 @@ static TilePlan plan_tiles(int nxp, int ny, int sms) {
 		}
 		return t;
 	}
+	if ((int64_t)nxp * ny > 100000) return t;
 	const int tx = TileSmall::W - 2 * TILE_K;
 	for (t.ty = 4; t.ty <= 8; t.ty += 2)
 		if (blocks(tx, t.ty) <= sms) return t;
-	for (t.ty = 4; t.ty <= 24; t.ty += 2)
+	for (t.ty = 4; t.ty < 24; t.ty += 2)
 		if (blocks(tx, t.ty) <= 2 * sms) return t;
-	t.ty = 20;
 	return t;
 }
 
@@ -1062,14 +1063,14 @@ static bool ensure_f2(kel_lattice *L) {
 
 // 2 TILE_K steps from an even one: into the second array and back, so that
 // the populations are where they were.
-static cudaError_t launch_tile_pair(const kel_lattice *L, const SweepParams &p, int coll, bool exact) {
+static cudaError_t launch_tile_pair(const kel_lattice *L, const SweepParams &p, int coll) {
 	TileParams q;
 	q.p = p;
 	q.ty = L->tile.ty;
 	for (int k = 0; k < 2; ++k) {
 		q.p.f = k ? L->f2 : L->f;
 		q.out = k ? L->f : L->f2;
-		cudaError_t e = launch_tile(q, L->desc.storage, coll, exact, L->tile.wide, L->stream);
+		cudaError_t e = launch_tile(q, L->desc.storage, coll, L->tile.wide, L->stream);
 		if (e != cudaSuccess) return e;
 	}
 	return cudaSuccess;
@@ -1094,7 +1095,7 @@ static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, boo
 	}
 	cudaError_t e = cudaSuccess;
 	if (tiled)
-		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; k += 2 * TILE_K) e = launch_tile_pair(L, p, coll, exact);
+		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; k += 2 * TILE_K) e = launch_tile_pair(L, p, coll);
 	else
 		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) e = launch_one(L, p, coll, exact, (k & 1) != 0);
 	cudaError_t e2 = cudaStreamEndCapture(L->stream, &g);
@@ -1165,11 +1166,17 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 	const uint64_t plain = (step_flags & KEL_STEP_ALL_MACROS)
 							   ? 0
 							   : ((step_flags & KEL_STEP_WRITE_MACROS) && n_steps > 0 ? n_steps - 1 : n_steps);
-	// D2Q9 runs without macro output do TILE_K steps per launch on tiles, in
+	// D2Q9 runs without macro output may do TILE_K steps per launch on tiles, in
 	// pairs of launches from an even step (the remaining steps follow one by one).
-	const bool tiled = L->d.Q == 9 && !capturing && !L->shape_asked && !L->hw_active && p.idx32 &&
-					   P->collision <= KEL_COLL_PSM_GUO && plain >= (L->t & 1u) + 2 * TILE_K && ensure_f2(L);
-	if (tiled && !L->tile.ty) L->tile = plan_tiles(L->nxp, (int)L->desc.ny, L->sms);
+	bool tiled = L->d.Q == 9 && !exact && !capturing && !L->shape_asked && !L->hw_active && p.idx32 &&
+				 P->collision <= KEL_COLL_PSM_GUO && plain >= (L->t & 1u) + 2 * TILE_K;
+	if (tiled && !L->tile.planned) {
+		int l2 = 0;
+		KEL_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, L->device));
+		L->tile = plan_tiles(L->nxp, (int)L->desc.ny, (int64_t)L->d.Q * L->plane * (int64_t)L->elem, l2, L->sms);
+		L->tile.planned = true;
+	}
+	tiled = tiled && L->tile.ty > 0 && ensure_f2(L);
 	constexpr uint64_t pair = 2 * TILE_K;
 	const bool graphed = L->stream != nullptr && !capturing && L->cpt != CPT_ROWS && plain >= 2 * GRAPH_STEPS;
 	if (tiled || graphed) {
@@ -1188,7 +1195,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 			L->t += reps * GRAPH_STEPS;
 		}
 		for (; tiled && plain - s >= pair; s += pair, L->t += pair) {
-			cudaError_t e = launch_tile_pair(L, p, P->collision, exact);
+			cudaError_t e = launch_tile_pair(L, p, P->collision);
 			if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_step: launch failed: %s", cudaGetErrorString(e));
 		}
 	}

@@ -33,8 +33,9 @@ struct HostDesc {
 
 // How a D2Q9 lattice is cut into tiles of TILE_K steps per launch (sweep_tile.cuh).
 struct TilePlan {
+	bool planned = false;
 	bool wide = false;
-	int ty = 0; // tile rows; 0: not planned yet
+	int ty = 0; // tile rows; 0: no tiles
 };
 
 int grid_for(int64_t n);

@@ -1,10 +1,9 @@
 // Sweep kernels for the D2Q9 descriptor, FP32 storage, the reference's arithmetic: every launch shape,
-// parity and collision variant, and the multi-step tiles.
+// parity and collision variant.
 #include "sweep_launch.cuh"
 
 namespace kel {
 namespace gb {
 template cudaError_t launch_sweep_part<D2Q9, PART_EXACT32>(const SweepParams &, bool, int, cudaStream_t);
-template cudaError_t launch_tile_part<PART_EXACT32>(const TileParams &, int, bool, cudaStream_t);
 } // namespace gb
 } // namespace kel

@@ -23,17 +23,15 @@ cudaError_t launch_sweep(const SweepParams &p, int storage, bool odd, int coll, 
 	return launch_sweep_part<L, PART_FP16S>(p, odd, coll, st);
 }
 
-// Several steps of a D2Q9 lattice in one launch (sweep_tile.cuh), on tiles of
-// shape TileWide or TileSmall.
+// Several steps of a D2Q9 lattice in one launch (sweep_tile.cuh; fast arithmetic),
+// on tiles of shape TileWide or TileSmall.
 struct TileParams;
 template <int PART>
 cudaError_t launch_tile_part(const TileParams &q, int coll, bool wide, cudaStream_t st);
 
-inline cudaError_t launch_tile(const TileParams &q, int storage, int coll, bool exact, bool wide, cudaStream_t st) {
-	if (storage == STORE_FP32)
-		return exact ? launch_tile_part<PART_EXACT32>(q, coll, wide, st) : launch_tile_part<PART_FAST32>(q, coll, wide, st);
-	if (exact) return cudaErrorInvalidValue;
-	return launch_tile_part<PART_FP16S>(q, coll, wide, st);
+inline cudaError_t launch_tile(const TileParams &q, int storage, int coll, bool wide, cudaStream_t st) {
+	return storage == STORE_FP32 ? launch_tile_part<PART_FAST32>(q, coll, wide, st)
+								 : launch_tile_part<PART_FP16S>(q, coll, wide, st);
 }
 
 } // namespace gb

@@ -128,10 +128,10 @@ cudaError_t launch_sweep_part(const SweepParams &p, bool odd, int coll, cudaStre
 				   : launch_coll<L, STORE_FP16S, false, false>(p, coll, st);
 }
 
-template <int STORE, int COLL, bool EXACT, class TS>
+template <int STORE, int COLL, class TS>
 static cudaError_t launch_tile_variant(const TileParams &q, cudaStream_t st) {
 	static std::atomic<uint64_t> done{0};
-	auto kern = sweep_tile_kernel<STORE, COLL, EXACT, TS>;
+	auto kern = sweep_tile_kernel<STORE, COLL, TS>;
 	const int smem = tile_smem(TS::W, TS::K, q.ty, (int)sizeof(typename TileStore<STORE>::T));
 	cudaError_t e = allow_smem(kern, smem, done);
 	if (e != cudaSuccess) return e;
@@ -143,11 +143,10 @@ static cudaError_t launch_tile_variant(const TileParams &q, cudaStream_t st) {
 template <int PART>
 cudaError_t launch_tile_part(const TileParams &q, int coll, bool wide, cudaStream_t st) {
 	constexpr int STORE = PART == PART_FP16S ? STORE_FP16S : STORE_FP32;
-	constexpr bool EXACT = PART == PART_EXACT32;
 #define KEL_TILE(C)                                                                                                    \
 	case C:                                                                                                            \
-		return wide ? launch_tile_variant<STORE, C, EXACT, TileWide>(q, st)                                            \
-					: launch_tile_variant<STORE, C, EXACT, TileSmall>(q, st)
+		return wide ? launch_tile_variant<STORE, C, TileWide>(q, st)                                                   \
+					: launch_tile_variant<STORE, C, TileSmall>(q, st)
 	switch (coll) {
 		KEL_TILE(COLL_BGK);
 		KEL_TILE(COLL_BGK_GUO);

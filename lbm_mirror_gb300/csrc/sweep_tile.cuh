@@ -7,13 +7,17 @@
 // compute too (the same operations on the same values: the same bits).
 //
 // Why: a 2D sweep moves 73 bytes per cell and step and is over in a few
-// microseconds.  Large lattices and batches are bound by HBM and by the index
-// arithmetic of nine loads and nine stores from global memory (250 to 280
-// instructions per cell, of which 85 are the collision); small ones by one
-// launch per step.  Here a cell is read and written once per K steps and
+// microseconds.  Small lattices are bound by one launch per step, lattices
+// beyond the L2 by HBM.  Here a cell is read and written once per K steps and
 // the steps between find their populations at constant offsets from one
 // shared-memory address; the price is the ring, computed redundantly (1.3 to
-// 1.6 times the tile's cells, by tile height).
+// 1.6 times the tile's cells, by tile height).  In between, on lattices that
+// the L2 holds, the one-step sweep is the faster one (D2Q9 FP32, tiles / one
+// step, us per step: 256x64 1.7 / 2.2, 512x128 2.2 / 2.4, 512x256 3.3 / 3.1,
+// 1021x347 5.4 / 4.7, 1024^2 12.6 / 10.6, 2048x1024 19.8 / 19.6, 2048^2 34.6 /
+// 42.7, 4096^2 118 / 186), and so it is in the reference's arithmetic at every
+// size from 256x64 up (3.2 / 3.1 there, 4096^2 438 / 300: the ring repeats an
+// expensive collision).
 //
 // Inside the tile the populations are in the AA layout of sweep.cuh (one copy
 // in shared memory, each slot read and written by the same cell within a
@@ -36,14 +40,11 @@ struct TileShape {
 	static constexpr int W = W_, K = K_, R = R_, NT = NT_, BPS = BPS_;
 };
 constexpr int TILE_K = 4;
-// Wide: the least redundant work, two cells per instruction (120 instructions
-// per cell and step); D2Q9 FP32 4096^2 117 us per step (143 G cells/s, the
-// one-step sweep about 215), 2048x1024 19.5.
-// Small: one cell per thread, for lattices that would fill too few blocks of
-// the other; 256x64 1.55 us per step (2.75 with a launch per step), 512x128
-// 2.4, 1021x347 5.5 (Wide 6.2; one-step 7.5).
-// Eight steps per launch lose more to the ring than they save in launches
-// (256x64 1.80, 1021x347 6.7).
+// Wide, for lattices beyond the L2: the least redundant work, two cells per
+// instruction (120 instructions per cell and step; 4096^2 118 us per step,
+// Small 129).  Small, for small lattices: one cell per thread, more blocks
+// (256x64 1.5 us per step, Wide 2.3).  Eight steps per launch lose more to the
+// ring than they save in launches (256x64 1.8).
 using TileWide = TileShape<64, TILE_K, 2, 384, 2>;
 using TileSmall = TileShape<32, TILE_K, 1, 512, 2>;
 
@@ -150,15 +151,14 @@ struct Bounded {
 
 // Out of line: the boundary kinds besides walls, which few cells have and
 // whose code would otherwise be in every step of the tile.
-template <bool EXACT>
-__device__ __noinline__ Bounded tile_boundary(const OpEntry *ops, const float *profile, float f0, float f1, float f2,
+static __device__ __noinline__ Bounded tile_boundary(const OpEntry *ops, const float *profile, float f0, float f1, float f2,
 											  float f3, float f4, float f5, float f6, float f7, float f8, int flag, int y) {
 	float f[9] = {f0, f1, f2, f3, f4, f5, f6, f7, f8};
 	CellCtx ctx;
 	ctx.ops = ops;
 	ctx.profile = profile;
 	Bounded r;
-	r.collides = boundary_step<D2Q9, EXACT>(f, flag, y, ctx);
+	r.collides = boundary_step<D2Q9, false>(f, flag, y, ctx);
 #pragma unroll
 	for (int i = 0; i < 9; ++i) r.f[i] = f[i];
 	return r;
@@ -295,7 +295,7 @@ struct TileParams {
 // Shared memory of a tile of ty rows: populations, boundary bits, flags.
 constexpr int tile_smem(int w, int k, int ty, int elem) { return (ty + 2 * k) * (w * (9 * elem + 1) + w / 32 * 4); }
 
-template <int COLL, bool EXACT>
+template <int COLL>
 struct LatticeCells {
 	const SweepParams &p;
 	__device__ __forceinline__ bool is_plain(int flag) const { return flag < MAX_FLAGS && ((p.plain >> flag) & 1u); }
@@ -306,14 +306,14 @@ struct LatticeCells {
 			bounce_or_zero(f, wall);
 			return false;
 		}
-		const Bounded r = tile_boundary<EXACT>(p.ops, p.profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], flag, y);
+		const Bounded r = tile_boundary(p.ops, p.profile, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], flag, y);
 #pragma unroll
 		for (int i = 0; i < 9; ++i) f[i] = r.f[i];
 		return r.collides != 0;
 	}
 	template <int R>
 	__device__ __forceinline__ void cells(float (&f)[R][9], int c0, int c1) const {
-		if constexpr (COLL == COLL_BGK && !EXACT && R == 2) {
+		if constexpr (COLL == COLL_BGK && R == 2) {
 			collide_bgk2(f[0], f[1], p.omega);
 		} else {
 #pragma unroll
@@ -325,13 +325,13 @@ struct LatticeCells {
 					Fc[0] = p.force[c];
 					Fc[1] = p.force[p.plane + c];
 				}
-				collide<D2Q9, COLL, EXACT>(f[k], cell_ctx(p), por, Fc, rho, u);
+				collide<D2Q9, COLL, false>(f[k], cell_ctx(p), por, Fc, rho, u);
 			}
 		}
 	}
 };
 
-template <int STORE, int COLL, bool EXACT, class TS>
+template <int STORE, int COLL, class TS>
 __global__ void __launch_bounds__(TS::NT, TS::BPS) sweep_tile_kernel(const __grid_constant__ TileParams q) {
 	using T = typename TileStore<STORE>::T;
 	extern __shared__ __align__(16) unsigned char tile_mem[];
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TS::NT, TS::BPS) sweep_tile_kernel(const __gri
 	T *const sm = reinterpret_cast<T *>(tile_mem);
 	uint32_t *const bnd = reinterpret_cast<uint32_t *>(sm + 9 * cells);
 	uint8_t *const fl = reinterpret_cast<uint8_t *>(bnd + cells / 32);
-	tile_steps<STORE, TS>(g, [&](int i) { return p.wshift[i]; }, sm, bnd, fl, LatticeCells<COLL, EXACT>{p});
+	tile_steps<STORE, TS>(g, [&](int i) { return p.wshift[i]; }, sm, bnd, fl, LatticeCells<COLL>{p});
 }
 
 } // namespace gb

@@ -7,7 +7,6 @@ asked for runs it for every step.)"""
 import numpy as np
 import pytest
 
-from lbm_mirror_gb300 import Batch
 from lbm_mirror_gb300 import capi as K
 from tests import cases
 from tests.gpu_util import make_lattice, with_arith
@@ -71,25 +70,3 @@ def test_wide_tiles(mode, collision, periodic):
     case.update(dims=dims, flags=flags.reshape(-1), init=cases.random_populations(9, n, rng), force=None)
     arith = K.KEL_ARITH_REFERENCE if mode == "reference" else K.KEL_ARITH_FAST
     assert_same(*both(case, arith, "fp16s" if mode == "fp16s" else "fp32", (9, 12)))
-
-
-@pytest.mark.parametrize("arithmetic", [K.KEL_ARITH_FAST, K.KEL_ARITH_REFERENCE, K.KEL_ARITH_SHIFTED])
-def test_batch_tiles_equal_one_step_launches(arithmetic):
-    """Channels around the tile edges: one call of many steps (tiles) against
-    calls of eight steps (too few for a tile pair)."""
-    rng = np.random.default_rng(3)
-    chans = []
-    for nx, ny in [(3, 3), (23, 5), (24, 24), (25, 25), (70, 41), (97, 40), (130, 9), (33, 200)]:
-        f = cases.channel_flags((nx, ny)).reshape(ny, nx)
-        f[rng.integers(1, max(2, ny - 1), 4), rng.integers(1, max(2, nx - 1), 4)] = 1
-        chans.append(dict(nx=nx, ny=ny, tau=float(rng.uniform(0.6, 1.0)), u_max=0.04, flags=f))
-    got = []
-    for calls in ([1, 57], [1] + [8] * 7 + [1]):
-        b = Batch(chans, cases.channel_program(0.8, arithmetic))
-        for n in calls:
-            b.step(n)
-        got.append([(b.populations(k), *b.macros(k)) for k in range(b.n)])
-        b.close()
-    for k, (x, y) in enumerate(zip(*got)):
-        for p, q in zip(x, y):
-            np.testing.assert_array_equal(p, q, err_msg=f"channel {k}")
