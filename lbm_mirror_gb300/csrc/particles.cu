@@ -1478,67 +1478,243 @@ __global__ void k_integrate(kel_particle_state *P, int np, int D, kel_particle_p
 	integrate_one(P, pi, D, prm, nx, periodic);
 }
 
+// A body's fields as 28 doubles, in kel_particle_state's order.
+enum : int { PS_POS = 0, PS_OLD = 3, PS_ROT = 6, PS_ROT_OLD = 9, PS_ACC = 12, PS_ANG = 15, PS_FORCE = 18, PS_TORQUE = 21, PS_N = 28 };
+static_assert(sizeof(kel_particle_state) == PS_N * sizeof(double), "28 doubles");
+
+// May bodies s and j touch?  In FP32, with a margin e far above the rounding
+// of the positions (false only where the FP64 test is false too; NaN: true).
+__device__ inline bool may_touch(int D, const float *xs, float rs, const kel_particle_state &o, int periodic, float Lx) {
+	float d2 = 0.f, sum = 0.f;
+	for (int k = 0; k < D; ++k) {
+		const float xo = (float)o.position[k];
+		float d = xs[k] - xo;
+		if (periodic && k == 0) {
+			if (d > 0.5f * Lx) d -= Lx;
+			else if (d < -0.5f * Lx) d += Lx;
+			sum += Lx;
+		}
+		sum += fabsf(xs[k]) + fabsf(xo);
+		d2 += d * d;
+	}
+	const float reach = rs + (float)o.radius, lim = reach + 1e-6f * (sum + reach);
+	return !(d2 > lim * lim * 1.00001f);
+}
+
 // Contact and integrate of the coupled step in one launch, one warp (block)
-// per body: the contact of body s reads every body's state in P_in; lane 0
-// then integrates a copy of body s with that force and writes it to P_out
-// (the next step's state, so that no block reads a body another has already
-// moved), and prepares the next couple's boxes and the body's record for
-// the next couple + gather (its candidate for couple mode cm; lanes
-// 1 .. Q-1 form c_i . u_p).
+// per body: the contact of body s reads every body's state in P_in; the body
+// integrated with that force goes to P_out (the next step's state, so that no
+// block reads a body another has already moved), with the next couple's boxes
+// and the body's record for the next couple + gather (its candidate for
+// couple mode cm and c_i . u_p per direction).
+//
+// The work is a few hundred FP64 operations per body, and an FP64 instruction
+// holds the pipe for tens of cycles however few lanes it has.  So a component
+// is a lane (0-2 the axes, 3-5 the rotations and torques) and every operation
+// is one instruction for all of them, in the order contact_one,
+// integrate_state, body_aabb and cand_prepare have (the same bits); pairs and
+// walls too far to touch are left out by an FP32 test.  As one lane's chain
+// this pass took 24 us and was the coupled step's critical path beside a sweep
+// of 15 us (2048x512, 64 bodies); the step KEL_CI_STEP.
 template <class L>
 __global__ void __launch_bounds__(32) k_contact_integrate(const kel_particle_state *P_in, kel_particle_state *P_out,
 														  PView v, kel_particle_params prm, const double *partial,
 														  int G, BodyBox *cur, BodyBox *prev, int cm, double reach,
 														  CoupleRec *rec) {
+	constexpr int D = L::D;
+	constexpr unsigned FULL = 0xffffffffu;
 	__shared__ double fs[32][4];
 	__shared__ int hs[32];
 	const int s = blockIdx.x, np = (int)gridDim.x;
 	const int lane = threadIdx.x & 31;
-	kel_particle_state q;
-	contact_one(const_cast<kel_particle_state *>(P_in), s, np, v.D, prm, v.nx, v.ny, v.nz, v.periodic, partial, G, true,
-				fs, hs, &q);
-	if (lane == 0) {
-		// contact_one set q's force and torque; the rest of the body from P_in
-		const kel_particle_state &o = P_in[s];
-		const double f0 = q.force[0], f1 = q.force[1], f2 = q.force[2];
-		const double t0 = q.torque[0], t1 = q.torque[1], t2 = q.torque[2];
-		q = o;
-		q.force[0] = f0;
-		q.force[1] = f1;
-		q.force[2] = f2;
-		q.torque[0] = t0;
-		if (v.D == 3) {
-			q.torque[1] = t1;
-			q.torque[2] = t2;
-		}
-		integrate_state(q, v.D, prm, v.nx, v.periodic);
-		P_out[s] = q;
-		int64_t a[3], b[3];
-		body_aabb(v.D, q, v.nx, v.ny, v.nz, v.periodic, cm != 0, a, b, v.box_mul, v.box_add);
-		BodyBox r;
-		for (int k = 0; k < 3; ++k) {
-			r.a[k] = (int)a[k];
-			r.b[k] = (int)b[k];
-		}
-		prev[s] = cur[s];
-		cur[s] = r;
-		Cand c;
-		c.box = r;
-		for (int d = 0; d < 3; ++d) c.X[d] = q.position[d];
-		c.R = q.radius;
-		cand_prepare(c, cm, reach, prm.eps, q.rotation, v.D);
-		rec[s].cand = c;
+	const kel_particle_state &self = P_in[s];
+	const double *const in = reinterpret_cast<const double *>(P_in + s);
+	double *const out = reinterpret_cast<double *>(P_out + s);
+	const bool axis = lane < D, turn = lane >= 3 && lane < (D == 2 ? 4 : 6); // this lane's component
+	const int comp = axis ? lane : (turn ? lane - 3 : 0);
+
+	// ---- force (axis lanes) and torque (turn lanes): the gather sums, g in order
+	double load = 0.0;
+	if (axis || turn)
+		for (int g = 0; g < G; ++g) load += partial[((int64_t)s * G + g) * 6 + lane];
+
+	// ---- pairs, added in index order; D3 contacts give no torque
+	const double steps = (double)(prm.sub_steps == 0 ? 1 : prm.sub_steps);
+	const double Lx = (double)v.nx, ext[3] = {(double)v.nx, (double)v.ny, (double)v.nz};
+	const float xs[3] = {(float)self.position[0], (float)self.position[1], D == 3 ? (float)self.position[2] : 0.f};
+	const float rs = (float)self.radius;
+	auto add_contact = [&](int q) { // contact q of the scratch
+		if (axis) load = load + fs[q][lane];
+		if (D == 2 && lane == 3) load = load + fs[q][3];
+	};
+	for (int j0 = 0; j0 < np; j0 += 32) {
+		const int j = j0 + lane;
+		const bool near = j < np && j != s && may_touch(D, xs, rs, P_in[j], v.periodic, (float)v.nx);
+		if (!__any_sync(FULL, near)) continue;
+		double f[3] = {0, 0, 0}, t0 = 0.0;
+		const bool hit = near && pair_response(self, P_in[j], s, j, D, prm, steps, Lx, v.periodic, f, &t0);
+		fs[lane][0] = f[0];
+		fs[lane][1] = f[1];
+		fs[lane][2] = f[2];
+		fs[lane][3] = t0;
+		hs[lane] = hit ? 1 : 0;
+		__syncwarp();
+		for (int q = 0; q < 32; ++q)
+			if (hs[q]) add_contact(q);
+		__syncwarp();
 	}
+	// ---- walls, in the order axis, side
+#pragma unroll
+	for (int ax = 0; ax < D; ++ax) {
+		if (!(prm.wall_axes & (1u << ax))) continue;
+		const float hbf = (float)ext[ax], e = 1e-6f * (hbf + fabsf(xs[ax]) + rs);
+		for (int side = 0; side < 2; ++side) {
+			// depth > 0 is out of the question
+			if (side == 0 ? xs[ax] - rs > e : hbf - rs - xs[ax] > e) continue;
+			if (lane == 0) {
+				const double x = self.position[ax], r = self.radius, hb = ext[ax];
+				double depth = side == 0 ? (r - x) : (x - (hb - r));
+				hs[0] = depth > 0 ? 1 : 0;
+				if (depth > 0) {
+					if (depth > r) depth = r;
+					double n[3] = {0, 0, 0}, pt[3] = {0, 0, 0}, r_s[3] = {0, 0, 0}, vv[3] = {0, 0, 0};
+					for (int k = 0; k < D; ++k) pt[k] = self.position[k];
+					n[ax] = side == 0 ? 1.0 : -1.0;
+					pt[ax] = side == 0 ? 0.0 : hb;
+					for (int k = 0; k < D; ++k) r_s[k] = pt[k] - self.position[k];
+					surface_velocity(D, self, r_s, steps, vv);
+					double f[3] = {0, 0, 0}, t[3] = {0, 0, 0};
+					soft_shell(D, n, depth, r_s, vv, self.mass, prm, f, t);
+					for (int k = 0; k < 3; ++k) fs[0][k] = f[k];
+					fs[0][3] = t[0];
+				}
+			}
+			__syncwarp();
+			if (hs[0]) add_contact(0);
+			__syncwarp();
+		}
+	}
+
+	// ---- position Verlet (integrate_state)
+	const int sub = prm.sub_steps == 0 ? 1 : prm.sub_steps;
+	const double ts = sub == 1 ? 1.0 : 1.0 / (double)sub, t2 = ts * ts;
+	double acc = load / (axis ? self.mass : self.inertia);
+	if (axis) acc = acc + prm.body_acceleration[comp];
+	if (D == 3 && turn) acc = in[PS_ANG + comp]; // 3D rotations keep the body's angular acceleration
+	double x = axis ? in[PS_POS + comp] : in[PS_ROT + comp], old = axis ? in[PS_OLD + comp] : in[PS_ROT_OLD + comp];
+	for (int k = 0; k < sub; ++k) {
+		const double nw = x * 2.0 - old + acc * t2;
+		old = x;
+		x = nw;
+	}
+	if (v.periodic && lane == 0) {
+		if (x >= Lx) {
+			x -= Lx;
+			old -= Lx;
+		} else if (x < 0.0) {
+			x += Lx;
+			old += Lx;
+		}
+	}
+	if (lane < PS_N) out[lane] = in[lane];
 	__syncwarp();
+	if (axis) {
+		out[PS_POS + comp] = x;
+		out[PS_OLD + comp] = old;
+		out[PS_ACC + comp] = acc;
+		out[PS_FORCE + comp] = load;
+	} else if (turn) {
+		out[PS_ROT + comp] = x;
+		out[PS_ROT_OLD + comp] = old;
+		if (D == 2) out[PS_ANG] = acc;
+		out[PS_TORQUE + comp] = load;
+	}
+	if (D == 2 && lane == 2) out[PS_FORCE + 2] = 0.0;
+
+	// ---- the next couple's box (body_aabb), an axis per lane
+	const double R = self.radius;
+	BodyBox box;
+	{
+		int a = 0, b = 1;
+		if (axis) {
+			const double r = R * v.box_mul + v.box_add;
+			const int n = comp == 0 ? v.nx : (comp == 1 ? v.ny : v.nz);
+			int64_t lo, hi;
+			if (cm != 0) {
+				lo = (int64_t)floor(x - r - 0.5);
+				hi = (int64_t)ceil(x + r + 0.5) + 1;
+			} else {
+				lo = (x >= r) ? (int64_t)(x - r) : 0;
+				if (v.periodic && comp == 0 && x < r) lo = (int64_t)floor(x - r);
+				hi = (int64_t)(x + r + 1.0);
+			}
+			if (!(v.periodic && comp == 0)) {
+				if (lo < 0) lo = 0;
+				if (hi > n) hi = n;
+			}
+			a = (int)lo;
+			b = (int)hi;
+		}
+#pragma unroll
+		for (int k = 0; k < 3; ++k) {
+			box.a[k] = __shfl_sync(FULL, a, k);
+			box.b[k] = __shfl_sync(FULL, b, k);
+		}
+	}
+	// ---- the couple candidate (cand_prepare)
+	double X[3];
+#pragma unroll
+	for (int k = 0; k < 3; ++k) X[k] = k < D ? __shfl_sync(FULL, x, k) : self.position[k];
+	Cand &c = rec[s].cand;
+	if (lane == 0) {
+		prev[s] = cur[s];
+		cur[s] = box;
+	}
+	if (cm == 1 || cm == 2) {
+		// cand_limits: lane 0 the outer limit, lane 1 the inner one
+		const double sgn = lane == 0 ? 1.0 : -1.0;
+		const double lim_r = R + sgn * reach + sgn * 1e-3, lim2 = lim_r * lim_r;
+		const int ic = axis || lane < 3 ? (int)llround(lane == 0 ? X[0] : (lane == 1 ? X[1] : X[2])) : 0;
+		if (lane == 0) {
+			c.box = box;
+			c.R = R;
+			c.lim_out2 = lim2;
+			c.s_out = (float)lim2 + SCREEN_MARGIN;
+			c.Rf = (float)R;
+		} else if (lane == 1) {
+			const double in2 = lim_r > 0.0 ? lim2 : -1.0;
+			c.lim_in2 = in2;
+			c.s_in = in2 > 0.0 ? (float)in2 - SCREEN_MARGIN : -1.0f;
+		}
+		if (lane < 3) {
+			const double xx = lane == 0 ? X[0] : (lane == 1 ? X[1] : X[2]);
+			c.X[lane] = xx;
+			c.ic[lane] = ic;
+			c.fr[lane] = (float)((double)ic - xx);
+		}
+	} else {
+		double rot[3];
+#pragma unroll
+		for (int k = 0; k < 3; ++k) rot[k] = k < (D == 2 ? 1 : 3) ? __shfl_sync(FULL, x, 3 + k) : self.rotation[k];
+		if (lane == 0) {
+			Cand t;
+			t.box = box;
+			for (int k = 0; k < 3; ++k) t.X[k] = X[k];
+			t.R = R;
+			cand_prepare(t, cm, reach, prm.eps, rot, D);
+			c = t;
+		}
+	}
+	// ---- the gather's c_i . u_p, rounded to float as the reference rounds it
+	const double w = axis ? wall_velocity(x - old, prm.sub_steps) : 0.0;
+	double vp[3];
+#pragma unroll
+	for (int k = 0; k < D; ++k) vp[k] = __shfl_sync(FULL, w, k);
 	if (lane >= 1 && lane < L::Q) {
-		// the gather's c_i . u_p, rounded to float as the reference rounds it
-		const kel_particle_state &n = P_out[s];
-		double vp[3] = {0.0, 0.0, 0.0};
-		for (int k = 0; k < L::D; ++k) vp[k] = wall_velocity(n.position[k] - n.position_old[k], prm.sub_steps);
 		double upe_d = 0.0;
 		upe_d = upe_d + (double)L::cx(lane) * vp[0];
 		upe_d = upe_d + (double)L::cy(lane) * vp[1];
-		if (L::D == 3) upe_d = upe_d + (double)L::cz(lane) * vp[2];
+		if (D == 3) upe_d = upe_d + (double)L::cz(lane) * vp[2];
 		rec[s].upe[lane] = (float)upe_d;
 	}
 }
