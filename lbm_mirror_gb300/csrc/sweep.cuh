@@ -26,6 +26,7 @@
 
 #include <cuda_fp16.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "descriptors.cuh"
 
@@ -228,6 +229,14 @@ struct Store<STORE_FP16S> {
 		__stcs(reinterpret_cast<unsigned *>(static_cast<__half *>(base) + idx), *reinterpret_cast<unsigned *>(&h));
 	}
 };
+
+// The first direction of direction i's weight.
+template <class L>
+__host__ __device__ constexpr int shift_class(int i) {
+	int k = 0;
+	while (L::w(k) != L::w(i)) ++k;
+	return k;
+}
 
 // ---------------------------------------------------------------------------
 // Cell physics (one cell, populations in registers).
@@ -1179,16 +1188,15 @@ __global__ void __launch_bounds__(256, 4) sweep2h_kernel(const __grid_constant__
 // global-load latency, and 32 resident warps per SM keep more loads in
 // flight than 24 at 80 registers (measured +3 % FP32, +6 % FP16S at 256^3;
 // the few spilled words stay in L1).
-// Index tables in the parameter bank, prefetch coordinates by carries and the
-// force terms shared between directions took the instructions per cell from
-// 567 / 621 (even / odd step) to 449 / 518 for D3Q19 FP32, 611 / 714 to
-// 533 / 616 FP16S, 1,421 / 1,366 to 1,071 / 1,234 for D3Q27 with a force.
-// Measured: FP16S 256^3 (40 steps) 15.55 -> 14.05 ms, D3Q27 173x131x97 with a
-// force (24 steps) 4.63 -> 3.91 ms, D3Q19 64^3 (100 steps) 1.37 -> 1.19 ms.
-// HW: the lattice has half-way walls (p.hw_mask set); a separate
-// instantiation, so that the stores' redirection costs the common case
-// nothing.
-template <class L, int STORE, bool ODD, int COLL, bool EXACT, bool HW = false>
+// IDX32: every population's index fits 32 bits (Q * plane < 2^31).
+// Index tables in the parameter bank, 32-bit indexes, prefetch coordinates by
+// carries and the force terms shared between directions took the instructions
+// per cell from 567 / 621 (even / odd step) to 412 / 506 for D3Q19 FP32, 611 /
+// 714 to 478 / 576 FP16S, 1,421 / 1,366 to 1,048 / 1,197 for D3Q27 with a
+// force, 274 / 297 to 203 / 256 for D2Q9.  Measured, with the overlapped
+// launches: FP16S 256^3 353 -> 286 us per step, D3Q27 173x131x97 with a force
+// 134 -> 102, D3Q19 64^3 12.4 -> 8.7, D2Q9 1021x347 8.4 -> 4.6.
+template <class L, int STORE, bool ODD, int COLL, bool EXACT, bool HW = false, bool IDX32 = true>
 __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ SweepParams p) {
 	using S = Store<STORE>;
 	constexpr int Q = L::Q;
@@ -1197,7 +1205,9 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	if (x >= p.nxp) return;
 	const int y = blockIdx.y, z = blockIdx.z;
 	const int nxp = p.nxp;
-	const int64_t cell = (static_cast<int64_t>(z) * p.ny + y) * nxp + x;
+	// the cell's index in plane 0: 32-bit arithmetic where every population's index fits
+	using Index = std::conditional_t<IDX32, int, int64_t>;
+	const Index cell = (static_cast<Index>(z) * p.ny + y) * nxp + x;
 	const int64_t oy = nxp, oz = static_cast<int64_t>(nxp) * p.ny;
 	// the lanes still running (a row's last warp may be partial); the fast
 	// paths below are chosen per warp, so that no warp runs two variants
@@ -1211,11 +1221,14 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	const bool ok_xp = has_xp || p.periodic;  // x + 1 exists
 	const bool row_interior = y > 0 && y + 1 < p.ny && (L::D == 2 || (z > 0 && z + 1 < p.nz));
 	using ST = typename S::T;
-	const int c32 = (int)cell; // p.idx32: the cell's index in plane 0
+	const int c32 = (int)cell;
+	// the shift depends on the weight alone: one constant per kind of direction
+	auto ws = [&](int i) { return p.wshift[shift_class<L>(i)]; };
 	// L2 prefetch of the rows the block (pf_x, pf_y, pf_z) later will read (its x range in every direction plane; in odd steps its
 	// neighbours' rows are prefetched by their own predecessors): requests in
 	// flight that hold no registers, one 128-byte line per thread.
-	{
+	const int pf_i = (int)threadIdx.x >> p.pf_shift; // the plane this thread prefetches
+	if (pf_i < Q) {
 		// by carries: the 64-bit divisions of a flat block index cost every
 		// thread 40 to 50 instructions
 		int bx = (int)blockIdx.x + p.pf_x, by = (int)blockIdx.y + p.pf_y, bz = (int)blockIdx.z + p.pf_z;
@@ -1229,10 +1242,11 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 		}
 		if (bz < (int)gridDim.z) {
 			constexpr int per = 128 / (int)sizeof(ST); // cells per line
-			const int i = (int)threadIdx.x >> p.pf_shift;
 			const int x0 = bx * (int)blockDim.x + ((int)threadIdx.x & ((1 << p.pf_shift) - 1)) * per;
-			if (i < Q && x0 < nxp) {
-				const ST *a = static_cast<const ST *>(p.f) + i * p.plane + (static_cast<int64_t>(bz) * p.ny + by) * nxp + x0;
+			if (x0 < nxp) {
+				const ST *a = static_cast<const ST *>(p.f) + ((static_cast<Index>(bz) * p.ny + by) * nxp + x0);
+				if (IDX32) a += p.off_even[pf_i];
+				else a += pf_i * p.plane;
 				asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
 			}
 		}
@@ -1242,25 +1256,25 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	grid_dependency_wait();
 
 	float f[Q];
-	// p.idx32, odd steps: the cell's index for accesses to x - 1 and x + 1
+	// IDX32, odd steps: the cell's index for accesses to x - 1 and x + 1
 	// (periodic rows wrap)
 	const int c32m = c32 + (has_xm ? 0 : nxp), c32p = c32 - (has_xp ? 0 : nxp);
-	if (!ODD && p.idx32) {
+	if (!ODD && IDX32) {
 #pragma unroll
-		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_even[i], p.wshift[i]);
+		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_even[i], ws(i));
 	} else if (!ODD) {
 #pragma unroll
-		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, i * p.plane + cell, p.wshift[i]);
-	} else if (row_interior && p.idx32 && x_inner) {
+		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, i * p.plane + cell, ws(i));
+	} else if (row_interior && IDX32 && x_inner) {
 		// every neighbour exists: no predicates (x - c_i in plane opp i)
 #pragma unroll
-		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_odd[L::opp(i)], p.wshift[i]);
-	} else if (row_interior && p.idx32) {
+		for (int i = 0; i < Q; ++i) f[i] = S::ld1(p.f, c32 + p.off_odd[L::opp(i)], ws(i));
+	} else if (row_interior && IDX32) {
 #pragma unroll
 		for (int i = 0; i < Q; ++i) {
 			const int cx = L::cx(i);
 			const bool ok = cx > 0 ? ok_xm : (cx < 0 ? ok_xp : true);
-			f[i] = ok ? S::ld1(p.f, (cx > 0 ? c32m : (cx < 0 ? c32p : c32)) + p.off_odd[L::opp(i)], p.wshift[i]) : 0.f;
+			f[i] = ok ? S::ld1(p.f, (cx > 0 ? c32m : (cx < 0 ? c32p : c32)) + p.off_odd[L::opp(i)], ws(i)) : 0.f;
 		}
 	} else if (row_interior) {
 #pragma unroll
@@ -1269,7 +1283,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 			const int cx = L::cx(i), cy = L::cy(i), cz = L::cz(i);
 			const int64_t off = (cx > 0 ? xm : (cx < 0 ? xp : 0)) - cy * oy - cz * oz;
 			const bool ok = cx > 0 ? ok_xm : (cx < 0 ? ok_xp : true);
-			f[i] = ok ? S::ld1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell + off, p.wshift[i]) : 0.f;
+			f[i] = ok ? S::ld1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell + off, ws(i)) : 0.f;
 		}
 	} else {
 #pragma unroll
@@ -1279,7 +1293,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 			if (p.periodic) sx = sx < 0 ? sx + nxp : (sx >= nxp ? sx - nxp : sx);
 			const bool in = sx >= 0 && sx < nxp && sy >= 0 && sy < p.ny && sz >= 0 && sz < p.nz;
 			f[i] = in ? S::ld1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane +
-										(static_cast<int64_t>(sz) * p.ny + sy) * nxp + sx, p.wshift[i])
+										(static_cast<int64_t>(sz) * p.ny + sy) * nxp + sx, ws(i))
 					  : 0.f;
 		}
 	}
@@ -1326,41 +1340,41 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 				const int64_t dcell = (static_cast<int64_t>(dz) * p.ny + dy) * nxp + dx;
 				const bool wall = (hw >> i) & 1u;
 				if (!ODD) {
-					S::st1(p.f, wall ? pb + dcell : po + cell, f[i], p.wshift[i]);
+					S::st1(p.f, wall ? pb + dcell : po + cell, f[i], ws(i));
 				} else {
 					int sx = x - cx;
 					const int sy = y - cy, sz = z - cz;
 					if (p.periodic) sx = sx < 0 ? sx + nxp : (sx >= nxp ? sx - nxp : sx);
 					if (sx < 0 || sx >= nxp || sy < 0 || sy >= p.ny || sz < 0 || sz >= p.nz)
-						S::st1(p.f, pb + cell, 0.f, p.wshift[i]); // ghost ring's zero
-					if (wall) S::st1(p.f, po + cell, f[i], p.wshift[i]);
+						S::st1(p.f, pb + cell, 0.f, ws(i)); // ghost ring's zero
+					if (wall) S::st1(p.f, po + cell, f[i], ws(i));
 					else if (dx >= 0 && dx < nxp && dy >= 0 && dy < p.ny && dz >= 0 && dz < p.nz)
-						S::st1(p.f, pb + dcell, f[i], p.wshift[i]);
+						S::st1(p.f, pb + dcell, f[i], ws(i));
 				}
 			}
 			return;
 		}
 	}
 	if (!ODD) {
-		if (p.idx32) {
+		if (IDX32) {
 #pragma unroll
-			for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_even[L::opp(i)], f[i], p.wshift[i]);
+			for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_even[L::opp(i)], f[i], ws(i));
 		} else {
 #pragma unroll
 			for (int i = 0; i < Q; ++i)
-				S::st1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell, f[i], p.wshift[i]);
+				S::st1(p.f, static_cast<int64_t>(L::opp(i)) * p.plane + cell, f[i], ws(i));
 		}
-	} else if (row_interior && p.idx32 && x_inner) {
+	} else if (row_interior && IDX32 && x_inner) {
 		// every destination exists and no source lies outside: no predicates
 #pragma unroll
-		for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_odd[i], f[i], p.wshift[i]);
-	} else if (row_interior && p.idx32) {
+		for (int i = 0; i < Q; ++i) S::st1(p.f, c32 + p.off_odd[i], f[i], ws(i));
+	} else if (row_interior && IDX32) {
 #pragma unroll
 		for (int i = 0; i < Q; ++i) {
 			const int cx = L::cx(i);
-			if ((cx > 0 && !ok_xm) || (cx < 0 && !ok_xp)) S::st1(p.f, c32 + p.off_even[i], 0.f, p.wshift[i]);
+			if ((cx > 0 && !ok_xm) || (cx < 0 && !ok_xp)) S::st1(p.f, c32 + p.off_even[i], 0.f, ws(i));
 			const bool ok = cx > 0 ? ok_xp : (cx < 0 ? ok_xm : true);
-			if (ok) S::st1(p.f, (cx > 0 ? c32p : (cx < 0 ? c32m : c32)) + p.off_odd[i], f[i], p.wshift[i]);
+			if (ok) S::st1(p.f, (cx > 0 ? c32p : (cx < 0 ? c32m : c32)) + p.off_odd[i], f[i], ws(i));
 		}
 	} else if (row_interior) {
 #pragma unroll
@@ -1369,11 +1383,11 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 			// lies outside gets the ghost ring's zero
 			const int cx = L::cx(i), cy = L::cy(i), cz = L::cz(i);
 			const int64_t pb = static_cast<int64_t>(i) * p.plane + cell;
-			if (cx > 0 && !ok_xm) S::st1(p.f, pb, 0.f, p.wshift[i]);
-			if (cx < 0 && !ok_xp) S::st1(p.f, pb, 0.f, p.wshift[i]);
+			if (cx > 0 && !ok_xm) S::st1(p.f, pb, 0.f, ws(i));
+			if (cx < 0 && !ok_xp) S::st1(p.f, pb, 0.f, ws(i));
 			const int64_t off = (cx > 0 ? xp : (cx < 0 ? xm : 0)) + cy * oy + cz * oz;
 			const bool ok = cx > 0 ? ok_xp : (cx < 0 ? ok_xm : true);
-			if (ok) S::st1(p.f, pb + off, f[i], p.wshift[i]);
+			if (ok) S::st1(p.f, pb + off, f[i], ws(i));
 		}
 	} else {
 #pragma unroll
@@ -1382,13 +1396,13 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 			{
 				const int sx = x - L::cx(i), sy = y - L::cy(i), sz = z - L::cz(i);
 				const bool out_x = !p.periodic && (sx < 0 || sx >= nxp);
-				if (out_x || sy < 0 || sy >= p.ny || sz < 0 || sz >= p.nz) S::st1(p.f, pb + cell, 0.f, p.wshift[i]);
+				if (out_x || sy < 0 || sy >= p.ny || sz < 0 || sz >= p.nz) S::st1(p.f, pb + cell, 0.f, ws(i));
 			}
 			int dx = x + L::cx(i);
 			const int dy = y + L::cy(i), dz = z + L::cz(i);
 			if (p.periodic) dx = dx < 0 ? dx + nxp : (dx >= nxp ? dx - nxp : dx);
 			if (dx >= 0 && dx < nxp && dy >= 0 && dy < p.ny && dz >= 0 && dz < p.nz)
-				S::st1(p.f, pb + (static_cast<int64_t>(dz) * p.ny + dy) * nxp + dx, f[i], p.wshift[i]);
+				S::st1(p.f, pb + (static_cast<int64_t>(dz) * p.ny + dy) * nxp + dx, f[i], ws(i));
 		}
 	}
 }

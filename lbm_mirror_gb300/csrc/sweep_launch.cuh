@@ -70,7 +70,8 @@ static cudaError_t launch_sweep1(SweepParams p, int block, cudaStream_t st) {
 	p.pf_z = ahead / (int)grid.x / (int)grid.y;
 	const int lines = block * (int)sizeof(typename Store<STORE>::T) / 128;
 	p.pf_shift = lines >= 8 ? 3 : (lines >= 4 ? 2 : (lines >= 2 ? 1 : 0));
-	return launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW>, grid, block, 0, st, p.overlap != 0, p);
+	return p.idx32 ? launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, true>, grid, block, 0, st, p.overlap != 0, p)
+				   : launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, false>, grid, block, 0, st, p.overlap != 0, p);
 }
 
 template <class L, int STORE, bool ODD, int COLL, bool EXACT>
