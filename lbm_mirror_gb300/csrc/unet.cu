@@ -2099,6 +2099,10 @@ struct kel_unet {
 	float *col_open = nullptr, *col_h3 = nullptr, *col_res = nullptr, *col_pl = nullptr; // input-feature scratch (max_batch x W)
 	HeadRes res; // residual head per output channel (kel_unet_set_residual)
 	cudaStream_t own_stream = nullptr; // the stream the net created (stream may be a caller's)
+	// Weight gradients run beside the chain of data gradients: on side, between
+	// ev_ready (a layer's output gradient is in place) and ev_done.
+	cudaStream_t side = nullptr;
+	cudaEvent_t ev_ready = nullptr, ev_done = nullptr;
 	int sms = 0;                       // the device's SM count (grid sizing)
 	// kel_unet_train_step: the target copy, Adam's lr and bias corrections on
 	// the device, the last loss, and the captured step (forward, backward,
@@ -2484,6 +2488,24 @@ int sum_blocks(int64_t M, int64_t &chunk) {
 	return (int)((M + chunk - 1) / chunk);
 }
 
+// The weight gradients run on U->side beside the chain of data gradients on
+// U->stream: nothing on that chain reads them, each of the two fills the other's
+// last waves, and the reductions (a few blocks each) leave the chain.  Two
+// launches whose tensor memory does not fit one SM together take turns there: an
+// allocation waits for the other CTA, which holds its columns and waits for
+// nothing.  U->partial is used on U->side alone between fork and join.
+int fork_side(kel_unet *U) {
+	KEL_CUDA(cudaEventRecord(U->ev_ready, U->stream));
+	KEL_CUDA(cudaStreamWaitEvent(U->side, U->ev_ready, 0));
+	return KEL_OK;
+}
+
+int join_side(kel_unet *U) {
+	KEL_CUDA(cudaEventRecord(U->ev_done, U->side));
+	KEL_CUDA(cudaStreamWaitEvent(U->stream, U->ev_done, 0));
+	return KEL_OK;
+}
+
 // A layer's gradients from its weight partials (U->partial) and the channel
 // sums of dy (left by the pass that made dy; a wide layer sums them here).
 int reduce_layer(kel_unet *U, const UnetLayer &l, const bf16 *dy, int n, int chunks) {
@@ -2492,9 +2514,9 @@ int reduce_layer(kel_unet *U, const UnetLayer &l, const bf16 *dy, int n, int chu
 	float *wg = U->g + l.woff, *bg = wg + per;
 	int64_t chunk;
 	const int nb = sum_blocks(M, chunk);
-	if (l.boff < 0) bias_grad<<<l.co, 256, 0, U->stream>>>(dy, M, l.co, bg);
+	if (l.boff < 0) bias_grad<<<l.co, 256, 0, U->side>>>(dy, M, l.co, bg);
 	launch_reduce_partials(U->partial, per, chunks, wg, l.boff < 0 ? nullptr : U->bias_partial + l.boff,
-						   l.boff < 0 ? 0 : l.co, nb, bg, U->stream);
+						   l.boff < 0 ? 0 : l.co, nb, bg, U->side);
 	KEL_CUDA(cudaGetLastError());
 	return KEL_OK;
 }
@@ -2552,7 +2574,7 @@ int wgrad_halo_launch(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16
 	KEL_CUDA(allow_dynamic_smem<conv_wgrad_halo>(222 * 1024));
 	// one CTA per SM when its TMEM columns would not leave room for a second
 	const size_t smem_launch = per_sm == 1 && smem < 116u * 1024u ? 116u * 1024u : smem;
-	conv_wgrad_halo<<<(unsigned)(chunks * per_chunk_ctas), 128, smem_launch, U->stream>>>(tx, tdy, a);
+	conv_wgrad_halo<<<(unsigned)(chunks * per_chunk_ctas), 128, smem_launch, U->side>>>(tx, tdy, a);
 	KEL_CUDA(cudaGetLastError());
 	*launched = 1;
 	return reduce_layer(U, l, dy, n, (int)chunks);
@@ -2591,7 +2613,7 @@ int conv_grads_tc(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy
 	a.err = U->d_err;
 	const size_t smem = (size_t)a.stages * ((size_t)l.co * 128 + (size_t)TC_M * 128) + (size_t)a.stages * 8 + 16;
 	KEL_CUDA(allow_dynamic_smem<conv_wgrad_tc>(200 * 1024));
-	conv_wgrad_tc<<<dim3((unsigned)tiles, (unsigned)chunks), 128, smem, U->stream>>>(a);
+	conv_wgrad_tc<<<dim3((unsigned)tiles, (unsigned)chunks), 128, smem, U->side>>>(a);
 	return reduce_layer(U, l, dy, n, (int)chunks);
 }
 
@@ -2617,7 +2639,7 @@ int conv_grads(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16 *dy, i
 	a.chunk = ((M + chunks - 1) / chunks + 15) / 16 * 16;
 	chunks = (M + a.chunk - 1) / a.chunk;
 	dim3 grid((unsigned)((l.co + CB_M - 1) / CB_M), (unsigned)((K + CB_N - 1) / CB_N), (unsigned)chunks);
-	conv_wgrad<<<grid, 128, 0, U->stream>>>(a);
+	conv_wgrad<<<grid, 128, 0, U->side>>>(a);
 	return reduce_layer(U, l, dy, n, (int)chunks);
 }
 
@@ -2725,6 +2747,9 @@ extern "C" int kel_unet_create(const kel_unet_desc *desc, uint64_t seed, kel_une
 					cudaGetErrorString(e));
 	};
 	cudaError_t e;
+	if ((e = cudaStreamCreateWithFlags(&U->side, cudaStreamNonBlocking)) != cudaSuccess) return fail_out(e);
+	if ((e = cudaEventCreateWithFlags(&U->ev_ready, cudaEventDisableTiming)) != cudaSuccess) return fail_out(e);
+	if ((e = cudaEventCreateWithFlags(&U->ev_done, cudaEventDisableTiming)) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMalloc(&U->p, sizeof(float) * off)) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMalloc(&U->g, sizeof(float) * off)) != cudaSuccess) return fail_out(e);
 	if ((e = cudaMalloc(&U->m, sizeof(float) * off)) != cudaSuccess) return fail_out(e);
@@ -2809,6 +2834,12 @@ extern "C" int kel_unet_destroy(kel_unet *U) {
 	cudaFree(U->adam_c);
 	cudaFree(U->dev_loss);
 	if (U->train_graph) cudaGraphExecDestroy(U->train_graph);
+	if (U->side) {
+		cudaStreamSynchronize(U->side);
+		cudaStreamDestroy(U->side);
+	}
+	if (U->ev_ready) cudaEventDestroy(U->ev_ready);
+	if (U->ev_done) cudaEventDestroy(U->ev_done);
 	if (U->own_stream) {
 		cudaStreamSynchronize(U->own_stream);
 		cudaStreamDestroy(U->own_stream);
@@ -2966,8 +2997,9 @@ static int unet_backward(kel_unet *U, const float *d_target, int32_t n, double *
 																U->partial,
 																L[13].boff < 0 ? nullptr : U->bias_partial + L[13].boff);
 		});
+		if ((rc = fork_side(U))) return rc;
 		launch_reduce_partials(U->partial, (int64_t)hd.co * hd.ci + hd.co, nb, U->g + hd.woff, nullptr, 0, 0, nullptr,
-							   U->stream);
+							   U->side);
 	} else {
 		head_backward_dx<<<grid_of(M), 256, sizeof(float) * hd.co * hd.ci, U->stream>>>(U->dout, U->p + hd.woff, G[T_D0B],
 																						 M, hd.ci, hd.co);
@@ -2978,8 +3010,8 @@ static int unet_backward(kel_unet *U, const float *d_target, int32_t n, double *
 	// one conv layer, dy = G[t_out] ready: weight and bias gradients, data gradient into dx
 	auto back = [&](int li, const bf16 *x_in, int t_out, bf16 *dx) -> int {
 		const UnetLayer &l = L[li];
-		int r = conv_grads(U, l, x_in, G[t_out], n);
-		if (r) return r;
+		int r = fork_side(U);
+		if (r || (r = conv_grads(U, l, x_in, G[t_out], n))) return r;
 		if (dx) r = conv_fwd(U, G[t_out], l.wf, nullptr, dx, n, l.level, l.co, l.ci, false, false);
 		return r;
 	};
@@ -2997,8 +3029,11 @@ static int unet_backward(kel_unet *U, const float *d_target, int32_t n, double *
 		(rc = pair(7, T_BB, DY_UPSAMPLE, from_up(T_C2, w[3], w[2]), 6, T_BA, A[T_P2], G[T_P2])) ||
 		(rc = pair(5, T_E2B, DY_POOL, from_pool(T_C2, w[3], w[2], T_P2), 4, T_E2A, A[T_P1], G[T_P1])) ||
 		(rc = pair(3, T_E1B, DY_POOL, from_pool(T_C1, w[2], w[1], T_P1), 2, T_E1A, A[T_P0], G[T_P0])) ||
-		(rc = pair(1, T_E0B, DY_POOL, from_pool(T_C0, w[1], w[0], T_P0), 0, T_E0A, U->input, nullptr)))
+		(rc = pair(1, T_E0B, DY_POOL, from_pool(T_C0, w[1], w[0], T_P0), 0, T_E0A, U->input, nullptr))) {
+		join_side(U);
 		return rc;
+	}
+	if ((rc = join_side(U))) return rc;
 	KEL_CUDA(cudaGetLastError());
 	if (dev_loss) {
 		loss_finish<<<1, 64, 0, U->stream>>>(U->loss_partial, lb, nout, dev_loss);

@@ -135,3 +135,26 @@ def test_gradients_at_the_edges_of_the_split(h, w, n, widths, outs, kind):
         o += b.size
         assert np.linalg.norm(a - b) <= BOUND * np.linalg.norm(b), (k, np.linalg.norm(a - b) / np.linalg.norm(b))
     assert o == got.size
+
+
+@pytest.mark.parametrize("own_stream", [True, False], ids=["net_stream", "caller_stream"])
+def test_gradients_repeat_bit_for_bit(own_stream):
+    """the weight gradients' side stream against the chain it runs beside"""
+    from lbm_mirror_gb300 import UNet
+    h, w, n = 32, 128, 2
+    gen = torch.Generator().manual_seed(5)
+    net = UNet(height=h, width=w, widths=(32, 64, 64, 128), out_channels=3, max_batch=n, seed=3)
+    stream = torch.cuda.Stream()
+    if not own_stream:
+        net.set_stream(stream.cuda_stream)
+    x = torch.randn((n, h, w, 16), generator=gen).to(torch.bfloat16).cuda()
+    t = torch.randn((n, h, w, 3), generator=gen).cuda()
+    torch.cuda.synchronize()
+    net.set_input(x.data_ptr(), n)
+    net.forward(n)
+    first = None
+    for _ in range(20):
+        net.backward(t.data_ptr(), n)
+        g = net.grads()
+        first = g if first is None else first
+        assert np.array_equal(g, first)
