@@ -442,9 +442,13 @@ __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
 // -1, 0, +1 (zero-filled at the image edge), and the shift dx selects the
 // copy instead of moving by a pixel.  The nine taps of a chunk read one
 // halo, where an im2col tile holds every input value nine times.  The chunk's
-// weights (Co x 9 x CK) arrive by TMA as [g][tap][co][8 channels]: B of tap t
-// and channel groups 2j, 2j + 1 at ((2 j) * 9 + t) * Co * 16, LBO = 9 * Co *
-// 16, SBO = 128.  One thread issues the copies (one mbarrier per stage counts
+// weights (Co x 9 x CK) lie in global memory as they do in shared memory, [g][dx]
+// [dy][co][8 channels] (UnetLayer::pw), and arrive as one bulk copy (a copy per
+// group and tap where the CTA has half of the channels): as a TMA box of 16-byte
+// rows they took most of a CTA's staging time (training step 256 x 64, batch
+// 32: 1903 -> 1754 us with conv_rows).  B of
+// tap (dy, dx) and channel groups 2j, 2j + 1 at ((2 j) * 9 + 3 dx + dy) * Co *
+// 16, LBO = 9 * Co * 16, SBO = 128.  One thread issues the copies (one mbarrier per stage counts
 // their bytes) and the MMAs (committed to the stage's second mbarrier, which
 // frees the stage for the chunk S later).  Every wait is bounded; on timeout
 // the CTA records the failure in *err, waits (bounded) for the copies it
@@ -453,6 +457,7 @@ __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
 constexpr int HX = 130; // halo pixels per row
 
 struct HaloArgs {
+	const bf16 *pw; // packed weights
 	const float *bias;
 	bf16 *y; // (N,H,W,Co)
 	int N, H, W, Ci, Co, CK;
@@ -462,7 +467,7 @@ struct HaloArgs {
 	int relu, use_bias;
 	int stages;
 	uint32_t copy_bytes;       // one halo copy of a chunk
-	uint32_t a_bytes, b_bytes; // bytes of the TMA boxes of a chunk (NC copies; the weights)
+	uint32_t a_bytes, b_bytes; // bytes of a chunk's halo (NC copies) and weights
 	uint32_t a_span, stage_bytes; // B's offset in a stage and the stage size (1024-byte multiples)
 	uint32_t tmem_cols;
 	int *err;
@@ -480,16 +485,14 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map
 				 : "memory");
 }
 
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t mbar, int c0, int c1, int c2,
-											int c3) {
-	asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, "
-				 "%6}], [%2];\n" ::"r"(dst),
-				 "l"(map), "r"(mbar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+// `bytes` (a multiple of 16) consecutive bytes; both addresses 16-byte aligned
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t mbar) {
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+				 "l"(src), "r"(bytes), "r"(mbar)
 				 : "memory");
 }
 
-__global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtensorMap tx,
-												 const __grid_constant__ CUtensorMap tw, HaloArgs a) {
+__global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtensorMap tx, HaloArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int S = a.stages;
@@ -539,7 +542,13 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 			for (int cp = 0; cp < a.NC; ++cp)
 				tma_load_5d(base + (uint32_t)cp * a.copy_bytes, &tx, smem_u32(full + s), 0, x0 - 1 + (a.NC == 3 ? cp : 0),
 							yy - 1, c * (a.CK / 8), n);
-			tma_load_4d(base + a.a_span, &tw, smem_u32(full + s), 0, co0, 0, c * (a.CK / 8));
+			const bf16 *w = a.pw + ((int64_t)c * (a.CK / 8) * 9 * a.Co + co0) * 8;
+			if (a.CoT == a.Co)
+				bulk_load(base + a.a_span, w, a.b_bytes, smem_u32(full + s));
+			else
+				for (int k = 0; k < a.CK / 8 * 9; ++k)
+					bulk_load(base + a.a_span + (uint32_t)(k * a.CoT) * 16u, w + (int64_t)k * a.Co * 8, (uint32_t)a.CoT * 16u,
+							  smem_u32(full + s));
 		};
 		for (int c = 0; c < S && c < nch; ++c) load(c);
 		loaded = S < nch ? S : nch;
@@ -557,7 +566,7 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 			for (int j = 0; j < a.CK / 16; ++j)
 				for (int t = 0; t < 9; ++t) {
 					const int dy = t / 3, dx = t % 3;
-					const uint64_t bd = bd0 + (uint64_t)((2 * j * 9 + t) * a.CoT);
+					const uint64_t bd = bd0 + (uint64_t)((2 * j * 9 + dx * 3 + dy) * a.CoT);
 					const uint32_t acc = (c > 0 || j > 0 || t > 0) ? 1u : 0u;
 					uint64_t ad = ad0 + (uint64_t)(2 * j) * (lbo_a >> 4) + (uint64_t)(dy * a.P) + (uint64_t)dx * dx_step;
 					for (int r = 0; r < RT; ++r) {
@@ -637,8 +646,8 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 //
 // For layers whose weights and four input rows fit shared memory: one CTA
 // computes RL consecutive output rows of one 128-pixel column tile (n, x0).
-// The weights (Co x 9 x Ci) arrive once, by TMA, as [g][kx][ky][co][8
-// channels]: for a column shift dx the three kernel rows' Co x 8 blocks are
+// The weights (Co x 9 x Ci) arrive once, as one bulk copy of UnetLayer::pw,
+// [g][kx][ky][co][8 channels]: for a column shift dx the three kernel rows' Co x 8 blocks are
 // consecutive, so B rows (ky, co) form one operand of up to 3 Co rows (8-row
 // stride 128 B, channel-group stride 9 * Co * 16 B).  Input rows y0 - 1 ..
 // y0 + RL stream once each through a ring of NR slots, each row a TMA box of
@@ -664,6 +673,7 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 // and the MMA thread for its MMAs before TMEM is freed.
 
 struct RowsArgs {
+	const bf16 *pw; // packed weights
 	const float *bias;
 	bf16 *y; // (N,H,W,Co)
 	int N, H, W, Ci, Co;
@@ -675,8 +685,7 @@ struct RowsArgs {
 	int *err;
 };
 
-__global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtensorMap tx,
-												 const __grid_constant__ CUtensorMap tw, RowsArgs a) {
+__global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtensorMap tx, RowsArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int NR = a.NR, RB = a.RB;
@@ -726,7 +735,7 @@ __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtenso
 		if (lane == 0) { // producer
 			int fail = 0, issued = 0;
 			mbar_expect_tx(smem_u32(w_full), a.w_bytes);
-			tma_load_5d(smem_u32(sm + a.w_off), &tw, smem_u32(w_full), 0, 0, 0, 0, 0);
+			bulk_load(smem_u32(sm + a.w_off), a.pw, a.w_bytes, smem_u32(w_full));
 			for (int j = 0; j < nx; ++j) {
 				const int s = j % NR;
 				if (j >= NR && !mbar_wait(smem_u32(row_empty + s), (uint32_t)(((j / NR) - 1) & 1))) {
@@ -1876,21 +1885,23 @@ __global__ void loss_finish(const double *partial, int nb, int64_t n, double *lo
 }
 
 // bf16 copies of the 3x3 conv weights: w = [co][ky][kx][ci] and the flipped,
-// transposed wf = [ci][2-ky][2-kx][co] of the data gradient.  One launch for
-// every layer: blockIdx.y picks the layer from the table.
+// transposed wf = [ci][2-ky][2-kx][co] of the data gradient; pw and pwf hold the
+// same for conv_rows and conv_halo, as those keep them in shared memory:
+// [ci / 8][kx][ky][co][ci % 8].  One launch for every layer: blockIdx.y picks
+// the layer from the table.
 constexpr int MAX_CONV = 16;
 struct ConvTable {
 	int nl;
 	int64_t off[MAX_CONV]; // FP32 weights in the parameter vector
 	int co[MAX_CONV], ci[MAX_CONV];
-	bf16 *w[MAX_CONV], *wf[MAX_CONV];
+	bf16 *w[MAX_CONV], *wf[MAX_CONV], *pw[MAX_CONV], *pwf[MAX_CONV];
 };
 
 __global__ void refresh_conv_weights(const float *p, const __grid_constant__ ConvTable t) {
 	const int l = blockIdx.y;
 	const int Co = t.co[l], Ci = t.ci[l], k = 3;
 	const float *w32 = p + t.off[l];
-	bf16 *w = t.w[l], *wf = t.wf[l];
+	bf16 *w = t.w[l], *wf = t.wf[l], *pw = t.pw[l], *pwf = t.pwf[l];
 	const int64_t n = (int64_t)Co * k * k * Ci;
 	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 		const int ci = (int)(i % Ci);
@@ -1901,7 +1912,9 @@ __global__ void refresh_conv_weights(const float *p, const __grid_constant__ Con
 		const int co = (int)(r / k);
 		const bf16 v = __float2bfloat16(w32[i]);
 		w[i] = v;
-		if (wf) wf[(((int64_t)ci * k + (k - 1 - ky)) * k + (k - 1 - kx)) * Co + co] = v;
+		wf[(((int64_t)ci * k + (k - 1 - ky)) * k + (k - 1 - kx)) * Co + co] = v;
+		pw[((int64_t)((ci >> 3) * 9 + kx * 3 + ky) * Co + co) * 8 + (ci & 7)] = v;
+		pwf[((int64_t)((co >> 3) * 9 + (2 - kx) * 3 + 2 - ky) * Ci + ci) * 8 + (co & 7)] = v;
 	}
 }
 
@@ -2074,7 +2087,8 @@ int grid_of(int64_t n) { return grid_for(n); }
 struct UnetLayer {
 	int co, ci, k;  // conv shape
 	int64_t woff;   // offset of the weights in the flat parameter vector (bias follows)
-	bf16 *w = nullptr, *wf = nullptr;
+	bf16 *w = nullptr, *wf = nullptr;   // refresh_conv_weights
+	bf16 *pw = nullptr, *pwf = nullptr;
 	int level;      // spatial level (0 = full resolution)
 	int64_t boff = -1; // offset of the layer's bias sums in bias_partial (-1: none)
 };
@@ -2213,7 +2227,7 @@ int halo_plan(int Ci, int Co, int RT, HaloArgs &a) {
 
 // The halo convolution (conv_halo); returns 0 without
 // launching when the layer does not fit it.
-int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, bf16 *y, int n, int H, int W, int ci,
+int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b, bf16 *y, int n, int H, int W, int ci,
 					 int co, bool relu, bool bias, int *launched) {
 	*launched = 0;
 	const EncodeTiledFn enc = encode_tiled();
@@ -2248,7 +2262,7 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, 
 		if (halo_plan(ci, co, 1, a)) a.RT = 1;
 	}
 	if (!a.RT) return KEL_OK;
-	CUtensorMap tx, tw;
+	CUtensorMap tx;
 	{ // x (N,H,W,Ci) as (8 channels, x, y, channel group, n)
 		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)(ci / 8), (cuuint64_t)n};
 		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, (cuuint64_t)W * ci * 2, 16, (cuuint64_t)H * W * ci * 2};
@@ -2259,16 +2273,7 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, 
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
-	{ // w (Co, 9, Ci) as (8 channels, co, tap, channel group)
-		const cuuint64_t dims[4] = {8, (cuuint64_t)co, 9, (cuuint64_t)(ci / 8)};
-		const cuuint64_t strides[3] = {(cuuint64_t)9 * ci * 2, (cuuint64_t)ci * 2, 16};
-		const cuuint32_t box[4] = {8, (cuuint32_t)a.CoT, 9, (cuuint32_t)(a.CK / 8)};
-		const cuuint32_t es[4] = {1, 1, 1, 1};
-		if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(w), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-			return KEL_OK;
-	}
+	a.pw = pw;
 	a.bias = b;
 	a.y = y;
 	a.N = n;
@@ -2283,7 +2288,7 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, 
 	a.err = U->d_err;
 	const size_t smem = (size_t)a.stages * a.stage_bytes + (size_t)a.stages * 16 + 16;
 	KEL_CUDA(allow_dynamic_smem<conv_halo>(210 * 1024));
-	conv_halo<<<(unsigned)((int64_t)n * (H / (a.RT * a.MR)) * tpr * (co / a.CoT)), 128, smem, U->stream>>>(tx, tw, a);
+	conv_halo<<<(unsigned)((int64_t)n * (H / (a.RT * a.MR)) * tpr * (co / a.CoT)), 128, smem, U->stream>>>(tx, a);
 	KEL_CUDA(cudaGetLastError());
 	*launched = 1;
 	return KEL_OK;
@@ -2335,14 +2340,14 @@ int rows_plan(const kel_unet *U, int n, int H, int W, int Ci, int Co, RowsArgs &
 }
 
 // conv_rows for one layer; returns 0 without launching when it does not fit.
-int conv_rows_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, bf16 *y, int n, int H, int W, int ci,
+int conv_rows_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b, bf16 *y, int n, int H, int W, int ci,
 					 int co, bool relu, bool bias, int *launched) {
 	*launched = 0;
 	const EncodeTiledFn enc = encode_tiled();
 	RowsArgs a;
 	memset(&a, 0, sizeof(a));
 	if (!enc || !rows_plan(U, n, H, W, ci, co, a)) return KEL_OK;
-	CUtensorMap tx, tw;
+	CUtensorMap tx;
 	{ // x (N,H,W,Ci) as (8 channels, x, channel group, y, n): one row per box
 		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(ci / 8), (cuuint64_t)H, (cuuint64_t)n};
 		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, 16, (cuuint64_t)W * ci * 2, (cuuint64_t)H * W * ci * 2};
@@ -2353,17 +2358,7 @@ int conv_rows_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, 
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
-	{ // w (Co, 3, 3, Ci) as (8 channels, co, ky, kx, channel group): the whole
-	  // tensor, in shared memory as [g][kx][ky][co][8]
-		const cuuint64_t dims[5] = {8, (cuuint64_t)co, 3, 3, (cuuint64_t)(ci / 8)};
-		const cuuint64_t strides[4] = {(cuuint64_t)9 * ci * 2, (cuuint64_t)3 * ci * 2, (cuuint64_t)ci * 2, 16};
-		const cuuint32_t box[5] = {8, (cuuint32_t)co, 3, 3, (cuuint32_t)(ci / 8)};
-		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-		if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(w), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-			return KEL_OK;
-	}
+	a.pw = pw;
 	a.bias = b;
 	a.y = y;
 	a.N = n;
@@ -2376,14 +2371,14 @@ int conv_rows_launch(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, 
 	a.err = U->d_err;
 	const size_t smem = (size_t)a.mbar_off + (2u * (size_t)a.NR + 3u + 16u) * 8u + 16u;
 	KEL_CUDA(allow_dynamic_smem<conv_rows>(210 * 1024));
-	conv_rows<<<(unsigned)((int64_t)n * (W / 128) * a.runs), 192, smem, U->stream>>>(tx, tw, a);
+	conv_rows<<<(unsigned)((int64_t)n * (W / 128) * a.runs), 192, smem, U->stream>>>(tx, a);
 	KEL_CUDA(cudaGetLastError());
 	*launched = 1;
 	return KEL_OK;
 }
 
-int conv_fwd(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, bf16 *y, int n, int level, int ci, int co,
-			 bool relu, bool bias) {
+int conv_fwd(kel_unet *U, const bf16 *x, const bf16 *w, const bf16 *pw, const float *b, bf16 *y, int n, int level, int ci,
+			 int co, bool relu, bool bias) {
 	ConvArgs a;
 	a.x = x;
 	a.w = w;
@@ -2401,9 +2396,9 @@ int conv_fwd(kel_unet *U, const bf16 *x, const bf16 *w, const float *b, bf16 *y,
 		if (ci % 16 || co % 16 || co < 16 || co > 256)
 			return fail(KEL_ERR_UNSUPPORTED, "conv: tensor-core path needs c_in, c_out multiples of 16, c_out <= 256");
 		int launched = 0, rc;
-		if ((rc = conv_rows_launch(U, x, w, b, y, n, a.H, a.W, ci, co, relu, bias, &launched))) return rc;
+		if ((rc = conv_rows_launch(U, x, pw, b, y, n, a.H, a.W, ci, co, relu, bias, &launched))) return rc;
 		if (launched) return KEL_OK;
-		if ((rc = conv_halo_launch(U, x, w, b, y, n, a.H, a.W, ci, co, relu, bias, &launched))) return rc;
+		if ((rc = conv_halo_launch(U, x, pw, b, y, n, a.H, a.W, ci, co, relu, bias, &launched))) return rc;
 		if (launched) return KEL_OK;
 		TcArgs t;
 		t.x = x;
@@ -2670,6 +2665,8 @@ int refresh(kel_unet *U) {
 		t.ci[t.nl] = l.ci;
 		t.w[t.nl] = l.w;
 		t.wf[t.nl] = l.wf;
+		t.pw[t.nl] = l.pw;
+		t.pwf[t.nl] = l.pwf;
 		++t.nl;
 		if ((int64_t)l.co * 9 * l.ci > most) most = (int64_t)l.co * 9 * l.ci;
 	}
@@ -2762,6 +2759,8 @@ extern "C" int kel_unet_create(const kel_unet_desc *desc, uint64_t seed, kel_une
 		const int64_t nw = (int64_t)l.co * 9 * l.ci;
 		if ((e = cudaMalloc(&l.w, sizeof(bf16) * nw)) != cudaSuccess) return fail_out(e);
 		if ((e = cudaMalloc(&l.wf, sizeof(bf16) * nw)) != cudaSuccess) return fail_out(e);
+		if ((e = cudaMalloc(&l.pw, sizeof(bf16) * nw)) != cudaSuccess) return fail_out(e);
+		if ((e = cudaMalloc(&l.pwf, sizeof(bf16) * nw)) != cudaSuccess) return fail_out(e);
 	}
 	U->partial_len = max_w * 64;
 	if ((e = cudaMalloc(&U->partial, sizeof(float) * U->partial_len)) != cudaSuccess) return fail_out(e);
@@ -2812,6 +2811,8 @@ extern "C" int kel_unet_destroy(kel_unet *U) {
 	for (auto &l : U->L) {
 		cudaFree(l.w);
 		cudaFree(l.wf);
+		cudaFree(l.pw);
+		cudaFree(l.pwf);
 	}
 	for (auto *p : U->act) cudaFree(p);
 	for (auto *p : U->grad) cudaFree(p);
@@ -2909,7 +2910,7 @@ extern "C" int kel_unet_forward(kel_unet *U, int32_t n, float *d_out) {
 	const int H = U->d.height, W = U->d.width;
 	auto cv = [&](int li, const bf16 *x, bf16 *y) {
 		const UnetLayer &l = L[li];
-		return conv_fwd(U, x, l.w, U->p + l.woff + (int64_t)l.co * 9 * l.ci, y, n, l.level, l.ci, l.co, true, true);
+		return conv_fwd(U, x, l.w, l.pw, U->p + l.woff + (int64_t)l.co * 9 * l.ci, y, n, l.level, l.ci, l.co, true, true);
 	};
 	if ((rc = cv(0, U->input, A[T_E0A])) || (rc = cv(1, A[T_E0A], A[T_E0B]))) return rc;
 	pool_forward<<<grid_of(telems(U, T_P0, n) / 8), 256, 0, U->stream>>>(A[T_E0B], A[T_P0], n, H, W, w[0]);
@@ -3012,7 +3013,7 @@ static int unet_backward(kel_unet *U, const float *d_target, int32_t n, double *
 		const UnetLayer &l = L[li];
 		int r = fork_side(U);
 		if (r || (r = conv_grads(U, l, x_in, G[t_out], n))) return r;
-		if (dx) r = conv_fwd(U, G[t_out], l.wf, nullptr, dx, n, l.level, l.co, l.ci, false, false);
+		if (dx) r = conv_fwd(U, G[t_out], l.wf, l.pwf, nullptr, dx, n, l.level, l.co, l.ci, false, false);
 		return r;
 	};
 	// a level's two layers: lb (output tb, gradient from src) after la (output ta), input x, gradient to dx
