@@ -215,13 +215,40 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo = 128
 	return d;
 }
 
+// The same for an operand of `cs` consecutive channels (64, 32 or 16) per pixel,
+// swizzled as the TMA leaves them (slab_swizzle): 16-byte pieces permuted by
+// higher address bits, so any pixel may be an operand's first.
+__device__ __forceinline__ uint64_t umma_desc_slab(uint32_t saddr, int cs, uint32_t lbo, uint32_t sbo) {
+	return umma_desc(saddr, lbo, sbo) | ((uint64_t)(cs == 64 ? 2 : (cs == 32 ? 4 : 6)) << 61);
+}
+
 // Descriptor of a shared-memory operand at 16-byte unit addr16 = address >> 4:
 // the address field is the low 14 bits, so adding n to the descriptor moves
 // the operand by 16 n bytes (shared addresses stay below 2^18).
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
-	asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-				 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-				 "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+__device__ __forceinline__ void umma_f16(uint32_t lead, uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t idesc,
+										 uint32_t acc) {
+	asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+				 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+				 "l"(ad), "l"(bd), "r"(idesc), "r"(acc), "r"(lead));
+}
+
+// One lane of the warp (all 32 call it): 1 there, 0 elsewhere.  The warp that
+// issues the MMAs runs its loops as a whole and only the instructions that must
+// come once are predicated by this: with uniform control the descriptors are
+// formed on the uniform path.  One diverged thread needed some 200 cycles for
+// each MMA of 16 to 64 (training step 256 x 64, batch 32: 1754 -> 1510 us,
+// inference, batch 8: 497 -> 414 us, with the swizzled slabs, which alone gave
+// nothing while the issue was the bound).
+__device__ __forceinline__ uint32_t elect_lane() {
+	uint32_t r;
+	asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.b32 %0, 1, 0, p;\n}\n" : "=r"(r));
+	return r;
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t lead, uint32_t mbar) {
+	asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+				 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(mbar),
+				 "r"(lead));
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t saddr, const void *g, bool valid) {
@@ -256,6 +283,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
 	while (!mbar_try(addr, parity))
 		if (clock64() - t0 > 2000000000ll) return false;
 	return true;
+}
+
+// The same for a whole warp, with one answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity) {
+	return __all_sync(0xffffffffu, mbar_wait(addr, parity)) != 0;
 }
 
 __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
@@ -428,14 +460,14 @@ __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
 // consecutive pixels of one image row (MR = 1) and the CTA takes RT
 // consecutive rows; the chunk's input reaches shared memory as one halo, a
 // TMA tile of RT + 2 rows x 130 pixels x CK channels at (x0 - 1 .. x0 + 128,
-// y0 - 1 .. y0 + RT), zero-filled by the copy outside the image, laid out
-// channel-group major: element (row r, pixel p, channel 8 g + e) at
-// ((g * rows + r) * P + p) * 16 + 2 e with P = 130.  Pixels are 16 bytes
-// apart within a channel group, so the A operand of tap (dy, dx) -- the 128
+// y0 - 1 .. y0 + RT), zero-filled by the copy outside the image, laid out in
+// slabs of CS = 64, 32 or 16 channels: pixel p of row r, slab g at ((g * rows +
+// r) * P + p) * 2 CS with P = 130, its 16-byte pieces swizzled (as boxes of 16-byte
+// rows, a channel group each, the halo took four to eight times the copies'
+// writes).  Pixels are evenly spaced within a slab, so the A operand of tap (dy, dx) -- the 128
 // pixels shifted by (dy, dx) -- is the same halo read through a descriptor
-// whose start moves by ((r + dy) * P + dx) * 16 bytes for tile r (K-major, no
-// swizzle: core matrices of 8 pixels x 8 channels, 8-pixel stride SBO = 128
-// B, channel-group stride LBO = rows * P * 16 B).  For a narrower layer (W
+// whose start moves by ((r + dy) * P + dx) * 2 CS bytes for tile r (K-major,
+// 8-pixel stride SBO = 16 CS).  For a narrower layer (W
 // dividing 128) a tile is MR = 128 / W whole image rows, which a single
 // descriptor covers only if consecutive rows are W pixels apart; so the halo
 // comes as NC = 3 copies of RT * MR + 2 rows x W pixels (P = W), taken at x =
@@ -460,7 +492,7 @@ struct HaloArgs {
 	const bf16 *pw; // packed weights
 	const float *bias;
 	bf16 *y; // (N,H,W,Co)
-	int N, H, W, Ci, Co, CK;
+	int N, H, W, Ci, Co, CK, CS;
 	int RT;        // accumulators (M tiles of 128 pixels) per CTA
 	int NC, P, MR; // halo copies (1, or 3 shifted by dx), pixels per copy row, image rows per M tile
 	int CoT;       // output channels per CTA (Co / CoT CTAs share a pixel tile)
@@ -494,7 +526,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 
 __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtensorMap tx, HaloArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 	const int S = a.stages;
 	uint64_t *full = reinterpret_cast<uint64_t *>(sm + (size_t)S * a.stage_bytes);
 	uint64_t *done = full + S;
@@ -530,18 +562,26 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 
 	// instruction descriptor: D f32, A bf16, B bf16, both K-major, N = Co, M = 128
 	const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.CoT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-	const uint32_t lbo_a = (uint32_t)(RT * a.MR + 2) * (uint32_t)a.P * 16u, lbo_b = 9u * (uint32_t)a.CoT * 16u;
+	const uint32_t lbo_b = 9u * (uint32_t)a.CoT * 16u;
+	// A's steps in 16-byte units: a pixel, a slab
+	const uint32_t px16 = (uint32_t)a.CS / 8u, slab16 = (uint32_t)((RT * a.MR + 2) * a.P) * px16;
+	const int kps = a.CS / 16; // MMAs of 16 channels per slab
 	// the shift dx: a pixel (one copy) or a copy (three)
-	const uint64_t dx_step = a.NC == 3 ? (uint64_t)(a.copy_bytes >> 4) : 1u;
+	const uint64_t dx_step = a.NC == 3 ? (uint64_t)(a.copy_bytes >> 4) : (uint64_t)px16;
+	const uint32_t row16 = (uint32_t)a.P * px16, tile16 = (uint32_t)a.MR * row16;
+	const uint64_t bstep = (uint64_t)(18 * a.CoT);
+	uint32_t acc = 0u;
 	int fail = 0, loaded = 0, issued = -1;
-	if (tid == 0) {
+	if (warp == 0) {
+		const uint32_t lead = elect_lane();
 		auto load = [&](int c) {
+			if (!lead) return;
 			const int s = c % S;
 			const uint32_t base = smem_u32(sm + (size_t)s * a.stage_bytes);
 			mbar_expect_tx(smem_u32(full + s), tx_bytes);
 			for (int cp = 0; cp < a.NC; ++cp)
 				tma_load_5d(base + (uint32_t)cp * a.copy_bytes, &tx, smem_u32(full + s), 0, x0 - 1 + (a.NC == 3 ? cp : 0),
-							yy - 1, c * (a.CK / 8), n);
+							yy - 1, c * (a.CK / a.CS), n);
 			const bf16 *w = a.pw + ((int64_t)c * (a.CK / 8) * 9 * a.Co + co0) * 8;
 			if (a.CoT == a.Co)
 				bulk_load(base + a.a_span, w, a.b_bytes, smem_u32(full + s));
@@ -554,7 +594,7 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 		loaded = S < nch ? S : nch;
 		for (int c = 0; c < nch; ++c) {
 			const int s = c % S;
-			if (!mbar_wait(smem_u32(full + s), (uint32_t)((c / S) & 1))) {
+			if (!mbar_wait_warp(smem_u32(full + s), (uint32_t)((c / S) & 1))) {
 				fail = 1;
 				break;
 			}
@@ -562,26 +602,32 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 			const uint32_t abase = smem_u32(sm + (size_t)s * a.stage_bytes);
 			const uint32_t bbase = abase + a.a_span;
 			// descriptors stepped by constant adds (16-byte units)
-			const uint64_t ad0 = umma_desc(abase, lbo_a, 128u), bd0 = umma_desc(bbase, lbo_b, 128u);
-			for (int j = 0; j < a.CK / 16; ++j)
-				for (int t = 0; t < 9; ++t) {
-					const int dy = t / 3, dx = t % 3;
-					const uint64_t bd = bd0 + (uint64_t)((2 * j * 9 + dx * 3 + dy) * a.CoT);
-					const uint32_t acc = (c > 0 || j > 0 || t > 0) ? 1u : 0u;
-					uint64_t ad = ad0 + (uint64_t)(2 * j) * (lbo_a >> 4) + (uint64_t)(dy * a.P) + (uint64_t)dx * dx_step;
-					for (int r = 0; r < RT; ++r) {
-						umma_f16(tmem + (uint32_t)(r * a.CoT), ad, bd, idesc, acc);
-						ad += (uint64_t)(a.MR * a.P);
+			const uint64_t ad0 = umma_desc_slab(abase, a.CS, 16u, (uint32_t)a.CS * 16u), bd0 = umma_desc(bbase, lbo_b, 128u);
+			uint64_t ag = ad0, bd = bd0;
+			for (int g = 0; g < a.CK / a.CS; ++g, ag += slab16)
+#pragma unroll 1
+				for (int k = 0; k < kps; ++k, bd += bstep) {
+#pragma unroll
+					for (int t = 0; t < 9; ++t) {
+						const int dy = t / 3, dx = t % 3;
+						uint64_t ad = ag + (uint64_t)(2 * k) + (uint64_t)((uint32_t)dy * row16) + (uint64_t)dx * dx_step;
+						uint32_t dt = tmem;
+#pragma unroll 1
+						for (int r = 0; r < RT; ++r) {
+							umma_f16(lead, dt, ad, bd + (uint64_t)((dx * 3 + dy) * a.CoT), idesc, acc);
+							ad += tile16;
+							dt += (uint32_t)a.CoT;
+						}
+						acc = 1u;
 					}
 				}
-			asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-				smem_u32(done + s)));
+			umma_commit(lead, smem_u32(done + s));
 			issued = c;
 			// refill the stage chunk c - 1 used with chunk c - 1 + S once its
 			// MMAs are done (chunk c's are queued behind them meanwhile)
 			if (c >= 1 && c - 1 + S < nch) {
 				const int cp = c - 1;
-				if (!mbar_wait(smem_u32(done + cp % S), (uint32_t)((cp / S) & 1))) {
+				if (!mbar_wait_warp(smem_u32(done + cp % S), (uint32_t)((cp / S) & 1))) {
 					fail = 1;
 					break;
 				}
@@ -590,14 +636,14 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 			}
 		}
 		// the last commit covers every MMA issued before it
-		if (issued >= 0 && !mbar_wait(smem_u32(done + issued % S), (uint32_t)((issued / S) & 1))) fail = 1;
+		if (issued >= 0 && !mbar_wait_warp(smem_u32(done + issued % S), (uint32_t)((issued / S) & 1))) fail = 1;
 		// copies issued but not consumed (after a failure): wait for them
 		// (bounded) before the CTA's shared memory can be reused
-		for (int c = issued + 1; c < loaded; ++c) mbar_wait(smem_u32(full + c % S), (uint32_t)((c / S) & 1));
-		if (fail || issued != nch - 1) atomicExch(a.err, 1);
+		for (int c = issued + 1; c < loaded; ++c) mbar_wait_warp(smem_u32(full + c % S), (uint32_t)((c / S) & 1));
+		if (lead && (fail || issued != nch - 1)) atomicExch(a.err, 1);
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-	const int failed = __syncthreads_or(tid == 0 && (fail || issued != nch - 1));
+	const int failed = __syncthreads_or(warp == 0 && (fail || issued != nch - 1));
 	asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 	if (!failed) {
 		// epilogue: warp w owns TMEM lanes (= tile pixels) 32 w .. 32 w + 31
@@ -651,10 +697,10 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 // consecutive, so B rows (ky, co) form one operand of up to 3 Co rows (8-row
 // stride 128 B, channel-group stride 9 * Co * 16 B).  Input rows y0 - 1 ..
 // y0 + RL stream once each through a ring of NR slots, each row a TMA box of
-// 130 pixels x Ci channels, zero-filled outside the image, laid out (channel
-// group, pixel, 8 channels): the A operand of input row X and shift dx is
-// the slot read from pixel dx (K-major, no swizzle: 8-pixel stride 128 B,
-// channel-group stride 130 * 16 B).  Input row X feeds output rows X + 1, X,
+// 130 pixels x Ci channels, zero-filled outside the image, laid out (slab of
+// CS channels, pixel, CS channels) and swizzled as in conv_halo: the A operand
+// of input row X and shift dx is the slot read from pixel dx (K-major, 8-pixel
+// stride 16 CS B).  Input row X feeds output rows X + 1, X,
 // X - 1 through kernel rows ky = 0, 1, 2; the accumulators of consecutive
 // output rows sit in TMEM in decreasing row order (Co columns each), so one
 // MMA with N = (number of kernel rows) x Co adds X's contribution to up to
@@ -676,7 +722,7 @@ struct RowsArgs {
 	const bf16 *pw; // packed weights
 	const float *bias;
 	bf16 *y; // (N,H,W,Co)
-	int N, H, W, Ci, Co;
+	int N, H, W, Ci, Co, CS;
 	int relu, use_bias;
 	int RL, NR, runs; // output rows per CTA, ring slots, CTAs per column tile
 	int RB, KY;       // output rows per accumulator block, kernel rows per MMA (N = KY Co <= 256)
@@ -687,7 +733,7 @@ struct RowsArgs {
 
 __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtensorMap tx, RowsArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 	const int NR = a.NR, RB = a.RB;
 	uint64_t *row_full = reinterpret_cast<uint64_t *>(sm + a.mbar_off);
 	uint64_t *row_empty = row_full + NR;
@@ -702,7 +748,6 @@ __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtenso
 	const int y0 = run * a.RL;
 	const int rows = a.H - y0 < a.RL ? a.H - y0 : a.RL;
 	const int nx = rows + 2;
-	constexpr uint32_t R = HX * 16u;
 	// TMEM column of output row r (0 .. rows - 1): block r / RB in buffer
 	// (r / RB) & 1, rows of a block in decreasing order; slot_of(r) numbers
 	// the 2 RB row slots, used by rows r, r + 2 RB, ...
@@ -754,16 +799,19 @@ __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtenso
 			if (fail) atomicExch(a.err, 1);
 		}
 	} else if (warp == 1) {
-		if (lane == 0) { // MMA issuer: input row j feeds output rows j - ky, ky = 0, 1, 2
+		{ // MMA issuer (the warp runs the loops, one lane issues): input row j feeds output rows j - ky, ky = 0, 1, 2
 			// D f32, A bf16, B bf16, both K-major, M = 128, N = nky * Co
 			const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 4) << 24);
 			const uint32_t lbo_b = 9u * (uint32_t)a.Co * 16u;
 			const uint64_t bd0 = umma_desc(smem_u32(sm + a.w_off), lbo_b, 128u);
-			const uint64_t a_k = (2u * R) >> 4, b_k = 18u * (uint64_t)a.Co;
-			const int nk = a.Ci / 16;
-			int fail = !mbar_wait(smem_u32(w_full), 0u), done = 0; // output rows committed
+			// A in 16-byte units: a pixel; from a slab's last 16 channels to the next slab
+			const uint32_t px16 = (uint32_t)a.CS / 8u, slab_step = (HX - 1) * px16;
+			const uint64_t b_k = 18u * (uint64_t)a.Co;
+			const int ns = a.Ci / a.CS, kps = a.CS / 16;
+			const uint32_t lead = elect_lane();
+			int fail = !mbar_wait_warp(smem_u32(w_full), 0u), done = 0; // output rows committed
 			for (int j = 0; j < nx && !fail; ++j) {
-				if (!mbar_wait(smem_u32(row_full + j % NR), (uint32_t)((j / NR) & 1))) {
+				if (!mbar_wait_warp(smem_u32(row_full + j % NR), (uint32_t)((j / NR) & 1))) {
 					fail = 1;
 					break;
 				}
@@ -771,14 +819,15 @@ __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtenso
 				// (and zeroed) by the epilogue
 				if (j < rows && j % RB == 0) {
 					const int blk = j / RB;
-					if (!mbar_wait(smem_u32(acc_empty + (blk & 1)), (uint32_t)((blk >> 1) & 1))) {
+					if (!mbar_wait_warp(smem_u32(acc_empty + (blk & 1)), (uint32_t)((blk >> 1) & 1))) {
 						fail = 1;
 						break;
 					}
 				}
 				asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 				const int kmin = j - rows + 1 > 0 ? j - rows + 1 : 0, kmax = j < 2 ? j : 2;
-				const uint64_t ad_row = umma_desc(smem_u32(sm + (size_t)(j % NR) * a.row_span), R, 128u);
+				const uint64_t ad_row =
+					umma_desc_slab(smem_u32(sm + (size_t)(j % NR) * a.row_span), a.CS, 16u, (uint32_t)a.CS * 16u);
 				// groups of kernel rows [k0, k1] whose output rows share a block
 				for (int k0 = kmin; k0 <= kmax;) {
 					int k1 = k0;
@@ -787,32 +836,30 @@ __global__ void __launch_bounds__(192) conv_rows(const __grid_constant__ CUtenso
 					const uint32_t idesc = idesc0 | ((uint32_t)((nky * a.Co) >> 3) << 17);
 					const uint32_t d_tmem = tmem + col_of(j - k0);
 					for (int dx = 0; dx < 3; ++dx) {
-						uint64_t ad = ad_row + (uint64_t)dx;
+						uint64_t ad = ad_row + (uint64_t)((uint32_t)dx * px16);
 						uint64_t bd = bd0 + (uint64_t)((dx * 3 + k0) * a.Co);
-#pragma unroll 2
-						for (int k = 0; k < nk; ++k) {
-							umma_f16(d_tmem, ad, bd, idesc, 1u);
-							ad += a_k;
-							bd += b_k;
-						}
+						for (int g = 0; g < ns; ++g, ad += slab_step)
+							for (int k = 0; k < kps; ++k) {
+								umma_f16(lead, d_tmem, ad, bd, idesc, 1u);
+								ad += 2u;
+								bd += b_k;
+							}
 					}
 					k0 = k1 + 1;
 				}
 				// input row j is read by no later MMA
-				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-					smem_u32(row_empty + j % NR)));
+				umma_commit(lead, smem_u32(row_empty + j % NR));
 				// output row j - 2 is complete
 				const int rl = j - 2;
 				if (rl >= 0 && rl < rows) {
-					asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-						smem_u32(row_done + slot_of(rl))));
+					umma_commit(lead, smem_u32(row_done + slot_of(rl)));
 					done = rl + 1;
 				}
 			}
 			// the MMAs and their arrivals have finished before TMEM is freed
 			if (done > 0)
-				mbar_wait(smem_u32(row_done + slot_of(done - 1)), (uint32_t)(((done - 1) / (2 * RB)) & 1));
-			if (fail) atomicExch(a.err, 1);
+				mbar_wait_warp(smem_u32(row_done + slot_of(done - 1)), (uint32_t)(((done - 1) / (2 * RB)) & 1));
+			if (fail && lead) atomicExch(a.err, 1);
 		}
 	} else { // epilogue: warp w reads TMEM lanes (pixels) 32 (w % 4) .. + 31
 		const int q = warp & 3;
@@ -1078,13 +1125,13 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc(TcWgradArgs a) {
 // input channel ci) pairs, N = Co, K = the WT pixels of a row tile (WT = W,
 // at most 128).  Per row tile the input arrives as one TMA box of rows_box
 // halo rows x (WT + 2) pixels x CT channels, zero-filled outside the image,
-// laid out halo row major: element (row r, channel group g, pixel p, channel
-// e) at ((r * CT / 8 + g) * (WT + 2) + p) * 16 + 2 e.  The 8-row groups of M
-// (channel groups, then halo rows) are then R = (WT + 2) * 16 bytes apart --
-// the descriptor's stride byte offset -- and pixels 16 bytes apart, so the
-// shift dx only moves the descriptor's start by 16 dx bytes (MN-major, no
-// swizzle: core matrices of 8 pixels x 8 channels, K-direction stride 128 B).
-// dY arrives as (channel group, pixel, 8 channels), N-direction stride WT * 16.
+// laid out halo row major in slabs of CS = 64, 32 or 16 channels: pixel p of
+// row r, slab g at ((r * CT / CS + g) * (WT + 2) + p) * 2 CS, its 16-byte pieces
+// swizzled as in conv_halo.  The slabs of M (those of a halo row, then the next row's)
+// are then R = (WT + 2) * 2 CS bytes apart -- the descriptor's leading byte
+// offset -- and pixels 2 CS, so the shift dx only moves the descriptor's start
+// by 2 CS dx bytes (MN-major, 8-pixel stride 16 CS).  dY arrives as (slab of CSy
+// channels, pixel, CSy channels), N-direction stride WT * 2 CSy.
 // With CT <= 32 channels per tile one accumulator holds all three halo rows
 // (RPM = 3 rows per MMA, 3 CT of its 128 rows used); with CT = 128 each halo
 // row is a row group of its own (RPM = 1), and when 9 Co columns do not fit
@@ -1098,6 +1145,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc(TcWgradArgs a) {
 struct WhaloArgs {
 	float *partial; // (chunks, Co, 9 Ci)
 	int N, H, W, Ci, Co;
+	int CS, CSy;            // slabs of x and dY
 	int WT, CT, RPM, RG;    // row tile width, channels per tile, halo rows per MMA, row groups
 	int rg_cta, rows_box;   // row groups per CTA, halo rows per TMA box
 	int ci_tiles, cta_groups;
@@ -1113,7 +1161,7 @@ struct WhaloArgs {
 __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ CUtensorMap tx,
 													   const __grid_constant__ CUtensorMap tdy, WhaloArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 	const int S = a.stages;
 	uint64_t *full = reinterpret_cast<uint64_t *>(sm + a.mbar_off);
 	uint64_t *done = full + S;
@@ -1128,8 +1176,9 @@ __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ C
 	const int nsteps = (int)(t1 - t0);
 	const int tpr = a.W / a.WT;
 	const int row0 = grp * a.rg_cta * a.RPM; // first halo row of this CTA (0: y - 1)
-	const int cg = a.CT / 8;
-	const uint32_t R = (uint32_t)(a.WT + 2) * 16u;
+	const int cg = a.CT / a.CS;
+	const uint32_t px = (uint32_t)a.CS * 2u, pxy = (uint32_t)a.CSy * 2u; // bytes of a pixel in a slab
+	const uint32_t R = (uint32_t)(a.WT + 2) * px;
 	const uint32_t grp_bytes = (uint32_t)(a.RPM * cg) * R;
 	const int nk = a.WT / 16;
 
@@ -1154,8 +1203,10 @@ __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ C
 	const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
 						   ((uint32_t)(a.Co >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 	int fail = 0, loaded = 0, issued = -1;
-	if (tid == 0) {
+	if (warp == 0) {
+		const uint32_t lead = elect_lane();
 		auto load = [&](int i) {
+			if (!lead) return;
 			const int s = i % S;
 			const int64_t t = t0 + i;
 			const int xt = (int)(t % tpr);
@@ -1171,7 +1222,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ C
 		loaded = S < nsteps ? S : nsteps;
 		for (int i = 0; i < nsteps; ++i) {
 			const int s = i % S;
-			if (!mbar_wait(smem_u32(full + s), (uint32_t)((i / S) & 1))) {
+			if (!mbar_wait_warp(smem_u32(full + s), (uint32_t)((i / S) & 1))) {
 				fail = 1;
 				break;
 			}
@@ -1180,24 +1231,24 @@ __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ C
 			const uint32_t db = smem_u32(sm + a.dy_off + (size_t)s * a.dy_span);
 			// descriptors stepped by constant adds (16-byte units): a k-step
 			// moves both operands by 16 pixels
-			const uint64_t ad0 = umma_desc(xb, 128u, R), bd0 = umma_desc(db, 128u, (uint32_t)a.WT * 16u);
+			const uint64_t ad0 = umma_desc_slab(xb, a.CS, R, 8u * px);
+			const uint64_t bd0 = umma_desc_slab(db, a.CSy, (uint32_t)a.WT * pxy, 8u * pxy);
 			for (int k = 0; k < nk; ++k) {
-				const uint64_t bd = bd0 + (uint64_t)(16 * k);
+				const uint64_t bd = bd0 + (uint64_t)((uint32_t)k * pxy);
 				const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
 				for (int g = 0; g < a.rg_cta; ++g) {
-					const uint64_t ad = ad0 + (uint64_t)g * (grp_bytes >> 4) + (uint64_t)(16 * k);
+					const uint64_t ad = ad0 + (uint64_t)g * (grp_bytes >> 4) + (uint64_t)((uint32_t)k * px);
 					for (int dx = 0; dx < 3; ++dx)
-						umma_f16(tmem + (uint32_t)((g * 3 + dx) * a.Co), ad + (uint64_t)dx, bd, idesc, acc);
+						umma_f16(lead, tmem + (uint32_t)((g * 3 + dx) * a.Co), ad + (uint64_t)((uint32_t)dx * (px >> 4)), bd, idesc, acc);
 				}
 			}
-			asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-				smem_u32(done + s)));
+			umma_commit(lead, smem_u32(done + s));
 			issued = i;
 			// refill the stage tile i - 1 used once its MMAs are done (tile
 			// i's are queued behind them meanwhile)
 			if (i >= 1 && i - 1 + S < nsteps) {
 				const int ip = i - 1;
-				if (!mbar_wait(smem_u32(done + ip % S), (uint32_t)((ip / S) & 1))) {
+				if (!mbar_wait_warp(smem_u32(done + ip % S), (uint32_t)((ip / S) & 1))) {
 					fail = 1;
 					break;
 				}
@@ -1205,12 +1256,12 @@ __global__ void __launch_bounds__(128) conv_wgrad_halo(const __grid_constant__ C
 				++loaded;
 			}
 		}
-		if (issued >= 0 && !mbar_wait(smem_u32(done + issued % S), (uint32_t)((issued / S) & 1))) fail = 1;
-		for (int i = issued + 1; i < loaded; ++i) mbar_wait(smem_u32(full + i % S), (uint32_t)((i / S) & 1));
-		if (fail || issued != nsteps - 1) atomicExch(a.err, 1);
+		if (issued >= 0 && !mbar_wait_warp(smem_u32(done + issued % S), (uint32_t)((issued / S) & 1))) fail = 1;
+		for (int i = issued + 1; i < loaded; ++i) mbar_wait_warp(smem_u32(full + i % S), (uint32_t)((i / S) & 1));
+		if (lead && (fail || issued != nsteps - 1)) atomicExch(a.err, 1);
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-	const int failed = __syncthreads_or(tid == 0 && (fail || issued != nsteps - 1));
+	const int failed = __syncthreads_or(warp == 0 && (fail || issued != nsteps - 1));
 	asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 	if (!failed && warp * 32 < a.RPM * a.CT) {
 		// warp w owns TMEM lanes 32 w .. 32 w + 31: lane L = (halo row r, channel ci)
@@ -2199,12 +2250,21 @@ cudaError_t allow_dynamic_smem(int bytes) {
 	return e;
 }
 
-// Channel chunk and stage count of conv_halo: the largest chunk (64, 48, 32 or
+// Channels of a pixel that lie together in shared memory, and their swizzle:
+// the TMA writes a pixel's 2 CS bytes per cycle, the MMAs read 8 pixels without
+// bank conflicts.
+int slab_channels(int c) { return c % 64 == 0 ? 64 : (c % 32 == 0 ? 32 : 16); }
+
+CUtensorMapSwizzle slab_swizzle(int cs) {
+	return cs == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : (cs == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+}
+
+// Channel chunk and stage count of conv_halo: the first chunk (64, 32, 48 or
 // 16 channels dividing Ci) whose stages (up to three, at least two when there
 // are two chunks or more) fit 110 KB (two CTAs per SM), else 200 KB; 0: none.
 int halo_plan(int Ci, int Co, int RT, HaloArgs &a) {
 	for (const uint32_t cap : {110u * 1024u, 200u * 1024u})
-		for (const int ck : {64, 48, 32, 16}) {
+		for (const int ck : {64, 32, 48, 16}) {
 			if (Ci % ck) continue;
 			const int nch = Ci / ck;
 			const uint32_t cb = (uint32_t)(RT * a.MR + 2) * (uint32_t)a.P * (uint32_t)ck * 2u;
@@ -2214,6 +2274,7 @@ int halo_plan(int Ci, int Co, int RT, HaloArgs &a) {
 			while (S > 1 && (uint64_t)S * stage + 1024 > cap) --S;
 			if ((nch > 1 && S < 2) || (uint64_t)S * stage + 1024 > cap) continue;
 			a.CK = ck;
+			a.CS = slab_channels(ck);
 			a.stages = S;
 			a.copy_bytes = cb;
 			a.a_bytes = ab;
@@ -2263,13 +2324,14 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b,
 	}
 	if (!a.RT) return KEL_OK;
 	CUtensorMap tx;
-	{ // x (N,H,W,Ci) as (8 channels, x, y, channel group, n)
-		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)(ci / 8), (cuuint64_t)n};
-		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, (cuuint64_t)W * ci * 2, 16, (cuuint64_t)H * W * ci * 2};
-		const cuuint32_t box[5] = {8, (cuuint32_t)a.P, (cuuint32_t)(a.RT * a.MR + 2), (cuuint32_t)(a.CK / 8), 1};
+	{ // x (N,H,W,Ci) as (CS channels, x, y, slab, n)
+		const cuuint64_t cs = (cuuint64_t)a.CS;
+		const cuuint64_t dims[5] = {cs, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)ci / cs, (cuuint64_t)n};
+		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, (cuuint64_t)W * ci * 2, cs * 2, (cuuint64_t)H * W * ci * 2};
+		const cuuint32_t box[5] = {(cuuint32_t)cs, (cuuint32_t)a.P, (cuuint32_t)(a.RT * a.MR + 2), (cuuint32_t)(a.CK / a.CS), 1};
 		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
 		if (enc(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(x), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+				CU_TENSOR_MAP_INTERLEAVE_NONE, slab_swizzle(a.CS), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
@@ -2302,7 +2364,8 @@ int rows_plan(const kel_unet *U, int n, int H, int W, int Ci, int Co, RowsArgs &
 	if (W % 128 || Ci % 16 || Co % 16 || Co < 16 || Co > 256 || H < 1) return 0;
 	a.NR = 4;
 	a.row_bytes = (uint32_t)HX * (uint32_t)Ci * 2u;
-	a.row_span = (a.row_bytes + 127u) / 128u * 128u;
+	a.CS = slab_channels(Ci);
+	a.row_span = align1k(a.row_bytes);
 	a.w_bytes = (uint32_t)Co * 9u * (uint32_t)Ci * 2u;
 	a.w_off = (uint32_t)a.NR * a.row_span;
 	a.mbar_off = a.w_off + (a.w_bytes + 127u) / 128u * 128u;
@@ -2348,13 +2411,14 @@ int conv_rows_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b,
 	memset(&a, 0, sizeof(a));
 	if (!enc || !rows_plan(U, n, H, W, ci, co, a)) return KEL_OK;
 	CUtensorMap tx;
-	{ // x (N,H,W,Ci) as (8 channels, x, channel group, y, n): one row per box
-		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(ci / 8), (cuuint64_t)H, (cuuint64_t)n};
-		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, 16, (cuuint64_t)W * ci * 2, (cuuint64_t)H * W * ci * 2};
-		const cuuint32_t box[5] = {8, HX, (cuuint32_t)(ci / 8), 1, 1};
+	{ // x (N,H,W,Ci) as (CS channels, x, slab, y, n): one row per box
+		const cuuint64_t cs = (cuuint64_t)a.CS;
+		const cuuint64_t dims[5] = {cs, (cuuint64_t)W, (cuuint64_t)ci / cs, (cuuint64_t)H, (cuuint64_t)n};
+		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, cs * 2, (cuuint64_t)W * ci * 2, (cuuint64_t)H * W * ci * 2};
+		const cuuint32_t box[5] = {(cuuint32_t)cs, HX, (cuuint32_t)ci / (cuuint32_t)a.CS, 1, 1};
 		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
 		if (enc(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(x), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+				CU_TENSOR_MAP_INTERLEAVE_NONE, slab_swizzle(a.CS), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
@@ -2449,6 +2513,8 @@ int whalo_plan(int Ci, int Co, int W, WhaloArgs &a) {
 	a.rg_cta = a.RG * 3 * Co <= 512 ? a.RG : 1;
 	if (a.rg_cta * 3 * Co > 512) return 0;
 	a.cta_groups = a.RG / a.rg_cta;
+	a.CS = slab_channels(a.CT);
+	a.CSy = slab_channels(Co);
 	a.ci_tiles = Ci / a.CT;
 	a.rows_box = a.rg_cta * a.RPM;
 	const uint32_t R = (uint32_t)(a.WT + 2) * 16u, cg = (uint32_t)a.CT / 8u;
@@ -2527,23 +2593,25 @@ int wgrad_halo_launch(kel_unet *U, const UnetLayer &l, const bf16 *x, const bf16
 	const int H = U->d.height >> l.level, W = U->d.width >> l.level;
 	if (!enc || !whalo_plan(l.ci, l.co, W, a)) return KEL_OK;
 	CUtensorMap tx, tdy;
-	{ // x (N,H,W,Ci) as (8 channels, x, channel group, y, n)
-		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(l.ci / 8), (cuuint64_t)H, (cuuint64_t)n};
-		const cuuint64_t strides[4] = {(cuuint64_t)l.ci * 2, 16, (cuuint64_t)W * l.ci * 2, (cuuint64_t)H * W * l.ci * 2};
-		const cuuint32_t box[5] = {8, (cuuint32_t)(a.WT + 2), (cuuint32_t)(a.CT / 8), (cuuint32_t)a.rows_box, 1};
+	{ // x (N,H,W,Ci) as (CS channels, x, slab, y, n)
+		const cuuint64_t cs = (cuuint64_t)a.CS;
+		const cuuint64_t dims[5] = {cs, (cuuint64_t)W, (cuuint64_t)l.ci / cs, (cuuint64_t)H, (cuuint64_t)n};
+		const cuuint64_t strides[4] = {(cuuint64_t)l.ci * 2, cs * 2, (cuuint64_t)W * l.ci * 2, (cuuint64_t)H * W * l.ci * 2};
+		const cuuint32_t box[5] = {(cuuint32_t)cs, (cuuint32_t)(a.WT + 2), (cuuint32_t)(a.CT / a.CS), (cuuint32_t)a.rows_box, 1};
 		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
 		if (enc(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(x), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+				CU_TENSOR_MAP_INTERLEAVE_NONE, slab_swizzle(a.CS), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
-	{ // dY (N,H,W,Co) as (8 channels, x, channel group, y, n)
-		const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(l.co / 8), (cuuint64_t)H, (cuuint64_t)n};
-		const cuuint64_t strides[4] = {(cuuint64_t)l.co * 2, 16, (cuuint64_t)W * l.co * 2, (cuuint64_t)H * W * l.co * 2};
-		const cuuint32_t box[5] = {8, (cuuint32_t)a.WT, (cuuint32_t)(l.co / 8), 1, 1};
+	{ // dY (N,H,W,Co) as (CSy channels, x, slab, y, n)
+		const cuuint64_t cs = (cuuint64_t)a.CSy;
+		const cuuint64_t dims[5] = {cs, (cuuint64_t)W, (cuuint64_t)l.co / cs, (cuuint64_t)H, (cuuint64_t)n};
+		const cuuint64_t strides[4] = {(cuuint64_t)l.co * 2, cs * 2, (cuuint64_t)W * l.co * 2, (cuuint64_t)H * W * l.co * 2};
+		const cuuint32_t box[5] = {(cuuint32_t)cs, (cuuint32_t)a.WT, (cuuint32_t)(l.co / a.CSy), 1, 1};
 		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
 		if (enc(&tdy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(dy), dims, strides, box, es,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+				CU_TENSOR_MAP_INTERLEAVE_NONE, slab_swizzle(a.CSy), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 			return KEL_OK;
 	}
