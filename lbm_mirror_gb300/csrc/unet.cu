@@ -2401,10 +2401,11 @@ int rows_plan(const kel_unet *U, int n, int H, int W, int Ci, int Co, RowsArgs &
 	const int smem_per_sm = (int)((227u * 1024u) / (smem + 1024u));
 	// accumulator blocks of RB output rows, up to three kernel rows per MMA:
 	// RB as large as the TMEM share of the CTAs that shared memory lets onto
-	// an SM allows (up to four CTAs, at most 8 rows).  RB >= 2: the three
+	// an SM allows (up to two CTAs, at most 8 rows: with four CTAs and rings of
+	// half the rows the training step took 1396 us, 1361 with two).  RB >= 2: the three
 	// output rows an input row feeds must lie in the two buffered blocks, or
 	// the MMAs would wait for a block that they have yet to complete.
-	const int share = 512 / (smem_per_sm < 1 ? 1 : (smem_per_sm > 4 ? 4 : smem_per_sm));
+	const int share = 512 / (smem_per_sm < 1 ? 1 : (smem_per_sm > 2 ? 2 : smem_per_sm));
 	a.RB = 2;
 	a.lring = 2;
 	while (a.RB < 8 && 4 * a.RB * Co <= share) { // a power of two, for the ring's index arithmetic
