@@ -462,37 +462,37 @@ __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
 
 // ---- the convolution from a TMA-loaded halo ----------------------------------------
 //
-// One CTA computes RT M tiles of 128 pixels by all Co outputs, each tile in
-// its own TMEM accumulator; the weights of a chunk of CK input channels serve
-// all RT tiles.  For a layer whose width is a multiple of 128 a tile is 128
-// consecutive pixels of one image row (MR = 1) and the CTA takes RT
-// consecutive rows; the chunk's input reaches shared memory as one halo, a
-// TMA tile of RT + 2 rows x 130 pixels x CK channels at (x0 - 1 .. x0 + 128,
-// y0 - 1 .. y0 + RT), zero-filled by the copy outside the image, laid out in
-// slabs of CS = 64, 32 or 16 channels: pixel p of row r, slab g at ((g * rows +
-// r) * P + p) * 2 CS with P = 130, its 16-byte pieces swizzled (as boxes of 16-byte
-// rows, a channel group each, the halo took four to eight times the copies'
-// writes).  Pixels are evenly spaced within a slab, so the A operand of tap (dy, dx) -- the 128
-// pixels shifted by (dy, dx) -- is the same halo read through a descriptor
-// whose start moves by ((r + dy) * P + dx) * 2 CS bytes for tile r (K-major,
-// 8-pixel stride SBO = 16 CS).  For a narrower layer (W
-// dividing 128) a tile is MR = 128 / W whole image rows, which a single
-// descriptor covers only if consecutive rows are W pixels apart; so the halo
-// comes as NC = 3 copies of RT * MR + 2 rows x W pixels (P = W), taken at x =
-// -1, 0, +1 (zero-filled at the image edge), and the shift dx selects the
-// copy instead of moving by a pixel.  The nine taps of a chunk read one
-// halo, where an im2col tile holds every input value nine times.  The chunk's
-// weights (Co x 9 x CK) lie in global memory as they do in shared memory, [g][dx]
-// [dy][co][8 channels] (UnetLayer::pw), and arrive as one bulk copy (a copy per
-// group and tap where the CTA has half of the channels): as a TMA box of 16-byte
-// rows they took most of a CTA's staging time (training step 256 x 64, batch
-// 32: 1903 -> 1754 us with conv_rows).  B of
-// tap (dy, dx) and channel groups 2j, 2j + 1 at ((2 j) * 9 + 3 dx + dy) * Co *
-// 16, LBO = 9 * Co * 16, SBO = 128.  One thread issues the copies (one mbarrier per stage counts
-// their bytes) and the MMAs (committed to the stage's second mbarrier, which
-// frees the stage for the chunk S later).  Every wait is bounded; on timeout
-// the CTA records the failure in *err, waits (bounded) for the copies it
-// issued, and frees its TMEM.
+// One CTA computes RT M tiles of 128 pixels by all Co outputs (or half of them),
+// each tile in its own TMEM accumulator.  The input reaches shared memory as a
+// halo, TMA boxes of HR rows x P pixels x CS = 64, 32 or 16 channels (a slab),
+// from x = -1 and the row above, zero-filled by the copy outside the image: pixel
+// p of row r at (r * P + p) * 2 CS, its 16-byte pieces swizzled.  Pixels are
+// evenly spaced, so the A operand of tap (dy, dx) is 128 pixels of the same slab
+// read through a descriptor whose start moves by (dy * P + dx) * 2 CS bytes
+// (K-major, 8-pixel stride SBO = 16 CS); an im2col tile would hold every input
+// nine times.
+//  - W a multiple of 128: a tile is 128 pixels of one image row, the CTA's tiles
+//    are RT consecutive rows, P = 130, HR = RT + 2.
+//  - a narrower layer (W dividing 128): the image is taken as one line of pixels
+//    with rows of P = W + 2, of which a tile is 128 in a row and the next tile
+//    the 128 after them.  Outputs at the two last positions of a row and below
+//    the image are not stored (3 % of the positions at W = 64, 6 % at 32).
+// A box's row of pixels takes the TMA about 4.5 cycles per pixel, whether 32 or
+// 64 bytes of channels are taken (9,360 pixels in 41 us, 13,300 in 31 us), which
+// bound the form with three halo copies shifted by dx and a slab per 16 channels
+// (64-pixel level, 256 -> 128 channels, batch 32: 40 us, now PERF11).  So a slab
+// holds as many channels as fit, and the weights have stages of their own, of 16
+// channels.  They lie in global memory as they do in shared memory, [g][dx][dy][co]
+// [8 channels] (UnetLayer::pw), and arrive as one bulk copy (a copy per group and
+// tap where the CTA has half of the channels): as TMA boxes of 16-byte rows they
+// took most of a CTA's staging time (training step 256 x 64, batch 32: 1903 ->
+// 1754 us with conv_rows).  B of tap (dy, dx) at (3 dx + dy) * Co * 16, LBO =
+// 9 * Co * 16, SBO = 128.  One lane issues the copies (an mbarrier per stage
+// counts their bytes) and the MMAs; those of 16 channels are committed to the
+// weight stage's second mbarrier, which frees that stage and, after a slab's
+// last channels, the slab's.  Every wait is bounded; on timeout the CTA records
+// the failure in *err, waits (bounded) for the copies it issued, and frees its
+// TMEM.
 
 constexpr int HX = 130; // halo pixels per row
 
@@ -500,15 +500,15 @@ struct HaloArgs {
 	const bf16 *pw; // packed weights
 	const float *bias;
 	bf16 *y; // (N,H,W,Co)
-	int N, H, W, Ci, Co, CK, CS;
+	int N, H, W, Ci, Co, CS;
 	int RT;        // accumulators (M tiles of 128 pixels) per CTA
-	int NC, P, MR; // halo copies (1, or 3 shifted by dx), pixels per copy row, image rows per M tile
+	int P, HR;     // pixels per halo row, halo rows
 	int CoT;       // output channels per CTA (Co / CoT CTAs share a pixel tile)
+	int ctas;      // CTAs per image (narrow layers), pixel tiles only
 	int relu, use_bias;
-	int stages;
-	uint32_t copy_bytes;       // one halo copy of a chunk
-	uint32_t a_bytes, b_bytes; // bytes of a chunk's halo (NC copies) and weights
-	uint32_t a_span, stage_bytes; // B's offset in a stage and the stage size (1024-byte multiples)
+	int SA, SB;    // stages of slabs and of weights
+	uint32_t a_bytes, a_span; // a slab, and its stage (a multiple of 1024)
+	uint32_t b_bytes;         // weights of 16 channels
 	uint32_t tmem_cols;
 	int *err;
 };
@@ -541,23 +541,30 @@ template <int CS, int RT>
 __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtensorMap tx, HaloArgs a) {
 	extern __shared__ __align__(1024) uint8_t sm[];
 	const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-	const int S = a.stages;
-	uint64_t *full = reinterpret_cast<uint64_t *>(sm + (size_t)S * a.stage_bytes);
-	uint64_t *done = full + S;
-	uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + S);
+	const int SA = a.SA, SB = a.SB;
+	uint8_t *const sb = sm + (size_t)SA * a.a_span;
+	uint64_t *fulla = reinterpret_cast<uint64_t *>(sb + (size_t)SB * a.b_bytes);
+	uint64_t *full = fulla + SA;
+	uint64_t *done = full + SB;
+	uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + SB);
 
-	const int tpr = a.W >= 128 ? a.W / 128 : 1; // tiles per row
+	const bool wide = a.W >= 128;
 	const int cot = a.Co / a.CoT;
 	const int co0 = (int)(blockIdx.x % cot) * a.CoT;
 	const int tile = (int)(blockIdx.x / cot);
-	const int x0 = (tile % tpr) * 128;
-	const int row = (tile / tpr) * a.RT * a.MR; // n * H + y0
-	const int n = row / a.H, yy = row - n * a.H;
-	const int nch = a.Ci / a.CK;
-	const uint32_t tx_bytes = a.a_bytes + a.b_bytes;
+	// wide: rows yy .. of image n from pixel x0; narrow: positions q0 .. of image n's line
+	const int tpr = wide ? a.W / 128 : 1; // tiles per row
+	const int x0 = wide ? (tile % tpr) * 128 : 0;
+	const int per_image = wide ? a.H / RT : a.ctas, t_image = tile / tpr;
+	const int n = t_image / per_image, first = t_image - n * per_image;
+	const int q0 = wide ? 0 : first * RT * 128;
+	const int yy = wide ? first * RT : q0 / a.P;
+	const int nk = a.Ci / 16;
 
 	if (tid == 0) {
-		for (int s = 0; s < S; ++s) {
+		for (int s = 0; s < SA; ++s)
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(fulla + s)));
+		for (int s = 0; s < SB; ++s) {
 			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(full + s)));
 			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(done + s)));
 		}
@@ -578,92 +585,94 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 	// instruction descriptor: D f32, A bf16, B bf16, both K-major, N = Co, M = 128
 	const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.CoT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 	const uint32_t lbo_b = 9u * (uint32_t)a.CoT * 16u;
-	// A's steps in 16-byte units: a pixel, a slab
+	// A's steps in 16-byte units: a pixel, a halo row, a tile
 	constexpr uint32_t px16 = (uint32_t)CS / 8u;
-	const uint32_t slab16 = (uint32_t)((RT * a.MR + 2) * a.P) * px16;
-	constexpr int kps = CS / 16; // MMAs of 16 channels per slab
-	// the shift dx: a pixel (one copy) or a copy (three)
-	const uint32_t dx_step = a.NC == 3 ? a.copy_bytes >> 4 : px16;
-	const uint32_t row16 = (uint32_t)a.P * px16, tile16 = (uint32_t)a.MR * row16;
-	const uint32_t bstep = (uint32_t)(18 * a.CoT);
+	constexpr int kps = CS / 16; // weight stages per slab
+	const uint32_t row16 = (uint32_t)a.P * px16, tile16 = wide ? row16 : 128u * px16;
+	const uint32_t off16 = (uint32_t)(q0 - (wide ? 0 : yy * a.P)) * px16; // the first tile's start
+	const int ns = a.Ci / CS;
 	uint32_t acc = 0u;
-	int fail = 0, loaded = 0, issued = -1;
+	int fail = 0, loaded = 0, loaded_a = 0, issued = -1;
 	if (warp == 0) {
 		const uint32_t lead = elect_lane();
-		auto load = [&](int c) {
+		auto load_a = [&](int g) {
 			if (!lead) return;
-			const int s = c % S;
-			const uint32_t base = smem_u32(sm + (size_t)s * a.stage_bytes);
-			mbar_expect_tx(smem_u32(full + s), tx_bytes);
-			for (int cp = 0; cp < a.NC; ++cp)
-				tma_load_5d(base + (uint32_t)cp * a.copy_bytes, &tx, smem_u32(full + s), 0, x0 - 1 + (a.NC == 3 ? cp : 0),
-							yy - 1, c * (a.CK / CS), n);
-			const bf16 *w = a.pw + ((int64_t)c * (a.CK / 8) * 9 * a.Co + co0) * 8;
-			if (a.CoT == a.Co)
-				bulk_load(base + a.a_span, w, a.b_bytes, smem_u32(full + s));
-			else
-				for (int k = 0; k < a.CK / 8 * 9; ++k)
-					bulk_load(base + a.a_span + (uint32_t)(k * a.CoT) * 16u, w + (int64_t)k * a.Co * 8, (uint32_t)a.CoT * 16u,
-							  smem_u32(full + s));
+			mbar_expect_tx(smem_u32(fulla + g % SA), a.a_bytes);
+			tma_load_5d(smem_u32(sm + (size_t)(g % SA) * a.a_span), &tx, smem_u32(fulla + g % SA), 0, x0 - 1, yy - 1, g, n);
 		};
-		for (int c = 0; c < S && c < nch; ++c) load(c);
-		loaded = S < nch ? S : nch;
-		for (int c = 0; c < nch; ++c) {
-			const int s = c % S;
-			if (!mbar_wait_warp(smem_u32(full + s), (uint32_t)((c / S) & 1))) {
+		auto load_b = [&](int k) {
+			if (!lead) return;
+			const uint32_t to = smem_u32(sb + (size_t)(k % SB) * a.b_bytes), bar = smem_u32(full + k % SB);
+			mbar_expect_tx(bar, a.b_bytes);
+			const bf16 *w = a.pw + ((int64_t)k * 18 * a.Co + co0) * 8;
+			if (a.CoT == a.Co)
+				bulk_load(to, w, a.b_bytes, bar);
+			else
+				for (int t = 0; t < 18; ++t)
+					bulk_load(to + (uint32_t)(t * a.CoT) * 16u, w + (int64_t)t * a.Co * 8, (uint32_t)a.CoT * 16u, bar);
+		};
+		for (; loaded_a < SA && loaded_a < ns; ++loaded_a) load_a(loaded_a);
+		for (; loaded < SB && loaded < nk; ++loaded) load_b(loaded);
+		for (int g = 0; g < ns && !fail; ++g) {
+			if (!mbar_wait_warp(smem_u32(fulla + g % SA), (uint32_t)((g / SA) & 1))) {
 				fail = 1;
 				break;
 			}
-			asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-			const uint32_t abase = smem_u32(sm + (size_t)s * a.stage_bytes);
-			const uint32_t bbase = abase + a.a_span;
-			// descriptors stepped by constant adds (16-byte units)
-			const Desc ad0 = umma_desc_slab(abase, CS, 16u, (uint32_t)CS * 16u), bd0 = umma_desc(bbase, lbo_b, 128u);
-			uint32_t ag = 0u, bg = 0u;
+			const Desc ad0 = Desc(umma_desc_slab(smem_u32(sm + (size_t)(g % SA) * a.a_span), CS, 16u, (uint32_t)CS * 16u)) + off16;
 #pragma unroll 1
-			for (int g = 0; g < a.CK / CS; ++g, ag += slab16)
-#pragma unroll 1
-				for (int k = 0; k < kps; ++k, bg += bstep)
-#pragma unroll
-					for (int t = 0; t < 9; ++t) {
-						const int dy = t / 3, dx = t % 3;
-						const Desc ad = ad0 + (ag + 2u * (uint32_t)k + (uint32_t)dy * row16 + (uint32_t)dx * dx_step);
-						const Desc bd = bd0 + (bg + (uint32_t)((dx * 3 + dy) * a.CoT));
-#pragma unroll
-						for (int r = 0; r < RT; ++r)
-							umma_f16(lead, tmem + (uint32_t)(r * a.CoT), ad + (uint32_t)r * tile16, bd, idesc, acc);
-						acc = 1u;
-					}
-			umma_commit(lead, smem_u32(done + s));
-			issued = c;
-			// refill the stage chunk c - 1 used with chunk c - 1 + S once its
-			// MMAs are done (chunk c's are queued behind them meanwhile)
-			if (c >= 1 && c - 1 + S < nch) {
-				const int cp = c - 1;
-				if (!mbar_wait_warp(smem_u32(done + cp % S), (uint32_t)((cp / S) & 1))) {
+			for (int kk = 0; kk < kps; ++kk) {
+				const int k = g * kps + kk, s = k % SB;
+				if (!mbar_wait_warp(smem_u32(full + s), (uint32_t)((k / SB) & 1))) {
 					fail = 1;
 					break;
 				}
-				load(cp + S);
-				++loaded;
+				asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+				const Desc bd0 = umma_desc(smem_u32(sb + (size_t)s * a.b_bytes), lbo_b, 128u);
+#pragma unroll
+				for (int t = 0; t < 9; ++t) {
+					const int dy = t / 3, dx = t % 3;
+					const Desc ad = ad0 + (2u * (uint32_t)kk + (uint32_t)dy * row16 + (uint32_t)dx * px16);
+					const Desc bd = bd0 + (uint32_t)((dx * 3 + dy) * a.CoT);
+#pragma unroll
+					for (int r = 0; r < RT; ++r)
+						umma_f16(lead, tmem + (uint32_t)(r * a.CoT), ad + (uint32_t)r * tile16, bd, idesc, acc);
+					acc = 1u;
+				}
+				umma_commit(lead, smem_u32(done + s));
+				issued = k;
+				// refill what step k - 1 used once its MMAs are done (step k's are
+				// queued behind them meanwhile): its weights' stage and, after the
+				// last channels of slab g - 1, that slab's
+				const bool next_b = k >= 1 && k - 1 + SB < nk, next_a = kk == 0 && g >= 1 && g - 1 + SA < ns;
+				if (next_a || next_b) {
+					if (!mbar_wait_warp(smem_u32(done + (k - 1) % SB), (uint32_t)(((k - 1) / SB) & 1))) {
+						fail = 1;
+						break;
+					}
+					if (next_a) load_a(loaded_a++);
+					if (next_b) load_b(loaded++);
+				}
 			}
 		}
 		// the last commit covers every MMA issued before it
-		if (issued >= 0 && !mbar_wait_warp(smem_u32(done + issued % S), (uint32_t)((issued / S) & 1))) fail = 1;
+		if (issued >= 0 && !mbar_wait_warp(smem_u32(done + issued % SB), (uint32_t)((issued / SB) & 1))) fail = 1;
 		// copies issued but not consumed (after a failure): wait for them
 		// (bounded) before the CTA's shared memory can be reused
-		for (int c = issued + 1; c < loaded; ++c) mbar_wait_warp(smem_u32(full + c % S), (uint32_t)((c / S) & 1));
-		if (lead && (fail || issued != nch - 1)) atomicExch(a.err, 1);
+		for (int k = issued + 1; k < loaded; ++k) mbar_wait_warp(smem_u32(full + k % SB), (uint32_t)((k / SB) & 1));
+		for (int g = (issued + 1) / kps; g < loaded_a; ++g) mbar_wait_warp(smem_u32(fulla + g % SA), (uint32_t)((g / SA) & 1));
+		if (lead && (fail || issued != nk - 1)) atomicExch(a.err, 1);
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-	const int failed = __syncthreads_or(warp == 0 && (fail || issued != nch - 1));
+	const int failed = __syncthreads_or(warp == 0 && (fail || issued != nk - 1));
 	asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 	if (!failed) {
 		// epilogue: warp w owns TMEM lanes (= tile pixels) 32 w .. 32 w + 31
 		const int px = warp * 32 + lane;
 		for (int rr = 0; rr < RT; ++rr) {
+			const int q = q0 + rr * 128 + px, ry = wide ? yy + rr : q / a.P, rx = wide ? x0 + px : q - ry * a.P;
+			const bool inside = ry < a.H && rx < a.W;
+			const int64_t m = ((int64_t)n * a.H + ry) * a.W + rx;
 			for (int c0 = 0; c0 < a.CoT; c0 += 16) {
-				const int64_t m = ((int64_t)(row + rr * a.MR) * a.W) + x0 + px;
 				uint32_t r[16];
 				const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(rr * a.CoT + c0);
 				asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
@@ -688,8 +697,10 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 					o[q] = __floats2bfloat162_rn(v0, v1);
 				}
 				uint4 *dst = reinterpret_cast<uint4 *>(a.y + m * a.Co + co0 + c0);
-				dst[0] = *reinterpret_cast<const uint4 *>(&o[0]);
-				dst[1] = *reinterpret_cast<const uint4 *>(&o[4]);
+				if (inside) {
+					dst[0] = *reinterpret_cast<const uint4 *>(&o[0]);
+					dst[1] = *reinterpret_cast<const uint4 *>(&o[4]);
+				}
 			}
 		}
 	}
@@ -2009,7 +2020,7 @@ struct ConvTable {
 // A thread writes 16 bytes of two layouts: pw and w from eight input channels of
 // an output, pwf and wf from eight outputs of an input channel; threads are
 // ordered as pw and pwf lie.  (One thread per weight wrote four layouts two bytes
-// at a time, three of them a sector each: 18 us cold for 0.58 M weights, now 7.)
+// at a time, three of them a sector each: PERF10.)
 __global__ void __launch_bounds__(256) refresh_conv_weights(const float *__restrict__ p, const __grid_constant__ ConvTable t) {
 	const int l = blockIdx.y;
 	const unsigned Co = (unsigned)t.co[l], Ci = (unsigned)t.ci[l], n = Co * 9u * (Ci / 8u); // both multiples of 8
@@ -2348,31 +2359,68 @@ CUtensorMapSwizzle slab_swizzle(int cs) {
 	return cs == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : (cs == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-// Channel chunk and stage count of conv_halo: the first chunk (64, 32, 48 or
-// 16 channels dividing Ci) whose stages (up to three, at least two when there
-// are two chunks or more) fit 110 KB (two CTAs per SM), else 200 KB; 0: none.
-int halo_plan(int Ci, int Co, int RT, HaloArgs &a) {
-	for (const uint32_t cap : {110u * 1024u, 200u * 1024u})
-		for (const int ck : {64, 32, 48, 16}) {
-			if (Ci % ck) continue;
-			const int nch = Ci / ck;
-			const uint32_t cb = (uint32_t)(RT * a.MR + 2) * (uint32_t)a.P * (uint32_t)ck * 2u;
-			const uint32_t ab = (uint32_t)a.NC * cb, bb = 18u * (uint32_t)a.CoT * (uint32_t)ck;
-			const uint32_t stage = align1k(ab) + align1k(bb);
-			int S = nch < 3 ? nch : 3;
-			while (S > 1 && (uint64_t)S * stage + 1024 > cap) --S;
-			if ((nch > 1 && S < 2) || (uint64_t)S * stage + 1024 > cap) continue;
-			a.CK = ck;
-			a.CS = slab_channels(ck);
-			a.stages = S;
-			a.copy_bytes = cb;
-			a.a_bytes = ab;
-			a.b_bytes = bb;
-			a.a_span = align1k(ab);
-			a.stage_bytes = stage;
-			return 1;
-		}
+// Stages of conv_halo for slabs of a.CS channels, a.RT tiles and a.CoT outputs
+// per CTA within `cap` bytes: two slabs (one if there is one), two to four of
+// weights.  Returns the shared memory, 0 when it does not fit.
+uint32_t halo_stages(int Ci, uint32_t cap, HaloArgs &a) {
+	a.a_bytes = (uint32_t)(a.HR * a.P * a.CS) * 2u;
+	a.a_span = align1k(a.a_bytes);
+	a.b_bytes = 288u * (uint32_t)a.CoT;
+	a.SA = Ci / a.CS < 2 ? 1 : 2;
+	const int nk = Ci / 16;
+	for (a.SB = nk < 4 ? nk : 4; a.SB >= (nk < 2 ? 1 : 2); --a.SB) {
+		const uint32_t bytes = (uint32_t)a.SA * a.a_span + (uint32_t)a.SB * a.b_bytes + 1024u;
+		if (bytes <= cap) return bytes;
+	}
 	return 0;
+}
+
+// Tiles (4, 2, 1) and output channels (all, or half: at least 32) per CTA, slab
+// and stages: the form of least estimated time in cycles, waves of CTAs x (an
+// SM's copies -- 3 per pixel of a slab, 48 bytes of weights each -- or its MMAs,
+// 90 each and N / 2 beyond 180 outputs, + 4,000 for a CTA's start and epilogue).
+// The figures are fitted to launches: 192 -> 64 channels, 1,024 rows of 128, four
+// tiles per CTA, two CTAs per SM 42 us, one CTA per SM 51; 256 -> 128 channels,
+// 512 rows of 64, halves of the outputs with four tiles 50 us.  Returns 0 when
+// no form fits.
+int halo_shape(int n, int H, int W, int ci, int co, int sms, HaloArgs &a) {
+	int64_t best = -1;
+	HaloArgs pick = a;
+	for (const int rt : {4, 2, 1})
+		for (const int split : {1, 2})
+			for (const int cs : {64, 32, 16})
+				for (const uint32_t cap : {110u * 1024u, 200u * 1024u}) {
+					HaloArgs t = a;
+					t.RT = rt;
+					t.CoT = co / split;
+					t.CS = cs;
+					if (ci % cs || rt * t.CoT > 512 || (split == 2 && (co % 32 || t.CoT < 32)) || (W >= 128 && H % rt)) continue;
+					t.P = W >= 128 ? HX : W + 2;
+					// narrow: the pixels from the first tile's row on that the last one's taps reach
+					t.HR = W >= 128 ? rt + 2 : (t.P - 1 + rt * 128 + 2 * t.P + 2 + t.P - 1) / t.P;
+					t.ctas = W >= 128 ? 0 : ((H * t.P + 127) / 128 + rt - 1) / rt;
+					if (t.HR > 256) continue;
+					const uint32_t smem = halo_stages(ci, cap, t);
+					if (!smem) continue;
+					t.tmem_cols = 32;
+					while (t.tmem_cols < (uint32_t)(rt * t.CoT)) t.tmem_cols <<= 1;
+					int per_sm = (int)(227u * 1024u / (smem + 1024u));
+					if (per_sm > (int)(512u / t.tmem_cols)) per_sm = (int)(512u / t.tmem_cols);
+					if (per_sm < 1) per_sm = 1;
+					const int64_t ctas = (int64_t)n * (W >= 128 ? (int64_t)(H / rt) * (W / 128) : t.ctas) * split;
+					const int64_t each = (ctas + sms - 1) / sms, waves = (each + per_sm - 1) / per_sm;
+					const int64_t shared = each < per_sm ? each : per_sm;
+					const int64_t copy = (int64_t)t.HR * t.P * (ci / cs) * 3 + (int64_t)t.b_bytes * (ci / 16) / 48;
+					const int64_t mma = (int64_t)rt * 9 * (ci / 16) * (t.CoT > 180 ? t.CoT / 2 : 90);
+					const int64_t cost = waves * (shared * (copy > mma ? copy : mma) + 4000);
+					if (best < 0 || cost < best) {
+						best = cost;
+						pick = t;
+					}
+				}
+	if (best < 0) return 0;
+	a = pick;
+	return 1;
 }
 
 // The halo convolution (conv_halo); returns 0 without
@@ -2384,40 +2432,14 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b,
 	HaloArgs a;
 	memset(&a, 0, sizeof(a));
 	if (!enc || ci % 16 || co % 16 || co < 16 || co > 256) return KEL_OK;
-	if (W % 128 == 0) {
-		a.NC = 1;
-		a.P = HX;
-		a.MR = 1;
-	} else if (W >= 8 && W % 8 == 0 && 128 % W == 0 && H % (128 / W) == 0) {
-		a.NC = 3;
-		a.P = W;
-		a.MR = 128 / W;
-	} else {
-		return KEL_OK;
-	}
-	const int tpr = W >= 128 ? W / 128 : 1;
-	const int sms = U->sms > 0 ? U->sms : 148;
-	// M tiles per CTA: the most (4, 2, 1) whose accumulators fit TMEM and
-	// that still leave a CTA per SM; with fewer tiles than SMs, the output
-	// channels split over two CTAs (at least 32 channels each)
-	a.RT = 0;
-	a.CoT = co;
-	for (const int rt : {4, 2, 1})
-		if (!a.RT && rt * co <= 512 && H % (rt * a.MR) == 0 && (int64_t)n * (H / (rt * a.MR)) * tpr >= sms &&
-			halo_plan(ci, co, rt, a))
-			a.RT = rt;
-	if (!a.RT && H % a.MR == 0) {
-		const int64_t tiles = (int64_t)n * (H / a.MR) * tpr;
-		if (tiles < sms && co % 32 == 0 && co / 2 >= 32) a.CoT = co / 2;
-		if (halo_plan(ci, co, 1, a)) a.RT = 1;
-	}
-	if (!a.RT) return KEL_OK;
+	if (W % 128 != 0 && (W < 8 || W % 8 != 0 || 128 % W != 0 || H % (128 / W) != 0)) return KEL_OK;
+	if (!halo_shape(n, H, W, ci, co, U->sms > 0 ? U->sms : 148, a)) return KEL_OK;
 	CUtensorMap tx;
 	{ // x (N,H,W,Ci) as (CS channels, x, y, slab, n)
 		const cuuint64_t cs = (cuuint64_t)a.CS;
 		const cuuint64_t dims[5] = {cs, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)ci / cs, (cuuint64_t)n};
 		const cuuint64_t strides[4] = {(cuuint64_t)ci * 2, (cuuint64_t)W * ci * 2, cs * 2, (cuuint64_t)H * W * ci * 2};
-		const cuuint32_t box[5] = {(cuuint32_t)cs, (cuuint32_t)a.P, (cuuint32_t)(a.RT * a.MR + 2), (cuuint32_t)(a.CK / a.CS), 1};
+		const cuuint32_t box[5] = {(cuuint32_t)cs, (cuuint32_t)a.P, (cuuint32_t)a.HR, 1, 1};
 		const cuuint32_t es[5] = {1, 1, 1, 1, 1};
 		if (enc(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(x), dims, strides, box, es,
 				CU_TENSOR_MAP_INTERLEAVE_NONE, slab_swizzle(a.CS), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -2434,14 +2456,13 @@ int conv_halo_launch(kel_unet *U, const bf16 *x, const bf16 *pw, const float *b,
 	a.Co = co;
 	a.relu = relu;
 	a.use_bias = bias;
-	a.tmem_cols = 32;
-	while (a.tmem_cols < (uint32_t)(a.RT * a.CoT)) a.tmem_cols <<= 1;
 	a.err = U->d_err;
-	const size_t smem = (size_t)a.stages * a.stage_bytes + (size_t)a.stages * 16 + 16;
+	const size_t smem = (size_t)a.SA * a.a_span + (size_t)a.SB * a.b_bytes + (size_t)(a.SA + 2 * a.SB) * 8 + 16;
+	const int64_t tiles = (int64_t)n * (W >= 128 ? (int64_t)(H / a.RT) * (W / 128) : a.ctas);
 	auto launch = [&](auto cs, auto rt) -> int {
 		constexpr auto kern = conv_halo<cs.value, rt.value>;
 		KEL_CUDA(allow_dynamic_smem<kern>(210 * 1024));
-		KEL_CUDA(launch_next(overlap, kern, (unsigned)((int64_t)n * (H / (a.RT * a.MR)) * tpr * (co / a.CoT)), 128, smem, U->stream, tx, a));
+		KEL_CUDA(launch_next(overlap, kern, (unsigned)(tiles * (co / a.CoT)), 128, smem, U->stream, tx, a));
 		return KEL_OK;
 	};
 	auto with_rt = [&](auto cs) -> int {
