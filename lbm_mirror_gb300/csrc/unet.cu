@@ -15,8 +15,8 @@
 //   conv_rows        forward and data gradient of layers 128+ pixels wide
 //                    whose weights stay in shared memory: input rows stream
 //                    once each, one MMA feeds three output-row accumulators;
-//   conv_halo        the other layers: per chunk of input channels a TMA halo
-//                    tile, the nine taps as shifted descriptors;
+//   conv_halo        the other layers: per slab of input channels a TMA halo,
+//                    the nine taps as shifted descriptors;
 //   conv_wgrad_halo  weight gradients from TMA-loaded halo rows, FP32
 //                    partials per pixel chunk reduced in fixed order;
 //   conv_tc, conv_wgrad_tc  im2col forms for levels narrower than the halo
@@ -477,12 +477,11 @@ __global__ void __launch_bounds__(128) conv_tc(TcArgs a) {
 //    with rows of P = W + 2, of which a tile is 128 in a row and the next tile
 //    the 128 after them.  Outputs at the two last positions of a row and below
 //    the image are not stored (3 % of the positions at W = 64, 6 % at 32).
-// A box's row of pixels takes the TMA about 4.5 cycles per pixel, whether 32 or
-// 64 bytes of channels are taken (9,360 pixels in 41 us, 13,300 in 31 us), which
-// bound the form with three halo copies shifted by dx and a slab per 16 channels
-// (64-pixel level, 256 -> 128 channels, batch 32: 40 us, now PERF11).  So a slab
-// holds as many channels as fit, and the weights have stages of their own, of 16
-// channels.  They lie in global memory as they do in shared memory, [g][dx][dy][co]
+// The narrow form used to take three copies of the halo, shifted by dx, in slabs
+// of the 16 channels that fit beside their weights: nine times the TMA's pixels
+// (64-pixel level, 256 -> 128 channels, batch 32: 40 us, now 36; inference of 8 at
+// 256 x 64: 347 -> 301 us, training step 1319 -> 1301).  Now a slab holds up to 64
+// channels and the weights have stages of their own, of 16.  They lie in global memory as they do in shared memory, [g][dx][dy][co]
 // [8 channels] (UnetLayer::pw), and arrive as one bulk copy (a copy per group and
 // tap where the CTA has half of the channels): as TMA boxes of 16-byte rows they
 // took most of a CTA's staging time (training step 256 x 64, batch 32: 1903 ->
@@ -720,7 +719,7 @@ __global__ void __launch_bounds__(128) conv_halo(const __grid_constant__ CUtenso
 // [g][kx][ky][co][8 channels]: for a column shift dx the three kernel rows' Co x 8 blocks are
 // consecutive, so B rows (ky, co) form one operand of up to 3 Co rows (8-row
 // stride 128 B, channel-group stride 9 * Co * 16 B).  Input rows y0 - 1 ..
-// y0 + RL stream once each through a ring of NR slots, each row a TMA box of
+// y0 + RL stream once each through a ring of ROWS_NR slots, each row a TMA box of
 // 130 pixels x Ci channels, zero-filled outside the image, laid out (slab of
 // CS channels, pixel, CS channels) and swizzled as in conv_halo: the A operand
 // of input row X and shift dx is the slot read from pixel dx (K-major, 8-pixel
@@ -2020,7 +2019,7 @@ struct ConvTable {
 // A thread writes 16 bytes of two layouts: pw and w from eight input channels of
 // an output, pwf and wf from eight outputs of an input channel; threads are
 // ordered as pw and pwf lie.  (One thread per weight wrote four layouts two bytes
-// at a time, three of them a sector each: PERF10.)
+// at a time, three of them a sector each: 18 us cold for 0.58 M weights, now 7.)
 __global__ void __launch_bounds__(256) refresh_conv_weights(const float *__restrict__ p, const __grid_constant__ ConvTable t) {
 	const int l = blockIdx.y;
 	const unsigned Co = (unsigned)t.co[l], Ci = (unsigned)t.ci[l], n = Co * 9u * (Ci / 8u); // both multiples of 8
