@@ -2380,8 +2380,9 @@ uint32_t halo_stages(int Ci, uint32_t cap, HaloArgs &a) {
 // 90 each and N / 2 beyond 180 outputs, + 4,000 for a CTA's start and epilogue).
 // The figures are fitted to launches: 192 -> 64 channels, 1,024 rows of 128, four
 // tiles per CTA, two CTAs per SM 42 us, one CTA per SM 51; 256 -> 128 channels,
-// 512 rows of 64, halves of the outputs with four tiles 50 us.  Returns 0 when
-// no form fits.
+// 512 rows of 64, halves of the outputs with four tiles 50 us, all of them with
+// one tile 36 (the pick; 20 bytes of weights a cycle instead of 48 picks several
+// tiles: training step 1345 us, 1301 with this).  Returns 0 when no form fits.
 int halo_shape(int n, int H, int W, int ci, int co, int sms, HaloArgs &a) {
 	int64_t best = -1;
 	HaloArgs pick = a;

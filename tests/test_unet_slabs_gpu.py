@@ -18,3 +18,25 @@ pytestmark = pytest.mark.gpu
 ])
 def test_slabs(h, w, n, widths):
     check(h, w, n, widths, 3, 0)
+
+
+@pytest.mark.parametrize("h,w,n", [(8, 16, 96), (8, 64, 64), (8, 32, 61)])
+def test_several_tiles_per_block_on_narrow_rows(h, w, n):
+    """batches at which a block takes two or four tiles of the line of pixels: the outputs, exactly"""
+    torch = pytest.importorskip("torch")
+    from lbm_mirror_gb300 import UNet
+    from tests.test_unet_gradient_passes_gpu import _oracle, _whole_params
+    widths = (48, 16, 32, 16)
+    gen = torch.Generator().manual_seed(19)
+    net = UNet(height=h, width=w, widths=widths, out_channels=2, max_batch=n, seed=3)
+    params = _whole_params(gen, widths, 2)
+    net.set_params(params.numpy())
+    x = torch.randint(-2, 3, (n, h, w, 16), generator=gen).float()
+    y, _ = _oracle(params, x, torch.zeros((n, h, w, 2)), widths, 2)
+    xin = x.to(torch.bfloat16).cuda()
+    out = torch.empty((n, h, w, 2), device="cuda")
+    torch.cuda.synchronize()
+    net.set_input(xin.data_ptr(), n)
+    net.forward(n, out.data_ptr())
+    net.synchronize()
+    assert (out.cpu().numpy() == y).all()
