@@ -1223,7 +1223,10 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	using ST = typename S::T;
 	const int c32 = (int)cell;
 	// the shift depends on the weight alone: one constant per kind of direction
-	auto ws = [&](int i) { return p.wshift[shift_class<L>(i)]; };
+	// D3Q27 indexes by direction: the compiler does not fold the class there, and
+	// forming it in the kernel cost five times the sweep (FP16S 200x30x30, 40 steps
+	// 572 -> 3172 us)
+	auto ws = [&](int i) { return L::Q == 27 ? p.wshift[i] : p.wshift[shift_class<L>(i)]; };
 	// L2 prefetch of the rows the block (pf_x, pf_y, pf_z) later will read (its x range in every direction plane; in odd steps its
 	// neighbours' rows are prefetched by their own predecessors): requests in
 	// flight that hold no registers, one 128-byte line per thread.
