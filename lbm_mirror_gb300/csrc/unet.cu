@@ -2270,12 +2270,16 @@ struct kel_unet {
 	int sms = 0;                       // the device's SM count (grid sizing)
 	// kel_unet_train_step: the target copy, Adam's lr and bias corrections on
 	// the device, the last loss, and the captured step (forward, backward,
-	// Adam, weight refresh) for batch train_n and these Adam constants
+	// Adam, weight refresh) for batch train_n, these Adam constants and the
+	// settings that the captured launches hold: the residual head and the
+	// convolution kernels
 	float *tgt = nullptr, *adam_c = nullptr;
 	double *dev_loss = nullptr;
 	cudaGraphExec_t train_graph = nullptr;
 	int train_n = 0;
 	float train_b1 = 0.f, train_b2 = 0.f, train_eps = 0.f;
+	HeadRes train_res;
+	int train_conv_kernel = 0;
 	bool train_warm = false;
 };
 
@@ -3309,7 +3313,8 @@ extern "C" int kel_unet_train_step(kel_unet *U, const float *d_target, int32_t n
 	adam_consts<<<1, 1, 0, U->stream>>>(U->adam_c, lr, c1, c2);
 	KEL_CUDA(cudaGetLastError());
 	const bool same = U->train_graph && U->train_n == n && U->train_b1 == beta1 && U->train_b2 == beta2 &&
-					  U->train_eps == eps;
+					  U->train_eps == eps && U->train_conv_kernel == U->conv_kernel &&
+					  memcmp(&U->train_res, &U->res, sizeof(HeadRes)) == 0;
 	if (!same) {
 		if (U->train_graph) cudaGraphExecDestroy(U->train_graph);
 		U->train_graph = nullptr;
@@ -3340,6 +3345,8 @@ extern "C" int kel_unet_train_step(kel_unet *U, const float *d_target, int32_t n
 				U->train_b1 = beta1;
 				U->train_b2 = beta2;
 				U->train_eps = eps;
+				U->train_conv_kernel = U->conv_kernel;
+				U->train_res = U->res;
 			}
 		}
 	}
