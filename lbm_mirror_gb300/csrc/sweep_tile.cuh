@@ -267,8 +267,8 @@ __device__ __forceinline__ void tile_steps(const TileGeom &g, const Shift &shift
 		const unsigned lanes = __ballot_sync(FULL, mine);
 #pragma unroll 1
 		for (int ry = m + r0; ry < g.rows - m; ry += RS) {
-			// a rim lane reads its neighbours' slots too (inside the array: rows
-			// 0 and g.rows - 1 are not visited), so its values are finite
+			// a rim lane's slots are other cells', which may be storing to them: it
+			// reads nothing and follows the others at rest
 			T *const s = sm + ry * PITCH + rx;
 			float f[R][9];
 			unsigned rim[R];
@@ -277,8 +277,9 @@ __device__ __forceinline__ void tile_steps(const TileGeom &g, const Shift &shift
 				rim[k] = bnd[(ry + k) * WPR + wx] & lanes;
 #pragma unroll
 				for (int i = 0; i < 9; ++i)
-					f[k][i] = S::ld(s + (k * PITCH + ((m & 1) ? -L::cy(i) * PITCH + L::opp(i) * W - L::cx(i) : i * W)),
-									shift(i));
+					f[k][i] = mine ? S::ld(s + (k * PITCH + ((m & 1) ? -L::cy(i) * PITCH + L::opp(i) * W - L::cx(i) : i * W)),
+										   shift(i))
+								   : (float)L::w(i);
 			}
 			step(m, f, ry, mine, rim);
 		}
