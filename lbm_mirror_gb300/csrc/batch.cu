@@ -20,6 +20,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "lattice_internal.cuh"
@@ -592,7 +593,10 @@ struct kel_batch {
 	double2 *partial = nullptr;
 	double *d_residual = nullptr;
 	uint32_t plain = 0; // SweepParams::plain of the program
-	float *staging = nullptr;    // downloads
+	// downloads: kept, and used by one call at a time (threads may read
+	// different channels at once)
+	std::mutex staging_use;
+	float *staging = nullptr;
 	int64_t staging_len = 0;
 	OpEntry *ops = nullptr;
 	bool have_ops = false;
@@ -1047,6 +1051,7 @@ static int batch_download(kel_batch *B, int32_t channel, int what, float *host) 
 		return fail(KEL_ERR_INVALID_ARGUMENT, "kel_batch_download: bad arguments");
 	const ChannelRec ch = B->rec[channel];
 	const int64_t n = (int64_t)ch.nx * ch.ny * (what == 0 ? 9 : 3);
+	const std::lock_guard<std::mutex> use(B->staging_use);
 	// the staging buffer is kept (it grows to the largest channel read): an
 	// allocation and a free per call cost up to 100 us, by what else holds the
 	// driver's chunks
