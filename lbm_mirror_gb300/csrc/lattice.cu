@@ -1094,10 +1094,12 @@ static int ensure_step_graph(kel_lattice *L, const SweepParams &p, int coll, boo
 		return KEL_ERR_CUDA;
 	}
 	cudaError_t e = cudaSuccess;
+	SweepParams pg = p;
+	if (pg.overlap) pg.overlap = OVERLAP_GRAPH;
 	if (tiled)
-		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; k += 2 * TILE_K) e = launch_tile_pair(L, p, coll);
+		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; k += 2 * TILE_K) e = launch_tile_pair(L, pg, coll);
 	else
-		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) e = launch_one(L, p, coll, exact, (k & 1) != 0);
+		for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) e = launch_one(L, pg, coll, exact, (k & 1) != 0);
 	cudaError_t e2 = cudaStreamEndCapture(L->stream, &g);
 	if (e == cudaSuccess && e2 == cudaSuccess && g) e = cudaGraphInstantiate(&L->graph, g, 0);
 	else if (e == cudaSuccess) e = e2;
@@ -1157,7 +1159,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 	// a caller's graph may be replayed after an upload of the force field
 	if (capturing && !L->own_capture) p.force = L->force;
 	// consecutive sweeps of this call overlap the next one's launch
-	p.overlap = L->cpt == 1 && L->stream != nullptr && !capturing ? 1 : 0;
+	p.overlap = L->cpt == 1 && L->stream != nullptr && !capturing ? OVERLAP_STREAM : OVERLAP_NONE;
 	const bool exact = P->arithmetic == KEL_ARITH_REFERENCE;
 	uint64_t s = 0;
 	// Long runs without macro output replay a captured graph of GRAPH_STEPS

@@ -63,6 +63,8 @@ struct OpEntry {
 	float eq[27];  // equilibrium(rho, u) for the Equilibrium boundary
 };
 
+enum { OVERLAP_NONE = 0, OVERLAP_STREAM = 1, OVERLAP_GRAPH = 2 };
+
 struct SweepParams {
 	void *f;          // populations (float or __half), plane-major
 	int64_t plane;    // cells per direction plane (nz*ny*nxp)
@@ -101,7 +103,9 @@ struct SweepParams {
 	// bit f: flag value f (1 .. MAX_FLAGS-1) has no boundary step and collides,
 	// so its cells skip the operation-table dispatch (same result)
 	uint32_t plain;
-	int overlap;     // launch with programmatic stream serialization (see grid_dependency_wait)
+	// launch with programmatic stream serialization (see grid_dependency_wait): OVERLAP_STREAM
+	// for launches one by one, OVERLAP_GRAPH inside a captured graph of the library's
+	int overlap;
 	uint32_t bounce; // bit f: flag value f bounces back and does not collide
 	// sweep1_kernel: how far ahead a block prefetches rows into L2, in grid
 	// coordinates (the launch fills them in: no division in the kernel), and
@@ -1201,7 +1205,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	using S = Store<STORE>;
 	constexpr int Q = L::Q;
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
-	grid_dependents_launch();
+	if (p.overlap) grid_dependents_launch(); // see sweep1_overlaps
 	if (x >= p.nxp) return;
 	const int y = blockIdx.y, z = blockIdx.z;
 	const int nxp = p.nxp;
@@ -1256,7 +1260,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	}
 
 	const int flag = p.flags[cell];
-	grid_dependency_wait();
+	if (p.overlap) grid_dependency_wait();
 
 	float f[Q];
 	// IDX32, odd steps: the cell's index for accesses to x - 1 and x + 1
