@@ -1193,6 +1193,9 @@ __global__ void __launch_bounds__(256, 4) sweep2h_kernel(const __grid_constant__
 // flight than 24 at 80 registers (measured +3 % FP32, +6 % FP16S at 256^3;
 // the few spilled words stay in L1).
 // IDX32: every population's index fits 32 bits (Q * plane < 2^31).
+// OVERLAP: with the instructions of overlapped launches (see sweep1_overlaps; as a
+// launch parameter in place of a template's, a branch cost the sweeps with a force 4 %,
+// a predicate D3Q19 64^3 2.4 %).
 // Index tables in the parameter bank, 32-bit indexes, prefetch coordinates by
 // carries and the force terms shared between directions took the instructions
 // per cell from 567 / 621 (even / odd step) to 412 / 506 for D3Q19 FP32, 611 /
@@ -1200,12 +1203,13 @@ __global__ void __launch_bounds__(256, 4) sweep2h_kernel(const __grid_constant__
 // force, 274 / 297 to 203 / 256 for D2Q9.  Measured, with the overlapped
 // launches: FP16S 256^3 353 -> 286 us per step, D3Q27 173x131x97 with a force
 // 134 -> 102, D3Q19 64^3 12.4 -> 8.7, D2Q9 1021x347 8.4 -> 4.6.
-template <class L, int STORE, bool ODD, int COLL, bool EXACT, bool HW = false, bool IDX32 = true>
+template <class L, int STORE, bool ODD, int COLL, bool EXACT, bool HW = false, bool IDX32 = true,
+		  bool OVERLAP = true>
 __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ SweepParams p) {
 	using S = Store<STORE>;
 	constexpr int Q = L::Q;
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
-	if (p.overlap) grid_dependents_launch(); // see sweep1_overlaps
+	if (OVERLAP) grid_dependents_launch();
 	if (x >= p.nxp) return;
 	const int y = blockIdx.y, z = blockIdx.z;
 	const int nxp = p.nxp;
@@ -1260,7 +1264,7 @@ __global__ void __launch_bounds__(256, 4) sweep1_kernel(const __grid_constant__ 
 	}
 
 	const int flag = p.flags[cell];
-	if (p.overlap) grid_dependency_wait();
+	if (OVERLAP) grid_dependency_wait();
 
 	float f[Q];
 	// IDX32, odd steps: the cell's index for accesses to x - 1 and x + 1

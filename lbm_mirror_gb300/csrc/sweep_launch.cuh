@@ -60,18 +60,18 @@ static cudaError_t launch_rows(const SweepParams &p, cudaStream_t st) {
 // per launch, but not for free:
 //  - a block's griddepcontrol instructions go through a unit that serves about 1,000
 //    blocks per us, so many blocks of little work each are bound by it (D2Q9 FP32, 32 x
-//    65,000: 66 us overlapped, 41 without the instructions; 64 x 39,062 41 and 37;
+//    65,000: 66 us overlapped, 41 without the instructions; 64 x 39,062 41 and 34;
 //    128 x 19,531 25.6 and 29.0; D3Q19 32 x 280 x 280 82 and 73, D3Q27 32 x 177 x 177, of
-//    27 populations a cell, 37 and 41);
+//    27 populations a cell, 40 and 46);
 //  - inside a graph, where a launch costs little, a 3D grid of whole blocks that fills
-//    more than half of the SMs' slots but not all lets the next grid's first blocks
-//    take the free ones unevenly (D3Q19 FP32 512 x 14 x 14, 784 blocks on 152 SMs of 8:
-//    5.3 us per step overlapped, 5.0 without; 176 x 24 x 24 in ragged blocks 4.9 and 5.4).
+//    half to three quarters of the SMs' slots lets the next grid's first blocks take
+//    the free ones unevenly (D3Q19 FP32 512 x 14 x 14, 784 blocks on 152 SMs of 8: 5.3 us
+//    per step overlapped, 5.0 without; fuller grids gain: 128 x 33 x 33 4.9 and 5.6).
 static bool sweep1_overlaps(const SweepParams &p, int Q, int D, int block) {
 	const int64_t rows = (int64_t)p.ny * p.nz, blocks = (p.nxp + block - 1) / block * rows;
-	if (blocks > 16384 && p.nxp * rows * Q < 800 * blocks) return false;
+	if (blocks > 16384 && p.nxp * rows * Q < 650 * blocks) return false;
 	const int slots = p.sms * (1024 / block); // 64 registers per thread
-	return !(p.overlap == OVERLAP_GRAPH && D == 3 && p.nxp % block == 0 && blocks > slots / 2 && blocks <= slots);
+	return !(p.overlap == OVERLAP_GRAPH && D == 3 && p.nxp % block == 0 && blocks > slots / 2 && blocks <= slots * 3 / 4);
 }
 
 // One cell per thread: the grid, and the prefetch distance -- the block one
@@ -82,15 +82,18 @@ static bool sweep1_overlaps(const SweepParams &p, int Q, int D, int block) {
 template <class L, int STORE, bool ODD, int COLL, bool EXACT, bool HW = false>
 static cudaError_t launch_sweep1(SweepParams p, int block, cudaStream_t st) {
 	const dim3 grid((p.nxp + block - 1) / block, p.ny, p.nz);
-	if (!sweep1_overlaps(p, L::Q, L::D, block)) p.overlap = OVERLAP_NONE;
+	const bool overlap = p.overlap && sweep1_overlaps(p, L::Q, L::D, block);
 	const int ahead = p.sms * (1024 / block);
 	p.pf_x = ahead % (int)grid.x;
 	p.pf_y = ahead / (int)grid.x % (int)grid.y;
 	p.pf_z = ahead / (int)grid.x / (int)grid.y;
 	const int lines = block * (int)sizeof(typename Store<STORE>::T) / 128;
 	p.pf_shift = lines >= 8 ? 3 : (lines >= 4 ? 2 : (lines >= 2 ? 1 : 0));
-	return p.idx32 ? launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, true>, grid, block, 0, st, p.overlap != 0, p)
-				   : launch_overlapped(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, false>, grid, block, 0, st, p.overlap != 0, p);
+	auto go = [&](auto kern) { return launch_overlapped(kern, grid, block, 0, st, overlap, p); };
+	if (!p.idx32) return go(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, false>);
+	if constexpr (!HW)
+		if (!overlap) return go(sweep1_kernel<L, STORE, ODD, COLL, EXACT, false, true, false>);
+	return go(sweep1_kernel<L, STORE, ODD, COLL, EXACT, HW, true>);
 }
 
 template <class L, int STORE, bool ODD, int COLL, bool EXACT>
