@@ -928,12 +928,26 @@ static SweepParams make_params(kel_lattice *L, const kel_step_program *P) {
 			p.off_even[i] = (int)(i * L->plane);
 			p.off_odd[i] = (int)(i * L->plane + L->d.c[i][0] + (L->d.c[i][1] + L->d.c[i][2] * L->desc.ny) * L->nxp);
 		}
-	// Rows are covered by whole blocks: with no launch shape asked for, 64
-	// threads where 128 would leave an eighth of a row's threads idle (64-cell
-	// rows half filled their blocks: D3Q19 64^3 13.0 -> 12.0 us per step; on
-	// long rows 64 threads are the slower block: FP16S 3000x2000 96 us, 60 with 128)
-	const int row64 = (L->nxp + 63) / 64 * 64, row128 = (L->nxp + 127) / 128 * 128;
-	p.block = !L->tuned && L->cpt == 1 && row128 - row64 >= row128 / 8 ? 64 : L->block;
+	// With no launch shape asked for: blocks of 128 threads; blocks of 64
+	//  - for rows of 33 to 64 cells where many (13 per SM) keep the SMs full: D3Q19 FP32
+	//    48 x 144 x 144 27.2 us per step with 64 threads and 29.5 with 128, D2Q9 64 x 39,062
+	//    33.8 and 36.8; with fewer 48 x 25 x 25 5.3 and 4.4, 64 x 40 x 40 5.8 and 5.5;
+	// and in 3D
+	//  - for the longest of those where few (4 per SM) run at once (64 x 22 x 22 3.7
+	//    and 4.0);
+	//  - for longer rows that leave half of a last block of 128 idle (176 x 28 x 28 with a
+	//    force 5.9 and 7.6), or most of it where all blocks run at once (260 x 11 x 11 4.3
+	//    and 5.4; otherwise 136 x 136 x 136 with a force 93.9 and 80.2).
+	// Rows of up to 32 cells want 128 (their idle warps are gone at once, and blocks of 64
+	// come at the same rate: 32 x 177 x 177 42.0 and 32.3), and so do D2Q9's longer ones
+	// (2.5 million cells, FP32: rows of 136 41.8 and 34.4, of 320 27.3 and 26.1).
+	const int last = (L->nxp - 1) % 128 + 1; // cells of a row's last 128
+	const int64_t rows = L->desc.ny * L->desc.nz, few = 4 * L->sms;
+	bool half = L->nxp > 32 && L->nxp <= 64 && rows > 13 * L->sms;
+	if (L->d.D == 3)
+		half = half || (L->nxp > 56 && L->nxp <= 64 && rows <= few) ||
+			   (L->nxp > 64 && last <= 64 && (last > 32 || (L->nxp + 63) / 64 * rows <= few));
+	p.block = !L->tuned && L->cpt == 1 && half ? 64 : L->block;
 	p.hw_mask = L->hw_active ? L->hw_mask : nullptr;
 	p.plain = L->plain_flags;
 	p.bounce = L->bounce_flags;
