@@ -477,6 +477,11 @@ int kel_unet_set_residual(kel_unet *net, int32_t out_channel, int32_t in_channel
 #define KEL_LAUNCH_ROWS (-1)
 int kel_lattice_set_launch(kel_lattice *lat, int32_t cells_per_thread, int32_t block_threads);
 int kel_lattice_get_launch(const kel_lattice *lat, int32_t *cells_per_thread, int32_t *block_threads);
+/* Tiles of the lattice's runs of the program last passed to kel_step: D2Q9 steps
+ * without macro output may go `steps` at a time, in one launch on tiles of
+ * `columns` x `rows` cells held in shared memory (the same results).  1, 0, 0:
+ * step by step in the launch shape, as always after kel_lattice_set_launch. */
+int kel_lattice_get_tiles(const kel_lattice *lat, int32_t *steps, int32_t *columns, int32_t *rows);
 /* Time `steps` sweeps of `prog` with every launch shape on the lattice's
  * current state and keep the fastest.  The populations are restored after
  * each trial and the time step does not advance. */

@@ -306,6 +306,7 @@ def load_library(path: str | None = None):
         "kel_lattice_init_equilibrium": ([vp, vp, vp, C.c_double, C.POINTER(C.c_double)], C.c_int),
         "kel_particles_stamp": ([vp, C.POINTER(ParticleParams)], C.c_int),
         "kel_lattice_get_launch": ([vp, C.POINTER(i32), C.POINTER(i32)], C.c_int),
+        "kel_lattice_get_tiles": ([vp, C.POINTER(i32), C.POINTER(i32), C.POINTER(i32)], C.c_int),
         "kel_lattice_autotune": ([vp, C.POINTER(StepProgram), i32, C.POINTER(i32), C.POINTER(i32),
                                   C.POINTER(C.c_float)], C.c_int),
         "kel_particles_create": ([vp, i32, C.POINTER(vp)], C.c_int),

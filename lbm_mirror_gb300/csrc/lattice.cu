@@ -859,6 +859,72 @@ static bool launch_ok(const kel_lattice *L, int cpt, int block) {
 	return true;
 }
 
+// How program P's runs on lattice L are cut into tiles (two blocks of either shape
+// run on each SM), or not at all: where both sides were measured, tiles are the
+// faster form (figures in sweep_tile.cuh)
+//  - on small lattices, up to 100,000 cells, or fewer if a present flag has a boundary
+//    step other than bounce-back (`open`: its cells leave the tile's straight code).
+//    There the cells the tiles cover count: 70,000, or 52,000 with a force in FP32 and
+//    with a force and PSM;
+//  - in FP32 beyond the L2, by a share of it that grows with what a collision costs in
+//    the ring, and for rows that the tiles' columns do not exceed by much.
+// Small tiles take the fewest rows that give every SM one block (a block's
+// steps follow one another, so a launch takes as long as its rows: 256x64 6
+// rows 1.7 us per step, 16 rows 2.5), else two.
+static TilePlan plan_tiles(const kel_lattice *L, const kel_step_program *P) {
+	TilePlan t;
+	const int64_t ny = L->desc.ny, nxp = L->nxp;
+	if (L->d.Q != 9 || P->arithmetic == KEL_ARITH_REFERENCE || P->collision > KEL_COLL_PSM_GUO || L->shape_asked ||
+		L->hw_active || L->d.Q * L->plane >= ((int64_t)1 << 31))
+		return t;
+	bool open = false;
+	for (int fl = 1; fl < MAX_FLAGS; ++fl) open = open || (L->present[fl] && !((L->plain_flags | L->bounce_flags) >> fl & 1u));
+	auto blocks = [&](int64_t tx, int64_t ty) { return (nxp + tx - 1) / tx * ((ny + ty - 1) / ty); };
+	const bool dear = P->collision == KEL_COLL_PSM_GUO ||
+					  (P->collision == KEL_COLL_BGK_GUO && L->desc.storage == KEL_STORAGE_FP32);
+
+	const int64_t wide = TileWide::W - 2 * TILE_K, covered = (nxp + wide - 1) / wide * wide;
+	int eighths = 0, percent = open ? 110 : 145; // of the L2, at least; columns to row, at most
+	switch (P->collision) {
+	case KEL_COLL_BGK: eighths = 7; break;
+	case KEL_COLL_PSM:
+		eighths = open ? 9 : 7;
+		if (open) percent = 105;
+		break;
+	case KEL_COLL_BGK_GUO:
+		eighths = 14;
+		percent = 105;
+		break;
+	}
+	int l2 = 0;
+	if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, L->device) != cudaSuccess) {
+		cudaGetLastError();
+		return t;
+	}
+	const int64_t bytes = L->d.Q * L->plane * (int64_t)L->elem;
+	if (bytes > l2 - l2 / 8) {
+		if (L->desc.storage != KEL_STORAGE_FP32 || !eighths || bytes <= l2 / 8 * (int64_t)eighths || covered * 100 > nxp * percent)
+			return t;
+		t.wide = true; // fewest rows of work per SM, tile row sums 4 ty + 20
+		int64_t best = -1;
+		for (int ty = 24; ty <= 32; ty += 4) {
+			const int64_t w = (blocks(wide, ty) + 2 * L->sms - 1) / (2 * L->sms) * (4 * ty + 20);
+			if (best < 0 || w < best) {
+				best = w;
+				t.ty = ty;
+			}
+		}
+		return t;
+	}
+	const int64_t tx = TileSmall::W - 2 * TILE_K;
+	if (open ? (nxp + tx - 1) / tx * tx * ny > (dear ? 52000 : 70000) : nxp * ny > 100000) return t;
+	for (t.ty = 4; t.ty <= 8; t.ty += 2)
+		if (blocks(tx, t.ty) <= L->sms) return t;
+	for (t.ty = 4; t.ty < 24; t.ty += 2)
+		if (blocks(tx, t.ty) <= 2 * L->sms) return t;
+	return t;
+}
+
 extern "C" int kel_lattice_set_launch(kel_lattice *L, int32_t cells_per_thread, int32_t block_threads) {
 	if (!L) return fail(KEL_ERR_INVALID_ARGUMENT, "kel_lattice_set_launch: null lattice");
 	if (!launch_ok(L, cells_per_thread, block_threads))
@@ -868,6 +934,16 @@ extern "C" int kel_lattice_set_launch(kel_lattice *L, int32_t cells_per_thread, 
 	L->block = block_threads;
 	L->tuned = true;
 	L->shape_asked = true;
+	L->tile = TilePlan();
+	return KEL_OK;
+}
+
+extern "C" int kel_lattice_get_tiles(const kel_lattice *L, int32_t *steps, int32_t *columns, int32_t *rows) {
+	if (!L || !steps || !columns || !rows) return fail(KEL_ERR_INVALID_ARGUMENT, "kel_lattice_get_tiles: null");
+	const bool tiles = L->tile.ty > 0 && !L->no_f2;
+	*steps = tiles ? TILE_K : 1;
+	*columns = tiles ? (L->tile.wide ? TileWide::W : TileSmall::W) - 2 * TILE_K : 0;
+	*rows = tiles ? L->tile.ty : 0;
 	return KEL_OK;
 }
 
@@ -1020,42 +1096,11 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 	L->block = bb;
 	L->tuned = true;
 	L->shape_asked = false;
+	L->tile = plan_tiles(L, P);
 	if (cells_per_thread) *cells_per_thread = bc;
 	if (block_threads) *block_threads = bb;
 	if (ms_per_step) *ms_per_step = best;
 	return KEL_OK;
-}
-
-// Tiles of a lattice of nxp x ny cells on `sms` multiprocessors (two blocks of
-// either shape run on each), or none: small tiles up to 100,000 cells, wide
-// ones where the populations (pop_bytes) exceed the L2; the lines are where
-// the tiles stop and start to be the faster form (figures in sweep_tile.cuh).
-// Small tiles take the fewest rows that give every SM one block (a block's
-// steps follow one another, so a launch takes as long as its rows: 256x64 6
-// rows 1.55 us per step, 16 rows 2.5), else two.
-static TilePlan plan_tiles(int nxp, int ny, int64_t pop_bytes, int64_t l2_bytes, int sms) {
-	TilePlan t;
-	auto blocks = [&](int tx, int ty) { return (int64_t)((nxp + tx - 1) / tx) * ((ny + ty - 1) / ty); };
-	if (pop_bytes > l2_bytes - l2_bytes / 8) { // fewest rows of work per SM, tile row sums 4 ty + 20
-		t.wide = true;
-		const int tx = TileWide::W - 2 * TILE_K;
-		int64_t best = -1;
-		for (int ty = 24; ty <= 32; ty += 4) {
-			const int64_t w = (blocks(tx, ty) + 2 * sms - 1) / (2 * sms) * (4 * ty + 20);
-			if (best < 0 || w < best) {
-				best = w;
-				t.ty = ty;
-			}
-		}
-		return t;
-	}
-	if ((int64_t)nxp * ny > 100000) return t;
-	const int tx = TileSmall::W - 2 * TILE_K;
-	for (t.ty = 4; t.ty <= 8; t.ty += 2)
-		if (blocks(tx, t.ty) <= sms) return t;
-	for (t.ty = 4; t.ty < 24; t.ty += 2)
-		if (blocks(tx, t.ty) <= 2 * sms) return t;
-	return t;
 }
 
 // The second population array, on first use.  A lattice that would not leave
@@ -1166,6 +1211,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 		KEL_CUDA(cudaStreamSynchronize(L->stream));
 		L->last_prog = *P;
 		L->have_ops = true;
+		L->tile = plan_tiles(L, P);
 	}
 	if ((rc = ensure_collision_fields(L, P->collision))) return rc;
 
@@ -1184,15 +1230,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 							   : ((step_flags & KEL_STEP_WRITE_MACROS) && n_steps > 0 ? n_steps - 1 : n_steps);
 	// D2Q9 runs without macro output may do TILE_K steps per launch on tiles, in
 	// pairs of launches from an even step (the remaining steps follow one by one).
-	bool tiled = L->d.Q == 9 && !exact && !capturing && !L->shape_asked && !L->hw_active && p.idx32 &&
-				 P->collision <= KEL_COLL_PSM_GUO && plain >= (L->t & 1u) + 2 * TILE_K;
-	if (tiled && !L->tile.planned) {
-		int l2 = 0;
-		KEL_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, L->device));
-		L->tile = plan_tiles(L->nxp, (int)L->desc.ny, (int64_t)L->d.Q * L->plane * (int64_t)L->elem, l2, L->sms);
-		L->tile.planned = true;
-	}
-	tiled = tiled && L->tile.ty > 0 && ensure_f2(L);
+	const bool tiled = L->tile.ty > 0 && !capturing && plain >= (L->t & 1u) + 2 * TILE_K && ensure_f2(L);
 	constexpr uint64_t pair = 2 * TILE_K;
 	const bool graphed = L->stream != nullptr && !capturing && L->cpt != CPT_ROWS && plain >= 2 * GRAPH_STEPS;
 	if (tiled || graphed) {

@@ -33,7 +33,6 @@ struct HostDesc {
 
 // How a D2Q9 lattice is cut into tiles of TILE_K steps per launch (sweep_tile.cuh).
 struct TilePlan {
-	bool planned = false;
 	bool wide = false;
 	int ty = 0; // tile rows; 0: no tiles
 };
@@ -94,5 +93,5 @@ struct kel_lattice {
 	bool shape_asked = false; // kel_lattice_set_launch named a shape: every step runs it
 	void *f2 = nullptr;       // second population array of the multi-step tiles (TilePlan)
 	bool no_f2 = false;       // it could not be had
-	kel::gb::TilePlan tile;
+	kel::gb::TilePlan tile;   // of the current program (last_prog)
 };

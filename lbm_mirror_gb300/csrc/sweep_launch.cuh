@@ -166,17 +166,18 @@ static cudaError_t launch_tile_variant(const TileParams &q, cudaStream_t st) {
 template <int PART>
 cudaError_t launch_tile_part(const TileParams &q, int coll, bool wide, cudaStream_t st) {
 	constexpr int STORE = PART == PART_FP16S ? STORE_FP16S : STORE_FP32;
-#define KEL_TILE(C)                                                                                                    \
-	case C:                                                                                                            \
-		return wide ? launch_tile_variant<STORE, C, TileWide>(q, st)                                                   \
-					: launch_tile_variant<STORE, C, TileSmall>(q, st)
+	auto go = [&](auto c) -> cudaError_t { // wide tiles: FP32, and not with PSM and a force (plan_tiles)
+		constexpr int C = decltype(c)::value;
+		if constexpr (STORE == STORE_FP32 && C != COLL_PSM_GUO)
+			if (wide) return launch_tile_variant<STORE, C, TileWide>(q, st);
+		return wide ? cudaErrorInvalidValue : launch_tile_variant<STORE, C, TileSmall>(q, st);
+	};
 	switch (coll) {
-		KEL_TILE(COLL_BGK);
-		KEL_TILE(COLL_BGK_GUO);
-		KEL_TILE(COLL_PSM);
-		KEL_TILE(COLL_PSM_GUO);
+	case COLL_BGK: return go(std::integral_constant<int, COLL_BGK>());
+	case COLL_BGK_GUO: return go(std::integral_constant<int, COLL_BGK_GUO>());
+	case COLL_PSM: return go(std::integral_constant<int, COLL_PSM>());
+	case COLL_PSM_GUO: return go(std::integral_constant<int, COLL_PSM_GUO>());
 	}
-#undef KEL_TILE
 	return cudaErrorInvalidValue;
 }
 

@@ -11,13 +11,21 @@
 // beyond the L2 by HBM.  Here a cell is read and written once per K steps and
 // the steps between find their populations at constant offsets from one
 // shared-memory address; the price is the ring, computed redundantly (1.3 to
-// 1.6 times the tile's cells, by tile height).  In between, on lattices that
-// the L2 holds, the one-step sweep is the faster one (D2Q9 FP32, tiles / one
-// step, us per step: 256x64 1.7 / 2.2, 512x128 2.2 / 2.4, 512x256 3.3 / 3.1,
-// 1021x347 5.4 / 4.7, 1024^2 12.6 / 10.6, 2048x1024 19.8 / 19.6, 2048^2 34.6 /
-// 42.7, 4096^2 118 / 186), and so it is in the reference's arithmetic at every
-// size from 256x64 up (3.2 / 3.1 there, 4096^2 438 / 300: the ring repeats an
-// expensive collision).
+// 1.6 times the tile's cells, by tile height) and, for boundary steps other than
+// bounce-back, a call per cell.  Tiles and the one-step sweep, us per step of 20 in
+// FP32 (x periodic between walls; a channel with Zou-He ends in brackets):
+//   BGK   256x64 1.3 / 2.1 (1.9 / 2.3), 512x128 1.6 / 2.7 (2.4 / 2.9), 400x240 1.9 / 3.0
+//         (333x290 2.9 / 3.0), 1900x1752 27 / 32 (30 / 33), 2048^2 33 / 42 (37 / 43),
+//         4096^2 129 / 188 (135 / 189); between the last small and the first large one
+//         the L2 holds the lattice and the one-step sweep is the faster one;
+//   a force costs the tiles more: 0.72 of the one-step sweep's time at 256x64 (0.95), 0.84
+//         at 400x240 (1.14 at 333x290), 1.04 at 1900x1752, 0.90 at 2640x2600 (0.95);
+//   PSM   0.66 at 256x64 (0.95), 0.92 at 1900x1752 (1.01), 0.84 at 4096^2 (0.86); with a
+//         force 0.76 (1.03) at 256x64, 1.02 to 1.07 beyond the L2;
+//   columns that a row fills badly: 200x24000 0.72 (1.04), 120x50000 0.83 (1.26);
+//   FP16S beyond its L2 size (2640x2600 and more) 1.04 to 1.38: none there.
+// In the reference's arithmetic the one-step sweep is faster at every size from
+// 256x64 up (3.2 / 3.1 there, 4096^2 438 / 300: the ring repeats an expensive collision).
 //
 // Inside the tile the populations are in the AA layout of sweep.cuh (one copy
 // in shared memory, each slot read and written by the same cell within a
@@ -43,8 +51,8 @@ constexpr int TILE_K = 4;
 // Wide, for lattices beyond the L2: the least redundant work, two cells per
 // instruction (120 instructions per cell and step; 4096^2 118 us per step,
 // Small 129).  Small, for small lattices: one cell per thread, more blocks
-// (256x64 1.5 us per step, Wide 2.3).  Eight steps per launch lose more to the
-// ring than they save in launches (256x64 1.8).
+// (256x64 in an earlier form 1.5 us per step, Wide 2.3).  Eight steps per launch lose
+// more to the ring than they save in launches (1.8 there).
 using TileWide = TileShape<64, TILE_K, 2, 384, 2>;
 using TileSmall = TileShape<32, TILE_K, 1, 512, 2>;
 

@@ -309,6 +309,13 @@ class Lattice:
         _check(self.lib.kel_lattice_get_launch(self._h, C.byref(a), C.byref(b)), self.lib)
         return a.value, b.value
 
+    def tiles(self):
+        """(steps, columns, rows) of the multi-step tiles of the program last passed to
+        step(); (1, 0, 0): step by step."""
+        a, b, c = C.c_int32(), C.c_int32(), C.c_int32()
+        _check(self.lib.kel_lattice_get_tiles(self._h, C.byref(a), C.byref(b), C.byref(c)), self.lib)
+        return a.value, b.value, c.value
+
     def synchronize(self):
         _check(self.lib.kel_lattice_synchronize(self._h), self.lib)
 
