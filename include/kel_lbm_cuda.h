@@ -168,7 +168,11 @@ int kel_upload_inlet_profile(kel_lattice *lat, const double *host_ux, int64_t n)
  * capture (a new program during capture is rejected).  The lattice's time
  * step advances when kel_step is called, not when a graph is replayed, so a
  * captured sequence should hold an even number of steps (the AA layout
- * depends on the parity of the time step). */
+ * depends on the parity of the time step).
+ * A call with a program that is new to the lattice (n_steps may be 0) allocates
+ * what its steps need: the fields its collision reads, and for D2Q9 lattices whose
+ * runs go several steps at a time (kel_lattice_get_tiles) a second population
+ * array, if that leaves three quarters of the free memory. */
 int kel_step(kel_lattice *lat, const kel_step_program *prog, uint64_t n_steps, uint32_t step_flags);
 
 /* ---- particles: spheres (3D) / discs (2D) coupled by PSM -------------- */
@@ -480,7 +484,8 @@ int kel_lattice_get_launch(const kel_lattice *lat, int32_t *cells_per_thread, in
 /* Tiles of the lattice's runs of the program last passed to kel_step: D2Q9 steps
  * without macro output may go `steps` at a time, in one launch on tiles of
  * `columns` x `rows` cells held in shared memory (the same results).  1, 0, 0:
- * step by step in the launch shape, as always after kel_lattice_set_launch. */
+ * step by step in the launch shape, as always after kel_lattice_set_launch, which
+ * gives the second population array of the tiles back. */
 int kel_lattice_get_tiles(const kel_lattice *lat, int32_t *steps, int32_t *columns, int32_t *rows);
 /* Time `steps` sweeps of `prog` with every launch shape on the lattice's
  * current state and keep the fastest.  The populations are restored after

@@ -925,6 +925,45 @@ static TilePlan plan_tiles(const kel_lattice *L, const kel_step_program *P) {
 	return t;
 }
 
+// The lattice's tiles for program P, and the second population array they need: here,
+// where a program is passed, and not in a step loop or in the middle of another
+// thread's stream capture (which the thread's capture mode exempts this from).  A
+// lattice that would not leave three quarters of the free memory to others runs
+// without tiles.
+static void prepare_tiles(kel_lattice *L, const kel_step_program *P) {
+	L->tile = plan_tiles(L, P);
+	if (!L->tile.ty || L->f2) return;
+	const size_t bytes = (size_t)L->d.Q * L->plane * L->elem;
+	size_t free_b = 0, total_b = 0;
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	cudaThreadExchangeStreamCaptureMode(&mode);
+	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 || cudaMalloc(&L->f2, bytes) != cudaSuccess) {
+		cudaGetLastError();
+		L->f2 = nullptr;
+		L->tile = TilePlan();
+	}
+	cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
+// Back to one step per launch; the second array is given back (unless the stream
+// is being captured, where nothing may be waited for).
+static void drop_tiles(kel_lattice *L) {
+	L->tile = TilePlan();
+	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+	if (!L->f2 || (L->stream && (cudaStreamIsCapturing(L->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)))
+		return;
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	cudaThreadExchangeStreamCaptureMode(&mode);
+	cudaStreamSynchronize(L->stream);
+	if (L->graph && L->graph_tiled) {
+		cudaGraphExecDestroy(L->graph);
+		L->graph = nullptr;
+	}
+	cudaFree(L->f2);
+	L->f2 = nullptr;
+	cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 extern "C" int kel_lattice_set_launch(kel_lattice *L, int32_t cells_per_thread, int32_t block_threads) {
 	if (!L) return fail(KEL_ERR_INVALID_ARGUMENT, "kel_lattice_set_launch: null lattice");
 	if (!launch_ok(L, cells_per_thread, block_threads))
@@ -934,13 +973,13 @@ extern "C" int kel_lattice_set_launch(kel_lattice *L, int32_t cells_per_thread, 
 	L->block = block_threads;
 	L->tuned = true;
 	L->shape_asked = true;
-	L->tile = TilePlan();
+	drop_tiles(L);
 	return KEL_OK;
 }
 
 extern "C" int kel_lattice_get_tiles(const kel_lattice *L, int32_t *steps, int32_t *columns, int32_t *rows) {
 	if (!L || !steps || !columns || !rows) return fail(KEL_ERR_INVALID_ARGUMENT, "kel_lattice_get_tiles: null");
-	const bool tiles = L->tile.ty > 0 && !L->no_f2;
+	const bool tiles = L->tile.ty > 0;
 	*steps = tiles ? TILE_K : 1;
 	*columns = tiles ? (L->tile.wide ? TileWide::W : TileSmall::W) - 2 * TILE_K : 0;
 	*rows = tiles ? L->tile.ty : 0;
@@ -1096,28 +1135,11 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 	L->block = bb;
 	L->tuned = true;
 	L->shape_asked = false;
-	L->tile = plan_tiles(L, P);
+	prepare_tiles(L, P);
 	if (cells_per_thread) *cells_per_thread = bc;
 	if (block_threads) *block_threads = bb;
 	if (ms_per_step) *ms_per_step = best;
 	return KEL_OK;
-}
-
-// The second population array, on first use.  A lattice that would not leave
-// three quarters of the free memory to others runs without the tiles.
-static bool ensure_f2(kel_lattice *L) {
-	if (L->f2) return true;
-	if (L->no_f2) return false;
-	const size_t bytes = (size_t)L->d.Q * L->plane * L->elem;
-	size_t free_b = 0, total_b = 0;
-	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
-		cudaMalloc(&L->f2, bytes) != cudaSuccess) {
-		cudaGetLastError();
-		L->f2 = nullptr;
-		L->no_f2 = true;
-		return false;
-	}
-	return true;
 }
 
 // 2 TILE_K steps from an even one: into the second array and back, so that
@@ -1211,7 +1233,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 		KEL_CUDA(cudaStreamSynchronize(L->stream));
 		L->last_prog = *P;
 		L->have_ops = true;
-		L->tile = plan_tiles(L, P);
+		prepare_tiles(L, P);
 	}
 	if ((rc = ensure_collision_fields(L, P->collision))) return rc;
 
@@ -1230,7 +1252,7 @@ extern "C" int kel_step(kel_lattice *L, const kel_step_program *P, uint64_t n_st
 							   : ((step_flags & KEL_STEP_WRITE_MACROS) && n_steps > 0 ? n_steps - 1 : n_steps);
 	// D2Q9 runs without macro output may do TILE_K steps per launch on tiles, in
 	// pairs of launches from an even step (the remaining steps follow one by one).
-	const bool tiled = L->tile.ty > 0 && !capturing && plain >= (L->t & 1u) + 2 * TILE_K && ensure_f2(L);
+	const bool tiled = L->tile.ty > 0 && !capturing && plain >= (L->t & 1u) + 2 * TILE_K;
 	constexpr uint64_t pair = 2 * TILE_K;
 	const bool graphed = L->stream != nullptr && !capturing && L->cpt != CPT_ROWS && plain >= 2 * GRAPH_STEPS;
 	if (tiled || graphed) {

@@ -92,6 +92,5 @@ struct kel_lattice {
 	bool tuned = false;
 	bool shape_asked = false; // kel_lattice_set_launch named a shape: every step runs it
 	void *f2 = nullptr;       // second population array of the multi-step tiles (TilePlan)
-	bool no_f2 = false;       // it could not be had
 	kel::gb::TilePlan tile;   // of the current program (last_prog)
 };
