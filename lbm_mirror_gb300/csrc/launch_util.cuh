@@ -23,7 +23,9 @@ static cudaError_t launch_overlapped(Kernel kern, dim3 grid, int block, int smem
 	cfg.stream = st;
 	cfg.attrs = &at;
 	cfg.numAttrs = overlap ? 1 : 0;
-	return cudaLaunchKernelEx(&cfg, kern, p);
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+	if (e != cudaSuccess) cudaGetLastError(); // reported here, not by the next call too
+	return e;
 }
 
 // Lets a kernel use `bytes` of dynamic shared memory; the attribute is set to

@@ -2226,7 +2226,9 @@ cudaError_t launch_next(bool overlap, void (*kern)(K...), unsigned grid, int blo
 	cfg.stream = st;
 	cfg.attrs = &at;
 	cfg.numAttrs = overlap && st ? 1 : 0;
-	return cudaLaunchKernelEx(&cfg, kern, K(args)...);
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, K(args)...);
+	if (e != cudaSuccess) cudaGetLastError(); // reported here, not by the next call too
+	return e;
 }
 
 } // namespace
