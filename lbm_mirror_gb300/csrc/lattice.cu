@@ -875,7 +875,7 @@ static TilePlan plan_tiles(const kel_lattice *L, const kel_step_program *P) {
 	TilePlan t;
 	const int64_t ny = L->desc.ny, nxp = L->nxp;
 	if (L->d.Q != 9 || P->arithmetic == KEL_ARITH_REFERENCE || P->collision > KEL_COLL_PSM_GUO || L->shape_asked ||
-		L->hw_active || L->d.Q * L->plane >= ((int64_t)1 << 31))
+		L->hw_active || ny > 65535 || L->d.Q * L->plane >= ((int64_t)1 << 31))
 		return t;
 	bool open = false;
 	for (int fl = 1; fl < MAX_FLAGS; ++fl) open = open || (L->present[fl] && !((L->plain_flags | L->bounce_flags) >> fl & 1u));

@@ -1,6 +1,7 @@
 """The second population array of the multi-step tiles: it is there once the
 program has been passed (no allocation in a later call, so another thread's
-stream capture is left alone), and a named launch shape gives it back."""
+stream capture is left alone), and a named launch shape gives it back; a lattice
+of more rows than the one-step sweep's grid takes is refused as without tiles."""
 import threading
 
 import numpy as np
@@ -82,3 +83,12 @@ def test_a_step_leaves_another_threads_capture_alone():
     assert lat.t == 40
     lat.close()
 
+
+def test_rows_beyond_the_grid_are_refused():
+    lat = _lattice((4, 70000))
+    prog = K.make_program(0.8, K.KEL_COLL_BGK, OPS)
+    for n in (1, 8, 200):
+        with pytest.raises(KelError):
+            lat.step(prog, n)
+        assert lat.t == 0
+    lat.close()
