@@ -487,9 +487,13 @@ int kel_lattice_get_launch(const kel_lattice *lat, int32_t *cells_per_thread, in
  * step by step in the launch shape, as always after kel_lattice_set_launch, which
  * gives the second population array of the tiles back. */
 int kel_lattice_get_tiles(const kel_lattice *lat, int32_t *steps, int32_t *columns, int32_t *rows);
-/* Time `steps` sweeps of `prog` with every launch shape on the lattice's
- * current state and keep the fastest.  The populations are restored after
- * each trial and the time step does not advance. */
+/* Time `steps` sweeps of `prog` with every launch shape, launched as kel_step
+ * launches them, and the lattice's tiles if it has any (kel_lattice_get_tiles), on
+ * the lattice's current state and keep the fastest: cells_per_thread and
+ * block_threads are the fastest shape (with tiles kept, that of the steps which do
+ * not go several at a time), ms_per_step the time of the fastest form.  Tiles that
+ * are not faster are dropped.  The populations are restored after each trial and
+ * the time step does not advance. */
 int kel_lattice_autotune(kel_lattice *lat, const kel_step_program *prog, int32_t steps, int32_t *cells_per_thread,
 						 int32_t *block_threads, float *ms_per_step);
 

@@ -1079,6 +1079,21 @@ SweepParams sweep_params(kel_lattice *L, const kel_step_program *P) { return mak
 } // namespace gb
 } // namespace kel
 
+// 2 TILE_K steps from an even one: into the second array and back, so that
+// the populations are where they were.
+static cudaError_t launch_tile_pair(const kel_lattice *L, const SweepParams &p, int coll) {
+	TileParams q;
+	q.p = p;
+	q.ty = L->tile.ty;
+	for (int k = 0; k < 2; ++k) {
+		q.p.f = k ? L->f2 : L->f;
+		q.out = k ? L->f : L->f2;
+		cudaError_t e = launch_tile(q, L->desc.storage, coll, L->tile.wide, L->stream);
+		if (e != cudaSuccess) return e;
+	}
+	return cudaSuccess;
+}
+
 // Time every supported launch shape on the lattice's own state, then put the
 // state back: the populations are saved to a scratch copy first and restored
 // after each trial, macros are not written, the time step does not move.
@@ -1087,6 +1102,9 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 	if (!L || !P || steps < 2) return fail(KEL_ERR_INVALID_ARGUMENT, "kel_lattice_autotune: bad arguments");
 	int rc;
 	if ((rc = kel_step(L, P, 0, 0))) return rc; // validates and uploads the program
+	const bool asked = L->shape_asked;
+	L->shape_asked = false;
+	prepare_tiles(L, P);
 	if ((rc = ensure_collision_fields(L, P->collision))) return rc;
 	const size_t bytes = (size_t)L->d.Q * L->plane * L->elem;
 	void *save = nullptr;
@@ -1108,6 +1126,7 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 		p.cpt = cands[k][0];
 		p.block = cands[k][1];
 		p.stages = p.cpt == CPT_ROWS ? p.block : 0;
+		p.overlap = p.cpt == 1 && L->stream != nullptr ? OVERLAP_STREAM : OVERLAP_NONE; // as kel_step
 		if (p.cpt == CPT_ROWS) L->rows_used = true;
 		const bool odd0 = (L->t & 1u) != 0;
 		for (int s = 0; s < 2 && e == cudaSuccess; ++s) e = launch_one(L, p, P->collision, exact, odd0 != (s & 1));
@@ -1125,36 +1144,43 @@ extern "C" int kel_lattice_autotune(kel_lattice *L, const kel_step_program *P, i
 		}
 		if (e == cudaSuccess) e = cudaMemcpyAsync(L->f, save, bytes, cudaMemcpyDeviceToDevice, L->stream);
 	}
+	// the tiles, from an even step
+	float tile_ms = 1e30f;
+	if (e == cudaSuccess && L->tile.ty > 0) {
+		p.cpt = 1;
+		p.block = 128;
+		p.stages = 0;
+		p.overlap = L->stream != nullptr ? OVERLAP_STREAM : OVERLAP_NONE;
+		const int pairs = steps / (2 * TILE_K) < 4 ? 4 : steps / (2 * TILE_K);
+		if (L->t & 1u) e = launch_one(L, p, P->collision, exact, true);
+		if (e == cudaSuccess) e = launch_tile_pair(L, p, P->collision);
+		cudaEventRecord(e0, L->stream);
+		for (int s = 0; s < pairs && e == cudaSuccess; ++s) e = launch_tile_pair(L, p, P->collision);
+		cudaEventRecord(e1, L->stream);
+		if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+		if (e == cudaSuccess) e = cudaEventElapsedTime(&tile_ms, e0, e1);
+		tile_ms /= 2 * TILE_K * pairs;
+		if (e == cudaSuccess) e = cudaMemcpyAsync(L->f, save, bytes, cudaMemcpyDeviceToDevice, L->stream);
+	}
 	if (e == cudaSuccess) e = cudaStreamSynchronize(L->stream);
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
 	cudaFree(save);
-	if (e != cudaSuccess) return fail(KEL_ERR_CUDA, "kel_lattice_autotune: %s", cudaGetErrorString(e));
-	if ((rc = check_sweep_error(L, "kel_lattice_autotune"))) return rc;
+	if (e != cudaSuccess) fail(KEL_ERR_CUDA, "kel_lattice_autotune: %s", cudaGetErrorString(e));
+	rc = e != cudaSuccess ? KEL_ERR_CUDA : check_sweep_error(L, "kel_lattice_autotune");
+	if (rc || (L->tile.ty > 0 && tile_ms >= best)) {
+		L->shape_asked = rc ? asked : true; // every step in the fastest shape
+		drop_tiles(L);
+	}
+	if (rc) return rc;
+	if (tile_ms < best) best = tile_ms;
 	L->cpt = bc;
 	L->block = bb;
 	L->tuned = true;
-	L->shape_asked = false;
-	prepare_tiles(L, P);
 	if (cells_per_thread) *cells_per_thread = bc;
 	if (block_threads) *block_threads = bb;
 	if (ms_per_step) *ms_per_step = best;
 	return KEL_OK;
-}
-
-// 2 TILE_K steps from an even one: into the second array and back, so that
-// the populations are where they were.
-static cudaError_t launch_tile_pair(const kel_lattice *L, const SweepParams &p, int coll) {
-	TileParams q;
-	q.p = p;
-	q.ty = L->tile.ty;
-	for (int k = 0; k < 2; ++k) {
-		q.p.f = k ? L->f2 : L->f;
-		q.out = k ? L->f : L->f2;
-		cudaError_t e = launch_tile(q, L->desc.storage, coll, L->tile.wide, L->stream);
-		if (e != cudaSuccess) return e;
-	}
-	return cudaSuccess;
 }
 
 constexpr int GRAPH_STEPS = 64;
