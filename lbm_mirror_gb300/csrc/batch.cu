@@ -786,8 +786,8 @@ int layout(kel_batch *B, int tile) {
 	return KEL_OK;
 }
 
-// overlap: the launch before on the stream is a sweep or tile launch of the
-// same run (see k_batch_sweep)
+// overlap: the launch before on the stream is a sweep of the same run (see
+// k_batch_sweep)
 cudaError_t launch_sweep_batch(const kel_batch *B, bool odd, int write_macros, bool overlap = false) {
 	const BatchParams p = params(B, write_macros);
 	const dim3 g(B->nlaunch);
